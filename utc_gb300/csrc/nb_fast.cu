@@ -24,18 +24,9 @@
 //    target in CTA order (deterministic) and applies the kick/drift update.
 #include <algorithm>
 
-#include "nb_internal.cuh"
+#include "nb_pair.cuh"
 
 namespace nb {
-
-// Packed two-sum (Knuth): s + e == a + b exactly, s = fl(a + b).  Inline
-// PTX keeps the compiler from reassociating it away.
-__device__ __forceinline__ void f2_two_sum(f2 a, f2 b, f2 &s, f2 &e)
-{
-    s = f2_add(a, b);
-    const f2 bb = f2_sub(s, a);
-    e = f2_add(f2_sub(a, f2_sub(s, bb)), f2_sub(b, bb));
-}
 
 // Each thread owns 2*NPAIR targets held as packed pairs (t + 2p*NT,
 // t + (2p+1)*NT).  FLAGS: SK_COMP -- fold each tile's partial sums into a

@@ -1,0 +1,168 @@
+// nb_pair.cuh -- the packed FP32 pair loops shared by the symmetric kernels
+// (nb_sym.cu, single system; nb_batch.cu, batches).
+//
+// A lane's targets are held as NP register pairs (targets 2p and 2p + 1 of
+// the lane in the halves of pair p), so that every pair-term operation is one
+// sm_100+ f32x2 instruction (FADD2 / FMUL2 / FFMA2) for two targets; the chunk
+// body is broadcast into pairs once per rotation step and reused for all NP
+// pairs.  Per pair of targets: 16 packed operations and two MUFU.RSQ.
+//
+// What bounds the loop: register-file reads.  An SM sub-partition reads two
+// 32-bit operands (one 64-bit operand) per cycle and lane, measured on GB300
+// as 1.0 cycle per operation for add, multiply and a*a+c, and 1.4 to 1.7 for
+// an FMA with three different register operands (the reuse cache serves a
+// weight that two neighbouring FMAs share).  The six accumulating FMAs of a
+// pair read three operands each: 37 operand cycles against 32 pipe cycles per
+// pair of targets, so 18.5 cycles per pair and warp (4140 G interactions/s
+// at 2.07 GHz) are the floor of this arithmetic without operand reuse.
+// Measured, force kernel, N = 65536, 16 targets per lane: 4002 G
+// interactions/s, against 3578 for the scalar loop that it replaced, whose 17
+// issue slots per pair left no room for the operand stalls (the packed loop
+// issues 9); 4 warps x 20 targets at N = 262144: 3965 against 3574;
+// compensated 1 x 12: 3673 against 3166.  Timed beside it (the loop alone, 16
+// targets, 4022): the reaction folded to a scalar before each shuffle 3926,
+// the chunk stored as duplicated pairs in shared memory 3929, the reaction
+// added through shared memory 3887, packed differences with scalar
+// accumulation 3770, two chunk bodies per pair instead of two targets 4016
+// (12 targets, 244 registers), 18 targets per lane 4002, 20 targets 3910.
+#pragma once
+
+#include "nb_internal.cuh"
+
+namespace nb {
+
+// A lane's 2 * NP targets: positions and masses negated (r = q + (-p); the
+// reaction on the chunk body points along -r), and their acceleration sums.
+template <int NP>
+struct PairTargets {
+    f2 px[NP], py[NP], pz[NP], nm[NP], ax[NP], ay[NP], az[NP];
+
+    // target t of the lane (0 <= t < 2 NP) is at(t): its (x, y, z, m), or
+    // zeros for a missing one, whose reactions are then 0
+    template <class At>
+    __device__ __forceinline__ void load(At at)
+    {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            const float4 a = at(2 * p), b = at(2 * p + 1);
+            px[p] = f2_pack(-a.x, -b.x);
+            py[p] = f2_pack(-a.y, -b.y);
+            pz[p] = f2_pack(-a.z, -b.z);
+            nm[p] = f2_pack(-a.w, -b.w);
+        }
+        clear();
+    }
+    __device__ __forceinline__ void clear()
+    {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) ax[p] = ay[p] = az[p] = f2_pack(0.f, 0.f);
+    }
+    // the sums of target t as (x, y, z, 0)
+    __device__ __forceinline__ float4 sum(int t) const
+    {
+        float x[2], y[2], z[2];
+        f2_unpack(ax[t >> 1], x[0], x[1]);
+        f2_unpack(ay[t >> 1], y[0], y[1]);
+        f2_unpack(az[t >> 1], z[0], z[1]);
+        return make_float4(x[t & 1], y[t & 1], z[t & 1], 0.f);
+    }
+};
+
+// r = q - p and 1 / (|r|^2 + eps2)^(3/2) for a pair of targets
+struct PairTerm {
+    f2 rx, ry, rz, inv3;
+};
+
+template <int NP>
+__device__ __forceinline__ PairTerm pair_term(const PairTargets<NP> &t, int p, f2 X, f2 Y, f2 Z, f2 EPS2)
+{
+    PairTerm o;
+    o.rx = f2_add(X, t.px[p]);
+    o.ry = f2_add(Y, t.py[p]);
+    o.rz = f2_add(Z, t.pz[p]);
+    f2 d2 = f2_fma(o.rx, o.rx, EPS2);
+    d2 = f2_fma(o.ry, o.ry, d2);
+    d2 = f2_fma(o.rz, o.rz, d2);
+    float lo, hi;
+    f2_unpack(d2, lo, hi);
+    const f2 inv = f2_pack(rsqrt_approx(lo), rsqrt_approx(hi));
+    o.inv3 = f2_mul(inv, f2_mul(inv, inv));
+    return o;
+}
+
+template <int NP>
+__device__ __forceinline__ void pair_pull(PairTargets<NP> &t, int p, const PairTerm &r, f2 M)
+{
+    const f2 st = f2_mul(M, r.inv3);
+    t.ax[p] = f2_fma(r.rx, st, t.ax[p]);
+    t.ay[p] = f2_fma(r.ry, st, t.ay[p]);
+    t.az[p] = f2_fma(r.rz, st, t.az[p]);
+}
+
+// The pull of the 32 chunk bodies in sC on the lane's targets (a chunk inside
+// the targets' own row block: both orders of each pair occur there).
+template <int NP>
+__device__ __forceinline__ void chunk_pull(PairTargets<NP> &t, const float4 *sC, f2 EPS2)
+{
+#pragma unroll 1
+    for (int j = 0; j < 32; ++j) {
+        const float4 q = sC[j];
+        const f2 X = f2_pack(q.x, q.x), Y = f2_pack(q.y, q.y), Z = f2_pack(q.z, q.z), M = f2_pack(q.w, q.w);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) pair_pull(t, p, pair_term(t, p, X, Y, Z, EPS2), M);
+    }
+}
+
+__device__ __forceinline__ f2 f2_shfl(f2 v, int from)
+{
+    float lo, hi;
+    f2_unpack(v, lo, hi);
+    return f2_pack(__shfl_sync(0xffffffffu, lo, from), __shfl_sync(0xffffffffu, hi, from));
+}
+
+__device__ __forceinline__ float f2_fold(f2 v)
+{
+    float lo, hi;
+    f2_unpack(v, lo, hi);
+    return lo + hi;
+}
+
+// The chunk's bodies against the lane's targets, each unordered pair once: at
+// step r lane l pairs its targets with chunk body (l + r) mod 32 and carries
+// that body's reaction (one half per target of a pair, folded at the end),
+// passed on to lane l - 1 after the step.  Returns the reaction on chunk body
+// l from the warp's targets.
+template <int NP>
+__device__ __forceinline__ float3 chunk_react(PairTargets<NP> &t, const float4 *sC, int lane, f2 EPS2)
+{
+    f2 fx = f2_pack(0.f, 0.f), fy = fx, fz = fx;
+    const int from = (lane + 1) & 31;
+#pragma unroll 8
+    for (int r = 0; r < 32; ++r) {
+        const float4 q = sC[(lane + r) & 31];
+        const f2 X = f2_pack(q.x, q.x), Y = f2_pack(q.y, q.y), Z = f2_pack(q.z, q.z), M = f2_pack(q.w, q.w);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            const PairTerm o = pair_term(t, p, X, Y, Z, EPS2);
+            pair_pull(t, p, o, M);
+            const f2 ss = f2_mul(t.nm[p], o.inv3);
+            fx = f2_fma(o.rx, ss, fx);
+            fy = f2_fma(o.ry, ss, fy);
+            fz = f2_fma(o.rz, ss, fz);
+        }
+        fx = f2_shfl(fx, from);
+        fy = f2_shfl(fy, from);
+        fz = f2_shfl(fz, from);
+    }
+    return make_float3(f2_fold(fx), f2_fold(fy), f2_fold(fz));
+}
+
+// Packed two-sum (Knuth): s + e == a + b exactly, s = fl(a + b).
+__device__ __forceinline__ void f2_two_sum(f2 a, f2 b, f2 &s, f2 &e)
+{
+    s = f2_add(a, b);
+    const f2 bb = f2_sub(s, a);
+    e = f2_add(f2_sub(a, f2_sub(s, bb)), f2_sub(b, bb));
+}
+
+}  // namespace nb

@@ -57,10 +57,9 @@
 // source side is so summed essentially exactly, for any eps2 > 0.  The scale
 // sits in a record after the accumulators, written at nb_set_state (and for
 // a new eps2) by sym_fx_prepare / sym_fx_rescale; the integrator zeroes the
-// accumulators after reading them.  On GB300 this variant ran 2-10 % slower
-// than the triangular array of the same shape (the pair loop's schedule
-// shifts with the code around it; 3513 against 3593 G interactions/s for
-// the banded 4 x 20 triangular plan at N = 2^21).
+// accumulators after reading them.  On GB300 this variant runs 3 % slower
+// than the triangular array of the same shape (3879 against 4002 G
+// interactions/s at N = 65536).
 //
 // Compensated variant (COMP): each target's per-chunk partial sum (32
 // sources) is folded into a two-sum (hi, lo) pair, the W warps' reactions on
@@ -68,16 +67,14 @@
 // block after the hi block of tpart and of spart); the compensated
 // integrator sums them with two-sums.
 //
-// Shape.  The loop is issue-bound (16 FP32 instructions + 1 MUFU per pair,
-// plus one LDS and three SHFL per lane and rotation step), and its issue
-// rate improves with more independent targets per lane rather than with more
-// warps: one-warp CTAs with 16 targets per lane (225 registers, 8 warps per
-// SM) run 15 % faster than 8-warp CTAs with 8 targets per lane (80 registers,
-// 24 warps per SM) on GB300.  Small row blocks make the triangular
-// source-side array large (about N^2 / (2 rb) float4), so the default shape
-// grows to 4 warps x 20 targets when that array would pass kSymSpartBudget,
-// and is cut into bands beyond that.
-#include "nb_internal.cuh"
+// Shape.  The pair loop (nb_pair.cuh) is bounded by register-file reads and,
+// below that, by how many independent targets a lane has: one-warp CTAs with
+// 16 targets per lane (236 registers, 8 warps per SM) run ahead of 12 targets
+// (12 warps) and of 8 (16 warps) by 4 % and 8 %.  Small row blocks make the
+// triangular source-side array large (about N^2 / (2 rb) float4), so the
+// default shape grows to 4 warps x 20 targets when that array would pass
+// kSymSpartBudget, and is cut into bands beyond that.
+#include "nb_pair.cuh"
 
 namespace nb {
 
@@ -112,6 +109,128 @@ __device__ __forceinline__ void fx_emit(unsigned long long *acc, int n, int j, f
     fx_add(acc + 2 * nn + j, acc + 5 * nn + j, fz, r);
 }
 
+// One CTA's share of a row: row block I's targets against the chunks
+// [kc0, kc1), target-side sums to dst (and dst + tlo), reactions to spart.
+// A function of its own, not inlined into the loop over rows below: inlined,
+// ptxas carries the target pairs through that loop with some 270 M register
+// moves per launch at N = 65536 (936 M instructions against 665 M, 3107
+// against 3660 G interactions/s on the same box).
+template <int W, int BPT, bool COMP, bool FX>
+__device__ __noinline__ void sym_row_segment(const float4 *__restrict__ pos, int n, float eps2, float4 *dst,
+                                             float4 *spart, long long soff, long long tlo, long long slo, int I,
+                                             int kc0, int kc1)
+{
+    constexpr int NP = BPT / 2;
+    constexpr int WB = 32 * BPT;
+    constexpr int RB = W * WB;
+    constexpr int RC = RB / 32;
+    __shared__ __align__(16) float4 sC[32];
+    __shared__ float sF[3][W][32];
+    const int lane = threadIdx.x & 31;
+    const int wid = threadIdx.x >> 5;
+    const int tbase = I * RB + wid * WB;
+    const float4 pad = make_float4(kPadCoord, kPadCoord, kPadCoord, 0.f);
+    const f2 EPS2 = f2_pack(eps2, eps2);
+
+    PairTargets<NP> T;
+    T.load([&](int t) {
+        const int i = tbase + lane + 32 * t;
+        return i < n ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    });
+    // COMP: compensated target sums (hi in h*, lo in l*)
+    constexpr int CB = COMP ? NP : 1;
+    f2 hx[CB], hy[CB], hz[CB], lx[CB], ly[CB], lz[CB];
+    if constexpr (COMP) {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) hx[p] = hy[p] = hz[p] = lx[p] = ly[p] = lz[p] = f2_pack(0.f, 0.f);
+    }
+    // the next chunk is read ahead: a warp has one neighbour to hide the load
+    // behind (3962 against 3848 G interactions/s at N = 65536)
+    float4 nxt = kc0 * 32 + lane < n ? pos[kc0 * 32 + lane] : pad;
+#pragma unroll 1
+    for (int kc = kc0; kc < kc1; ++kc) {
+        const int jb = kc * 32;
+        __syncthreads();  // previous chunk: sC reads and sF reads are done
+        if (wid == 0) sC[lane] = nxt;
+        __syncthreads();
+        if (wid == 0) nxt = jb + 32 + lane < n ? pos[jb + 32 + lane] : pad;
+        if (kc < (I + 1) * RC) {
+            // chunk inside the own row block: directed, target side only
+            chunk_pull(T, sC, EPS2);
+        } else {
+            // f: the reaction on chunk body `lane` from this warp
+            const float3 f = chunk_react(T, sC, lane, EPS2);
+            if constexpr (W > 1) {
+                sF[0][wid][lane] = f.x;
+                sF[1][wid][lane] = f.y;
+                sF[2][wid][lane] = f.z;
+                __syncthreads();
+            }
+            if (wid == 0 && jb + lane < n) {
+                float sx = f.x, sy = f.y, sz = f.z, cx = 0.f, cy = 0.f, cz = 0.f;
+#pragma unroll
+                for (int w = 1; w < W; ++w) {
+                    if constexpr (COMP) {
+                        float e;
+                        two_sum(sx, sF[0][w][lane], sx, e);
+                        cx = __fadd_rn(cx, e);
+                        two_sum(sy, sF[1][w][lane], sy, e);
+                        cy = __fadd_rn(cy, e);
+                        two_sum(sz, sF[2][w][lane], sz, e);
+                        cz = __fadd_rn(cz, e);
+                    } else {
+                        sx += sF[0][w][lane];
+                        sy += sF[1][w][lane];
+                        sz += sF[2][w][lane];
+                    }
+                }
+                if constexpr (FX) {
+                    fx_emit(reinterpret_cast<unsigned long long *>(spart), n, jb + lane, sx, sy, sz);
+                } else {
+                    const long long so = soff + (jb + lane - (I + 1) * RB);
+                    spart[so] = make_float4(sx, sy, sz, 0.f);
+                    if constexpr (COMP) spart[slo + so] = make_float4(cx, cy, cz, 0.f);
+                }
+            }
+        }
+        if constexpr (COMP) {
+            // fold this chunk's 32-source partial sums into (hi, lo)
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                f2 e;
+                f2_two_sum(hx[p], T.ax[p], hx[p], e);
+                lx[p] = f2_add(lx[p], e);
+                f2_two_sum(hy[p], T.ay[p], hy[p], e);
+                ly[p] = f2_add(ly[p], e);
+                f2_two_sum(hz[p], T.az[p], hz[p], e);
+                lz[p] = f2_add(lz[p], e);
+            }
+            T.clear();
+        }
+    }
+    dst += wid * WB + lane;
+    if constexpr (COMP) {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            T.ax[p] = hx[p];
+            T.ay[p] = hy[p];
+            T.az[p] = hz[p];
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < BPT; ++t) dst[32 * t] = T.sum(t);
+    if constexpr (COMP) {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            T.ax[p] = lx[p];
+            T.ay[p] = ly[p];
+            T.az[p] = lz[p];
+        }
+#pragma unroll
+        for (int t = 0; t < BPT; ++t) dst[tlo + 32 * t] = T.sum(t);
+    }
+}
+
 // FX: spart is the fixed-point accumulator buffer (with its record), not
 // the triangular array.  BAND: one band of a banded plan, items
 // [it0, it0 + total) covering row blocks from r0 on: target-side slot
@@ -124,13 +243,8 @@ __global__ void __launch_bounds__(32 * W, MINB) sym_force_kernel(const float4 *_
                                                            long long tlo, long long slo, long long it0,
                                                            int r0, long long soff0)
 {
-    constexpr int WB = 32 * BPT;
-    constexpr int RB = W * WB;
+    constexpr int RB = W * 32 * BPT;
     constexpr int RC = RB / 32;
-    __shared__ __align__(16) float4 sC[32];
-    __shared__ float sF[3][W][32];
-    const int lane = threadIdx.x & 31;
-    const int wid = threadIdx.x >> 5;
     const int c = blockIdx.x;
     long long it = sk_start(c, total, gridDim.x);
     long long end = sk_start(c + 1, total, gridDim.x);
@@ -138,283 +252,14 @@ __global__ void __launch_bounds__(32 * W, MINB) sym_force_kernel(const float4 *_
         it += it0;
         end += it0;
     }
-    const float4 pad = make_float4(kPadCoord, kPadCoord, kPadCoord, 0.f);
-
     while (it < end) {
         const int I = sym_row_of(it, nc, RC, nrb);
         const long long rfirst = sym_prefix(I, nc, RC);
         const long long rend = sym_prefix(I + 1, nc, RC);
         const long long seg_end = end < rend ? end : rend;
-        const int kc0 = I * RC + (int)(it - rfirst);
-        const int kc1 = I * RC + (int)(seg_end - rfirst);
-        const int tbase = I * RB + wid * WB;
-
-        // nm = -m: the reaction on the chunk body points along -r
-        float px[BPT], py[BPT], pz[BPT], nm[BPT], ax[BPT], ay[BPT], az[BPT];
-        // COMP: compensated target sums (hi in h*, lo in l*)
-        constexpr int CB = COMP ? BPT : 1;
-        float hx[CB], hy[CB], hz[CB], lx[CB], ly[CB], lz[CB];
-#pragma unroll
-        for (int k = 0; k < BPT; ++k) {
-            const int i = tbase + lane + 32 * k;
-            // missing targets get zero mass: their reactions on the chunk are 0
-            const float4 q = i < n ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-            px[k] = q.x;
-            py[k] = q.y;
-            pz[k] = q.z;
-            nm[k] = -q.w;
-            ax[k] = ay[k] = az[k] = 0.f;
-            if constexpr (COMP) hx[k] = hy[k] = hz[k] = lx[k] = ly[k] = lz[k] = 0.f;
-        }
-        for (int kc = kc0; kc < kc1; ++kc) {
-            const int jb = kc * 32;
-            __syncthreads();  // previous chunk: sC reads and sF reads are done
-            if (wid == 0) sC[lane] = (jb + lane < n) ? pos[jb + lane] : pad;
-            __syncthreads();
-            if (kc < (I + 1) * RC) {
-                // chunk inside the own row block: directed, target side only
-#pragma unroll 4
-                for (int j = 0; j < 32; ++j) {
-                    const float4 q = sC[j];
-#pragma unroll
-                    for (int k = 0; k < BPT; ++k) {
-                        const float rx = q.x - px[k], ry = q.y - py[k], rz = q.z - pz[k];
-                        float d2 = fmaf(rx, rx, eps2);
-                        d2 = fmaf(ry, ry, d2);
-                        d2 = fmaf(rz, rz, d2);
-                        const float inv = rsqrt_approx(d2);
-                        const float s = (q.w * inv) * (inv * inv);
-                        ax[k] = fmaf(rx, s, ax[k]);
-                        ay[k] = fmaf(ry, s, ay[k]);
-                        az[k] = fmaf(rz, s, az[k]);
-                    }
-                }
-            } else {
-                float fx = 0.f, fy = 0.f, fz = 0.f;
-#pragma unroll 2
-                for (int r = 0; r < 32; ++r) {
-                    const float4 q = sC[(lane + r) & 31];
-#pragma unroll
-                    for (int k = 0; k < BPT; ++k) {
-                        const float rx = q.x - px[k], ry = q.y - py[k], rz = q.z - pz[k];
-                        float d2 = fmaf(rx, rx, eps2);
-                        d2 = fmaf(ry, ry, d2);
-                        d2 = fmaf(rz, rz, d2);
-                        const float inv = rsqrt_approx(d2);
-                        const float inv3 = inv * (inv * inv);
-                        const float st = q.w * inv3;    // on the target, from the chunk body
-                        const float ss = nm[k] * inv3;  // on the chunk body, from the target
-                        ax[k] = fmaf(rx, st, ax[k]);
-                        ay[k] = fmaf(ry, st, ay[k]);
-                        az[k] = fmaf(rz, st, az[k]);
-                        fx = fmaf(rx, ss, fx);
-                        fy = fmaf(ry, ss, fy);
-                        fz = fmaf(rz, ss, fz);
-                    }
-                    const int from = (lane + 1) & 31;
-                    fx = __shfl_sync(0xffffffffu, fx, from);
-                    fy = __shfl_sync(0xffffffffu, fy, from);
-                    fz = __shfl_sync(0xffffffffu, fz, from);
-                }
-                // lane l now holds the reaction on chunk body l from this warp
-                sF[0][wid][lane] = fx;
-                sF[1][wid][lane] = fy;
-                sF[2][wid][lane] = fz;
-                __syncthreads();
-                if (FX && wid == 0 && jb + lane < n) {
-                    float sx = 0.f, sy = 0.f, sz = 0.f;
-#pragma unroll
-                    for (int w = 0; w < W; ++w) {
-                        sx += sF[0][w][lane];
-                        sy += sF[1][w][lane];
-                        sz += sF[2][w][lane];
-                    }
-                    fx_emit(reinterpret_cast<unsigned long long *>(spart), n, jb + lane, sx, sy, sz);
-                } else if (wid == 0 && jb + lane < n) {
-                    long long so = sym_soff(I, n, RB) + (jb + lane - (I + 1) * RB);
-                    if constexpr (BAND) so -= soff0;
-                    if constexpr (COMP) {
-                        float sx = 0.f, sy = 0.f, sz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f, e;
-#pragma unroll
-                        for (int w = 0; w < W; ++w) {
-                            two_sum(sx, sF[0][w][lane], sx, e);
-                            cx = __fadd_rn(cx, e);
-                            two_sum(sy, sF[1][w][lane], sy, e);
-                            cy = __fadd_rn(cy, e);
-                            two_sum(sz, sF[2][w][lane], sz, e);
-                            cz = __fadd_rn(cz, e);
-                        }
-                        spart[so] = make_float4(sx, sy, sz, 0.f);
-                        spart[slo + so] = make_float4(cx, cy, cz, 0.f);
-                    } else {
-                        float sx = 0.f, sy = 0.f, sz = 0.f;
-#pragma unroll
-                        for (int w = 0; w < W; ++w) {
-                            sx += sF[0][w][lane];
-                            sy += sF[1][w][lane];
-                            sz += sF[2][w][lane];
-                        }
-                        spart[so] = make_float4(sx, sy, sz, 0.f);
-                    }
-                }
-            }
-            if constexpr (COMP) {
-                // fold this chunk's 32-source partial sums into (hi, lo)
-#pragma unroll
-                for (int k = 0; k < BPT; ++k) {
-                    float e;
-                    two_sum(hx[k], ax[k], hx[k], e);
-                    lx[k] = __fadd_rn(lx[k], e);
-                    two_sum(hy[k], ay[k], hy[k], e);
-                    ly[k] = __fadd_rn(ly[k], e);
-                    two_sum(hz[k], az[k], hz[k], e);
-                    lz[k] = __fadd_rn(lz[k], e);
-                    ax[k] = ay[k] = az[k] = 0.f;
-                }
-            }
-        }
-        float4 *dst = tpart + (size_t)(c + I - (BAND ? r0 : 0)) * RB + wid * WB;
-#pragma unroll
-        for (int k = 0; k < BPT; ++k) {
-            if constexpr (COMP) {
-                dst[lane + 32 * k] = make_float4(hx[k], hy[k], hz[k], 0.f);
-                dst[tlo + lane + 32 * k] = make_float4(lx[k], ly[k], lz[k], 0.f);
-            } else {
-                dst[lane + 32 * k] = make_float4(ax[k], ay[k], az[k], 0.f);
-            }
-        }
-        it = seg_end;
-    }
-}
-
-// Packed variant: each lane's targets as NP f32x2 pairs (targets k and
-// k + NP of the lane), every pair-term operation one FADD2/FMUL2/FFMA2 for
-// two targets; the chunk body is duplicated into register pairs; the
-// reaction on the chunk body is accumulated as a pair (one half per target of
-// the pair) and folded to a scalar before each shuffle.  Same work layout,
-// partials and results' order of summation as sym_force_kernel.
-template <int W, int NP>
-__global__ void __launch_bounds__(32 * W) sym_force_kernel_f2(const float4 *__restrict__ pos, int n,
-                                                              float eps2, float4 *__restrict__ tpart,
-                                                              float4 *__restrict__ spart,
-                                                              long long total, int nc, int nrb,
-                                                              long long, long long, long long, int,
-                                                              long long)
-{
-    constexpr int BPT = 2 * NP;
-    constexpr int WB = 32 * BPT;
-    constexpr int RB = W * WB;
-    constexpr int RC = RB / 32;
-    __shared__ __align__(16) float4 sC[32];
-    __shared__ float sF[3][W][32];
-    const int lane = threadIdx.x & 31;
-    const int wid = threadIdx.x >> 5;
-    const int c = blockIdx.x;
-    long long it = sk_start(c, total, gridDim.x);
-    const long long end = sk_start(c + 1, total, gridDim.x);
-    const float4 pad = make_float4(kPadCoord, kPadCoord, kPadCoord, 0.f);
-    const f2 EPS2 = f2_pack(eps2, eps2);
-    const f2 ZERO = f2_pack(0.f, 0.f);
-
-    while (it < end) {
-        const int I = sym_row_of(it, nc, RC, nrb);
-        const long long rfirst = sym_prefix(I, nc, RC);
-        const long long rend = sym_prefix(I + 1, nc, RC);
-        const long long seg_end = end < rend ? end : rend;
-        const int kc0 = I * RC + (int)(it - rfirst);
-        const int kc1 = I * RC + (int)(seg_end - rfirst);
-        const int tbase = I * RB + wid * WB;
-
-        f2 PX[NP], PY[NP], PZ[NP], NM[NP], AX[NP], AY[NP], AZ[NP];
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-            const int i0 = tbase + lane + 32 * p;
-            const int i1 = i0 + 32 * NP;
-            const float4 q0 = i0 < n ? pos[i0] : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float4 q1 = i1 < n ? pos[i1] : make_float4(0.f, 0.f, 0.f, 0.f);
-            PX[p] = f2_pack(q0.x, q1.x);
-            PY[p] = f2_pack(q0.y, q1.y);
-            PZ[p] = f2_pack(q0.z, q1.z);
-            NM[p] = f2_pack(-q0.w, -q1.w);  // negated: reactions point along -r
-            AX[p] = AY[p] = AZ[p] = ZERO;
-        }
-        for (int kc = kc0; kc < kc1; ++kc) {
-            const int jb = kc * 32;
-            __syncthreads();
-            if (wid == 0) sC[lane] = (jb + lane < n) ? pos[jb + lane] : pad;
-            __syncthreads();
-            const bool diag = kc < (I + 1) * RC;
-            float fx = 0.f, fy = 0.f, fz = 0.f;
-#pragma unroll 2
-            for (int r = 0; r < 32; ++r) {
-                const float4 q = sC[diag ? r : ((lane + r) & 31)];
-                const f2 XB = f2_pack(q.x, q.x), YB = f2_pack(q.y, q.y);
-                const f2 ZB = f2_pack(q.z, q.z), MB = f2_pack(q.w, q.w);
-                f2 FX = f2_pack(fx, 0.f), FY = f2_pack(fy, 0.f), FZ = f2_pack(fz, 0.f);
-#pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    const f2 rx = f2_sub(XB, PX[p]);
-                    const f2 ry = f2_sub(YB, PY[p]);
-                    const f2 rz = f2_sub(ZB, PZ[p]);
-                    f2 d2 = f2_fma(rx, rx, EPS2);
-                    d2 = f2_fma(ry, ry, d2);
-                    d2 = f2_fma(rz, rz, d2);
-                    float dlo, dhi;
-                    f2_unpack(d2, dlo, dhi);
-                    const f2 inv = f2_pack(rsqrt_approx(dlo), rsqrt_approx(dhi));
-                    const f2 inv3 = f2_mul(f2_mul(inv, inv), inv);
-                    const f2 st = f2_mul(MB, inv3);
-                    AX[p] = f2_fma(rx, st, AX[p]);
-                    AY[p] = f2_fma(ry, st, AY[p]);
-                    AZ[p] = f2_fma(rz, st, AZ[p]);
-                    if (!diag) {
-                        const f2 ss = f2_mul(NM[p], inv3);
-                        FX = f2_fma(rx, ss, FX);
-                        FY = f2_fma(ry, ss, FY);
-                        FZ = f2_fma(rz, ss, FZ);
-                    }
-                }
-                if (!diag) {
-                    float lo, hi;
-                    f2_unpack(FX, lo, hi);
-                    fx = lo + hi;
-                    f2_unpack(FY, lo, hi);
-                    fy = lo + hi;
-                    f2_unpack(FZ, lo, hi);
-                    fz = lo + hi;
-                    const int from = (lane + 1) & 31;
-                    fx = __shfl_sync(0xffffffffu, fx, from);
-                    fy = __shfl_sync(0xffffffffu, fy, from);
-                    fz = __shfl_sync(0xffffffffu, fz, from);
-                }
-            }
-            if (!diag) {
-                sF[0][wid][lane] = fx;
-                sF[1][wid][lane] = fy;
-                sF[2][wid][lane] = fz;
-                __syncthreads();
-                if (wid == 0 && jb + lane < n) {
-                    float sx = 0.f, sy = 0.f, sz = 0.f;
-#pragma unroll
-                    for (int w = 0; w < W; ++w) {
-                        sx += sF[0][w][lane];
-                        sy += sF[1][w][lane];
-                        sz += sF[2][w][lane];
-                    }
-                    spart[sym_soff(I, n, RB) + (jb + lane - (I + 1) * RB)] = make_float4(sx, sy, sz, 0.f);
-                }
-            }
-        }
-        float4 *dst = tpart + (size_t)(c + I) * RB + wid * WB;
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-            float x0, x1, y0, y1, z0, z1;
-            f2_unpack(AX[p], x0, x1);
-            f2_unpack(AY[p], y0, y1);
-            f2_unpack(AZ[p], z0, z1);
-            dst[lane + 32 * p] = make_float4(x0, y0, z0, 0.f);
-            dst[lane + 32 * (p + NP)] = make_float4(x1, y1, z1, 0.f);
-        }
+        sym_row_segment<W, BPT, COMP, FX>(pos, n, eps2, tpart + (size_t)(c + I - (BAND ? r0 : 0)) * RB, spart,
+                                          sym_soff(I, n, RB) - (BAND ? soff0 : 0), tlo, slo, I,
+                                          I * RC + (int)(it - rfirst), I * RC + (int)(seg_end - rfirst));
         it = seg_end;
     }
 }
@@ -609,12 +454,16 @@ __global__ void __launch_bounds__(256) sym_fold_comp_kernel(const float4 *__rest
 typedef void (*sym_kernel_t)(const float4 *, int, float, float4 *, float4 *, long long, int, int,
                              long long, long long, long long, int, long long);
 
-// bpt > 0: scalar kernel with bpt bodies per lane (the third template
-// argument asks for that many resident CTAs per SM); bpt < 0: packed f32x2
-// kernel with -bpt bodies per lane.  comp: the compensated kernel (scalar
-// shapes with up to 12 targets per lane: 13 registers per target).
+// bpt bodies per lane (the third template argument asks for that many
+// resident CTAs per SM); 8 warps x 8 or 4 and 4 warps x 8 also go by the
+// negative of their bpt.  comp: the compensated kernel (up to 12 targets per
+// lane: 13 registers per target).
 static sym_kernel_t sym_kernel_for(int w, int bpt, int comp, int fixed = 0, int band = 0)
 {
+    if (bpt < 0) {
+        if (comp || fixed || band || !((w == 8 && (bpt == -8 || bpt == -4)) || (w == 4 && bpt == -8))) return nullptr;
+        bpt = -bpt;
+    }
     if (band) {  // banded triangular plans: the default shapes
         if (fixed) return nullptr;
         if (comp) {
@@ -653,9 +502,6 @@ static sym_kernel_t sym_kernel_for(int w, int bpt, int comp, int fixed = 0, int 
     if (w == 4 && bpt == 8) return sym_force_kernel<4, 8, 1, false>;
     if (w == 8 && bpt == 4) return sym_force_kernel<8, 4, 1, false>;
     if (w == 8 && bpt == 8) return sym_force_kernel<8, 8, 1, false>;
-    if (w == 8 && bpt == -8) return sym_force_kernel_f2<8, 4>;
-    if (w == 4 && bpt == -8) return sym_force_kernel_f2<4, 4>;
-    if (w == 8 && bpt == -4) return sym_force_kernel_f2<8, 2>;
     return nullptr;
 }
 
