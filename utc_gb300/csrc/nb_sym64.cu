@@ -136,51 +136,63 @@ __global__ void __launch_bounds__(32 * W, MINB) sym64_force_kernel(const double4
     }
 }
 
-// Per body: target-side slots (CTA order) + source-side rows 0..I-1 (row
-// order), then the reference's kick / damping / drift in its order with
-// unfused IEEE operations (bodysystem.cc:135-182), or the bare acceleration.
-__global__ void sym64_integrate_kernel(const double4 *__restrict__ pos_old, double4 *__restrict__ pos_new,
-                                       double4 *__restrict__ vel, const double4 *__restrict__ tpart,
-                                       const double4 *__restrict__ spart, int n, int rb, int nc, int nrb,
-                                       long long total, int grid, double damping, double dt, int kick,
-                                       double G, double4 *__restrict__ acc_out,
-                                       const unsigned long long *__restrict__ ffrange,
-                                       const double4 *__restrict__ accsum)
+// Per body: target-side slots + source-side rows 0..I-1, then the reference's
+// kick / damping / drift in its order with unfused IEEE operations
+// (bodysystem.cc:135-182), or the bare acceleration (with the potential sum
+// in w when the force pass recorded it: the float-float energy pass).
+//
+// Reads all partials once (N^2 / (2 rb) double4), so memory and the narrow
+// FP64 pipe's additions bound it.  A block takes 32 bodies x 8 slices: slice
+// q sums slots c0 + q, c0 + q + 8, ... and rows q, q + 8, ... in order, and the
+// slices are added in slice order (fixed order: deterministic); the w sums
+// only where they are asked for.  With one thread per body the walk over up
+// to 255 rows was a chain of loads (N = 16384, rb = 64: 84 us a step).
+constexpr int kSym64Slices = 8;
+
+__global__ void __launch_bounds__(32 * kSym64Slices)
+    sym64_integrate_kernel(const double4 *__restrict__ pos_old, double4 *__restrict__ pos_new,
+                           double4 *__restrict__ vel, const double4 *__restrict__ tpart,
+                           const double4 *__restrict__ spart, int n, int rb, int nc, int nrb, long long total,
+                           int grid, double damping, double dt, int kick, double G,
+                           double4 *__restrict__ acc_out, const unsigned long long *__restrict__ ffrange,
+                           const double4 *__restrict__ accsum)
 {
+    __shared__ double red[4][kSym64Slices][32];
+    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
     // bodies from the last one down: the longest row walks start first
-    const int i = n - 1 - (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (i < 0) return;
-    // w: the potential sum_j m_j / sqrt(d2), j != i, when the force pass
-    // recorded it (the float-float energy pass), else 0
+    const int i = n - 1 - (int)(blockIdx.x * 32 + lane);
+    const bool want_w = acc_out != nullptr;
     double ax = 0.0, ay = 0.0, az = 0.0, aw = 0.0;
-    if (accsum) {  // banded plan: the fold kernel's sums
-        const double4 q = accsum[i];
-        ax = q.x;
-        ay = q.y;
-        az = q.z;
-        aw = q.w;
-    } else {
+    auto add = [&](const double4 &v) {
+        ax = __dadd_rn(ax, v.x);
+        ay = __dadd_rn(ay, v.y);
+        az = __dadd_rn(az, v.z);
+        if (want_w) aw = __dadd_rn(aw, v.w);
+    };
+    if (i >= 0 && accsum) {  // banded plan: the fold kernel's sums
+        if (q == 0) add(accsum[i]);
+    } else if (i >= 0) {
         const int rc = rb / 32;
         const int I = i / rb;
         const int c0 = sk_owner(sym_prefix(I, nc, rc), total, grid);
         const int c1 = sk_owner(sym_prefix(I + 1, nc, rc) - 1, total, grid);
         const int li = i - I * rb;
-        for (int c = c0; c <= c1; ++c) {
-            const double4 q = tpart[(size_t)(c + I) * rb + li];
-            ax = __dadd_rn(ax, q.x);
-            ay = __dadd_rn(ay, q.y);
-            az = __dadd_rn(az, q.z);
-            aw = __dadd_rn(aw, q.w);
-        }
-        long long off = (long long)i - rb;  // row r at soff(r) + i - (r + 1) rb
-        for (int r = 0; r < I; ++r) {
-            const double4 q = spart[off];
-            off += (long long)n - (long long)(r + 2) * rb;
-            ax = __dadd_rn(ax, q.x);
-            ay = __dadd_rn(ay, q.y);
-            az = __dadd_rn(az, q.z);
-            aw = __dadd_rn(aw, q.w);
-        }
+        for (int c = c0 + q; c <= c1; c += kSym64Slices) add(tpart[(size_t)(c + I) * rb + li]);
+#pragma unroll 4
+        for (int r = q; r < I; r += kSym64Slices) add(spart[sym_soff(r, n, rb) + (i - (long long)(r + 1) * rb)]);
+    }
+    red[0][q][lane] = ax;
+    red[1][q][lane] = ay;
+    red[2][q][lane] = az;
+    red[3][q][lane] = aw;
+    __syncthreads();
+    if (q != 0 || i < 0) return;
+#pragma unroll
+    for (int k = 1; k < kSym64Slices; ++k) {
+        ax = __dadd_rn(ax, red[0][k][lane]);
+        ay = __dadd_rn(ay, red[1][k][lane]);
+        az = __dadd_rn(az, red[2][k][lane]);
+        aw = __dadd_rn(aw, red[3][k][lane]);
     }
     if (ffrange) {
         // float-float path: its sums are in units scaled by 2^kx (positions)
@@ -292,7 +304,7 @@ int sym64_integrate(const SymPlan &p, const double4 *pos_old, double4 *pos_new, 
 {
     if (p.n == 0) return NB_OK;
     if (p.nbands > 1 && !accsum) return set_error(NB_ERR_INVALID, "sym64_integrate: a banded plan needs its per-body sums");
-    sym64_integrate_kernel<<<(p.n + 255) / 256, 256, 0, s>>>(pos_old, pos_new, vel, tpart, spart, p.n, p.rb,
+    sym64_integrate_kernel<<<(p.n + 31) / 32, 32 * kSym64Slices, 0, s>>>(pos_old, pos_new, vel, tpart, spart, p.n, p.rb,
                                                              p.nc, p.nrb, p.total, p.grid, damping, dt, kick,
                                                              G, acc_out, ffrange, p.nbands > 1 ? accsum : nullptr);
     NB_LAUNCH_CHECK("sym64_integrate_kernel launch");
