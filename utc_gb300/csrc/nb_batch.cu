@@ -348,6 +348,69 @@ __global__ void bks_integrate_kernel(const float4 *__restrict__ pos_old, float4 
     batch_kick_drift(i, ax, ay, az, pos_old, pos_new, vel, damping, dt, kick, G, acc_out);
 }
 
+// A warp's share of a row of one system (its bodies from o on): as
+// symff_row_segment of nb_symff.cu, one warp.
+template <int WPB, int BPT>
+__device__ __noinline__ void bksff_row_segment(const float4 *__restrict__ H, const float4 *__restrict__ Mi,
+                                               const float4 *__restrict__ Lo, int o, int ns, float eps_h, float eps_l,
+                                               double4 *dst, double4 *sp, int I, int kc0, int kc1)
+{
+    constexpr int NP = BPT / 2;
+    constexpr int RB = 32 * BPT;
+    constexpr int RC = BPT;
+    __shared__ __align__(16) float4 sHb[WPB][32], sMb[WPB][32], sLb[WPB][32];
+    const int lane = threadIdx.x & 31;
+    const int wid = threadIdx.x >> 5;
+    float4 *sH = sHb[wid], *sM = sMb[wid], *sL = sLb[wid];
+    const int tbase = I * RB;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const f2 eh = ff_pack1(eps_h), el = ff_pack1(eps_l);
+    FFTargets<NP, false> T;
+    T.load(H, Mi, Lo, [&](int k) {
+        const int li = tbase + lane + 32 * k;
+        return li < ns ? o + li : -1;
+    });
+    double ax[BPT], ay[BPT], az[BPT];
+#pragma unroll
+    for (int k = 0; k < BPT; ++k) ax[k] = ay[k] = az[k] = 0.0;
+#pragma unroll 1
+    for (int kc = kc0; kc < kc1; ++kc) {
+        const int jb = kc * 32;
+        const bool in = jb + lane < ns;
+        __syncwarp();  // previous chunk's reads are done
+        // padding: far away (scaled coordinates are below 1), no mass
+        sH[lane] = in ? H[o + jb + lane] : make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f);
+        sM[lane] = in ? Mi[o + jb + lane] : zero;
+        sL[lane] = in ? Lo[o + jb + lane] : zero;
+        __syncwarp();
+        T.clear();
+        if (kc < (I + 1) * RC) {
+            // chunk inside the own row block: directed, target side only
+            ff_chunk_pull(T, sH, sM, sL, eh, el, [](int) { return -1; });
+        } else {
+            FFReact F;
+            ff_chunk_react(T, F, sH, sM, sL, lane, eh, el);
+            // lane l holds the reaction on chunk body l
+            if (in) sp[jb + lane - (I + 1) * RB] = make_double4(F.x.fold(), F.y.fold(), F.z.fold(), 0.0);
+        }
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            double lo, hi;
+            T.ax[p].get(lo, hi);
+            ax[2 * p] += lo;
+            ax[2 * p + 1] += hi;
+            T.ay[p].get(lo, hi);
+            ay[2 * p] += lo;
+            ay[2 * p + 1] += hi;
+            T.az[p].get(lo, hi);
+            az[2 * p] += lo;
+            az[2 * p + 1] += hi;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < BPT; ++k) dst[lane + 32 * k] = make_double4(ax[k], ay[k], az[k], 0.0);
+}
+
 // Float-float batched symmetric kernel for FP64 state: the layout and work
 // split of bks_force_kernel, the pair arithmetic of symff_force_kernel
 // (nb_ff.cuh; grid-split positions scaled by the batch's powers of two),
@@ -360,8 +423,6 @@ __global__ void __launch_bounds__(32 * WPB)
 {
     constexpr int RB = 32 * BPT;
     constexpr int RC = BPT;
-    __shared__ __align__(16) float4 sH[WPB][32], sM[WPB][32], sL[WPB][32];
-    const int lane = threadIdx.x & 31;
     const int wid = threadIdx.x >> 5;
     const int w = blockIdx.x * WPB + wid;
     if (w >= workers) return;
@@ -371,7 +432,6 @@ __global__ void __launch_bounds__(32 * WPB)
     // eps2 in the scaled units (x 2^(2 kx)), as a float-float
     const double e2s = ldexp(eps2, -2 * ff_exponent(range[0]));
     const float eh = __double2float_rn(e2s), el = __double2float_rn(e2s - (double)eh);
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     int s = find_sys(bd.it_off, bd.nsys, it);
     while (it < end) {
         while (it >= bd.it_off[s + 1]) ++s;
@@ -385,93 +445,8 @@ __global__ void __launch_bounds__(32 * WPB)
         const long long seg_end = end < rend ? end : rend;
         const int kc0 = I * RC + (int)(it - rfirst);
         const int kc1 = I * RC + (int)(seg_end - rfirst);
-        const int tbase = I * RB;
-        // missing targets: zero mass, so their reactions are 0; masses
-        // negated: reactions point along -r
-        float pxh[BPT], pxm[BPT], pxl[BPT], pyh[BPT], pym[BPT], pyl[BPT], pzh[BPT], pzm[BPT], pzl[BPT];
-        float nmh[BPT], nml[BPT];
-        double ax[BPT], ay[BPT], az[BPT];
-#pragma unroll
-        for (int k = 0; k < BPT; ++k) {
-            const int li = tbase + lane + 32 * k;
-            const float4 a = li < ns ? H[o + li] : zero;
-            const float4 m = li < ns ? Mi[o + li] : zero;
-            const float4 q = li < ns ? Lo[o + li] : zero;
-            pxh[k] = a.x; pxm[k] = m.x; pxl[k] = q.x;
-            pyh[k] = a.y; pym[k] = m.y; pyl[k] = q.y;
-            pzh[k] = a.z; pzm[k] = m.z; pzl[k] = q.z;
-            nmh[k] = -a.w; nml[k] = -m.w;
-            ax[k] = ay[k] = az[k] = 0.0;
-        }
-        for (int kc = kc0; kc < kc1; ++kc) {
-            const int jb = kc * 32;
-            const bool in = jb + lane < ns;
-            __syncwarp();  // previous chunk's reads are done
-            // padding: far away (scaled coordinates are below 1), no mass
-            sH[wid][lane] = in ? H[o + jb + lane] : make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f);
-            sM[wid][lane] = in ? Mi[o + jb + lane] : zero;
-            sL[wid][lane] = in ? Lo[o + jb + lane] : zero;
-            __syncwarp();
-            float Axh[BPT], Axl[BPT], Ayh[BPT], Ayl[BPT], Azh[BPT], Azl[BPT];
-#pragma unroll
-            for (int k = 0; k < BPT; ++k) Axh[k] = Axl[k] = Ayh[k] = Ayl[k] = Azh[k] = Azl[k] = 0.f;
-            if (kc < (I + 1) * RC) {
-                // chunk inside the own row block: directed, target side only
-#pragma unroll 1
-                for (int j = 0; j < 32; ++j) {
-                    const float4 a = sH[wid][j], am = sM[wid][j], q = sL[wid][j];
-#pragma unroll
-                    for (int k = 0; k < BPT; ++k) {
-                        FFPair f;
-                        ff_pair<false>(a, am, q, pxh[k], pxm[k], pxl[k], pyh[k], pym[k], pyl[k], pzh[k], pzm[k],
-                                       pzl[k], 0.f, 0.f, eh, el, f);
-                        ff_acc(Axh[k], Axl[k], f.rxh, f.rxl, f.wjh, f.wjl);
-                        ff_acc(Ayh[k], Ayl[k], f.ryh, f.ryl, f.wjh, f.wjl);
-                        ff_acc(Azh[k], Azl[k], f.rzh, f.rzl, f.wjh, f.wjl);
-                    }
-                }
-            } else {
-                float Fxh = 0.f, Fxl = 0.f, Fyh = 0.f, Fyl = 0.f, Fzh = 0.f, Fzl = 0.f;
-#pragma unroll 1
-                for (int r = 0; r < 32; ++r) {
-                    const int idx = (lane + r) & 31;
-                    const float4 a = sH[wid][idx], am = sM[wid][idx], q = sL[wid][idx];
-#pragma unroll
-                    for (int k = 0; k < BPT; ++k) {
-                        FFPair f;
-                        ff_pair<true>(a, am, q, pxh[k], pxm[k], pxl[k], pyh[k], pym[k], pyl[k], pzh[k], pzm[k],
-                                      pzl[k], nmh[k], nml[k], eh, el, f);
-                        ff_acc(Axh[k], Axl[k], f.rxh, f.rxl, f.wjh, f.wjl);
-                        ff_acc(Ayh[k], Ayl[k], f.ryh, f.ryl, f.wjh, f.wjl);
-                        ff_acc(Azh[k], Azl[k], f.rzh, f.rzl, f.wjh, f.wjl);
-                        ff_acc(Fxh, Fxl, f.rxh, f.rxl, f.wih, f.wil);
-                        ff_acc(Fyh, Fyl, f.ryh, f.ryl, f.wih, f.wil);
-                        ff_acc(Fzh, Fzl, f.rzh, f.rzl, f.wih, f.wil);
-                    }
-                    const int from = (lane + 1) & 31;
-                    Fxh = __shfl_sync(0xffffffffu, Fxh, from);
-                    Fxl = __shfl_sync(0xffffffffu, Fxl, from);
-                    Fyh = __shfl_sync(0xffffffffu, Fyh, from);
-                    Fyl = __shfl_sync(0xffffffffu, Fyl, from);
-                    Fzh = __shfl_sync(0xffffffffu, Fzh, from);
-                    Fzl = __shfl_sync(0xffffffffu, Fzl, from);
-                }
-                // lane l holds the reaction on chunk body l
-                if (in)
-                    spart[bd.sp_off[s] + sym_soff(I, ns, RB) + (jb + lane - (I + 1) * RB)] =
-                        make_double4((double)Fxh + (double)Fxl, (double)Fyh + (double)Fyl,
-                                     (double)Fzh + (double)Fzl, 0.0);
-            }
-#pragma unroll
-            for (int k = 0; k < BPT; ++k) {
-                ax[k] += (double)Axh[k] + (double)Axl[k];
-                ay[k] += (double)Ayh[k] + (double)Ayl[k];
-                az[k] += (double)Azh[k] + (double)Azl[k];
-            }
-        }
-        double4 *dst = tpart + ((long long)w + bd.row_off[s] + I) * RB;
-#pragma unroll
-        for (int k = 0; k < BPT; ++k) dst[lane + 32 * k] = make_double4(ax[k], ay[k], az[k], 0.0);
+        bksff_row_segment<WPB, BPT>(H, Mi, Lo, o, ns, eh, el, tpart + ((long long)w + bd.row_off[s] + I) * RB,
+                                    spart + bd.sp_off[s] + sym_soff(I, ns, RB), I, kc0, kc1);
         it = seg_end;
     }
 }

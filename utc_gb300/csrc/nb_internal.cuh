@@ -118,6 +118,14 @@ __device__ __forceinline__ void f2_unpack(f2 v, float &lo, float &hi)
 {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
+// -a: negated half by half, which ptxas folds into the operand of the
+// instruction that takes it (an xor of the 64-bit pair costs two of its own)
+__device__ __forceinline__ f2 f2_neg(f2 a)
+{
+    float lo, hi;
+    f2_unpack(a, lo, hi);
+    return f2_pack(-lo, -hi);
+}
 __device__ __forceinline__ f2 f2_sub(f2 a, f2 b)
 {
     f2 r;

@@ -145,8 +145,8 @@ __global__ void __launch_bounds__(32 * W, MINB) sym64_force_kernel(const double4
 // FP64 pipe's additions bound it.  A block takes 32 bodies x 8 slices: slice
 // q sums slots c0 + q, c0 + q + 8, ... and rows q, q + 8, ... in order, and the
 // slices are added in slice order (fixed order: deterministic); the w sums
-// only where they are asked for.  With one thread per body the walk over up
-// to 255 rows was a chain of loads (N = 16384, rb = 64: 84 us a step).
+// only where they are asked for.  With one thread per body the walk over up to
+// 255 rows was a chain of loads (N = 16384, rb = 64: 84 us a step).
 constexpr int kSym64Slices = 8;
 
 __global__ void __launch_bounds__(32 * kSym64Slices)

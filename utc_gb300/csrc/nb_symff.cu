@@ -32,7 +32,7 @@
 //    convergence; the small t keeps the correction's roundings near 2^-47);
 //  * inv^3, the weights m_j inv^3 and m_i inv^3, and the six products with
 //    r in float-float; target and reaction sums in float-float, renormalized
-//    after every term.
+//    every second and fourth step (nb_ff.cuh).
 // Each target's 32-source chunk sum is folded into FP64 accumulators; each
 // reaction (one chunk body, the warp's 32*BPT targets) is written as FP64.
 // The FP64 integrator of nb_sym64.cu then sums the partials in FP64, undoes
@@ -40,9 +40,14 @@
 // (row blocks of 64 bodies: a triangular array of N^2 / 4 bytes), is kept at
 // every size: past N = 185k the array is cut into bands of at most 8 GiB as
 // in nb_sym.cu (symff_fold_kernel folds each band in FP64), which ran 9-22 %
-// faster on GB300 than growing the row block (315 against 288 and 259 G
-// interactions/s at N = 2^19 and 2^20).  196 FP32 operations and one approximation
-// per pair (98 per interaction); results within a few 1e-15 of the FP64
+// faster on GB300 than growing the row block (scalar pair loop: 315 against
+// 288 and 259 G interactions/s at N = 2^19 and 2^20).  185 FP32 operations and
+// one approximation per pair, two pairs per f32x2 instruction (nb_ff.cuh): the
+// FMA pipe is 81 % busy, issue slots half used; what is left are the third
+// operands of some 35 FMAs per pair (register reads, as in nb_pair.cuh).
+// N = 16384: 328 G interactions/s (force and split) against 311 for the scalar
+// loop; N = 65536: 349 against 326; 16 systems x 4096 in a batch: 311 against
+// 272.  Results within a few 1e-15 of the FP64
 // oracle (FP64 arithmetic: a few 1e-16), not bit-identical (NB_ALGO_EXACT is).
 // Range: the scaled squared distances and eps2 must stay normal floats:
 // eps2 >= 2^-100 max|x|^2 and body masses >= 2^-100 of the largest.
@@ -108,8 +113,101 @@ __global__ void ff_split_kernel(const double4 *__restrict__ pos, int n, const un
     L[i] = make_float4(l[0], l[1], l[2], l[3]);
 }
 
+// One CTA's share of a row: row block I's targets against the chunks
+// [kc0, kc1), target-side sums to dst, reactions to spart.  Not inlined into
+// the loop over rows, as sym_row_segment of nb_sym.cu.
 // PHI: also the potential sum_j m_j inv (j != i) in the partials' w, the
 // reaction's included (energy pass).
+template <int W, int BPT, bool PHI>
+__device__ __noinline__ void symff_row_segment(const float4 *__restrict__ H, const float4 *__restrict__ Mi,
+                                               const float4 *__restrict__ Lo, int n, float eps_h, float eps_l,
+                                               double4 *dst, double4 *spart, long long soff, int I, int kc0, int kc1)
+{
+    constexpr int NP = BPT / 2;
+    constexpr int WB = 32 * BPT;
+    constexpr int RB = W * WB;
+    constexpr int RC = RB / 32;
+    __shared__ __align__(16) float4 sH[32], sM[32], sL[32];
+    __shared__ double sF[4][W][32];
+    const int lane = threadIdx.x & 31;
+    const int wid = threadIdx.x >> 5;
+    const int tbase = I * RB + wid * WB;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const f2 eh = ff_pack1(eps_h), el = ff_pack1(eps_l);
+
+    FFTargets<NP, PHI> T;
+    T.load(H, Mi, Lo, [&](int k) {
+        const int i = tbase + lane + 32 * k;
+        return i < n ? i : -1;
+    });
+    double ax[BPT], ay[BPT], az[BPT], aphi[BPT];
+#pragma unroll
+    for (int k = 0; k < BPT; ++k) ax[k] = ay[k] = az[k] = aphi[k] = 0.0;
+#pragma unroll 1
+    for (int kc = kc0; kc < kc1; ++kc) {
+        const int jb = kc * 32;
+        const bool in = jb + lane < n;
+        __syncthreads();  // previous chunk: shared reads are done
+        if (wid == 0) {
+            // padding: far away (scaled coordinates are below 1), no mass
+            sH[lane] = in ? H[jb + lane] : make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f);
+            sM[lane] = in ? Mi[jb + lane] : zero;
+            sL[lane] = in ? Lo[jb + lane] : zero;
+        }
+        __syncthreads();
+        T.clear();
+        if (kc < (I + 1) * RC) {
+            // chunk inside the own row block: directed, target side only
+            ff_chunk_pull(T, sH, sM, sL, eh, el, [&](int k) { return tbase + lane + 32 * k - jb; });
+        } else {
+            FFReact F;
+            ff_chunk_react(T, F, sH, sM, sL, lane, eh, el);
+            // the reaction on chunk body `lane` from this warp
+            double fx = F.x.fold(), fy = F.y.fold(), fz = F.z.fold(), fp = PHI ? F.p.fold() : 0.0;
+            if constexpr (W > 1) {
+                sF[0][wid][lane] = fx;
+                sF[1][wid][lane] = fy;
+                sF[2][wid][lane] = fz;
+                sF[3][wid][lane] = fp;
+                __syncthreads();
+                fx = fy = fz = fp = 0.0;
+                if (wid == 0) {
+#pragma unroll
+                    for (int w = 0; w < W; ++w) {
+                        fx += sF[0][w][lane];
+                        fy += sF[1][w][lane];
+                        fz += sF[2][w][lane];
+                        fp += sF[3][w][lane];
+                    }
+                }
+            }
+            if (wid == 0 && in) spart[soff + (jb + lane - (I + 1) * RB)] = make_double4(fx, fy, fz, fp);
+        }
+        // fold the chunk's sums into FP64
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            double lo, hi;
+            T.ax[p].get(lo, hi);
+            ax[2 * p] += lo;
+            ax[2 * p + 1] += hi;
+            T.ay[p].get(lo, hi);
+            ay[2 * p] += lo;
+            ay[2 * p + 1] += hi;
+            T.az[p].get(lo, hi);
+            az[2 * p] += lo;
+            az[2 * p + 1] += hi;
+            if (PHI) {
+                T.ap[p].get(lo, hi);
+                aphi[2 * p] += lo;
+                aphi[2 * p + 1] += hi;
+            }
+        }
+    }
+    dst += wid * WB + lane;
+#pragma unroll
+    for (int k = 0; k < BPT; ++k) dst[32 * k] = make_double4(ax[k], ay[k], az[k], aphi[k]);
+}
+
 // BAND: one band of a banded plan, as in sym_force_kernel: items
 // [it0, it0 + total) from row block r0 on, target-side slot c + I - r0,
 // source-side entries offset by soff0.
@@ -120,161 +218,26 @@ __global__ void __launch_bounds__(32 * W, MINB)
                        double4 *__restrict__ tpart, double4 *__restrict__ spart, long long total, int nc, int nrb,
                        long long it0, int r0, long long soff0)
 {
-    constexpr int WB = 32 * BPT;
-    constexpr int RB = W * WB;
+    constexpr int RB = W * 32 * BPT;
     constexpr int RC = RB / 32;
-    __shared__ __align__(16) float4 sH[32], sM[32], sL[32];
-    __shared__ double sF[4][W][32];
-    const int lane = threadIdx.x & 31;
-    const int wid = threadIdx.x >> 5;
     const int c = blockIdx.x;
     // eps2 in the scaled units (x 2^(2 kx)), as a float-float
     const double e2s = ldexp(eps2, -2 * ff_exponent(range[0]));
     const float eh = __double2float_rn(e2s), el = __double2float_rn(e2s - (double)eh);
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     long long it = sk_start(c, total, gridDim.x);
     long long end = sk_start(c + 1, total, gridDim.x);
     if constexpr (BAND) {
         it += it0;
         end += it0;
     }
-
     while (it < end) {
         const int I = sym_row_of(it, nc, RC, nrb);
         const long long rfirst = sym_prefix(I, nc, RC);
         const long long rend = sym_prefix(I + 1, nc, RC);
         const long long seg_end = end < rend ? end : rend;
-        const int kc0 = I * RC + (int)(it - rfirst);
-        const int kc1 = I * RC + (int)(seg_end - rfirst);
-        const int tbase = I * RB + wid * WB;
-
-        // missing targets: zero mass, so their reactions are 0; masses
-        // negated: reactions point along -r
-        float pxh[BPT], pxm[BPT], pxl[BPT], pyh[BPT], pym[BPT], pyl[BPT], pzh[BPT], pzm[BPT], pzl[BPT];
-        float nmh[BPT], nml[BPT];
-        double ax[BPT], ay[BPT], az[BPT], aphi[BPT];
-#pragma unroll
-        for (int k = 0; k < BPT; ++k) {
-            const int i = tbase + lane + 32 * k;
-            const float4 a = i < n ? H[i] : zero;
-            const float4 m = i < n ? Mi[i] : zero;
-            const float4 b = i < n ? Lo[i] : zero;
-            pxh[k] = a.x; pxm[k] = m.x; pxl[k] = b.x;
-            pyh[k] = a.y; pym[k] = m.y; pyl[k] = b.y;
-            pzh[k] = a.z; pzm[k] = m.z; pzl[k] = b.z;
-            nmh[k] = -a.w; nml[k] = -m.w;
-            ax[k] = ay[k] = az[k] = aphi[k] = 0.0;
-        }
-        for (int kc = kc0; kc < kc1; ++kc) {
-            const int jb = kc * 32;
-            const bool in = jb + lane < n;
-            __syncthreads();  // previous chunk: shared reads are done
-            if (wid == 0) {
-                // padding: far away (scaled coordinates are below 1), no mass
-                sH[lane] = in ? H[jb + lane] : make_float4(1.0e6f, 1.0e6f, 1.0e6f, 0.f);
-                sM[lane] = in ? Mi[jb + lane] : zero;
-                sL[lane] = in ? Lo[jb + lane] : zero;
-            }
-            __syncthreads();
-            float Axh[BPT], Axl[BPT], Ayh[BPT], Ayl[BPT], Azh[BPT], Azl[BPT], Aph[BPT], Apl[BPT];
-#pragma unroll
-            for (int k = 0; k < BPT; ++k)
-                Axh[k] = Axl[k] = Ayh[k] = Ayl[k] = Azh[k] = Azl[k] = Aph[k] = Apl[k] = 0.f;
-            if (kc < (I + 1) * RC) {
-                // chunk inside the own row block: directed, target side only
-#pragma unroll 1
-                for (int j = 0; j < 32; ++j) {
-                    const float4 a = sH[j], am = sM[j], b = sL[j];
-#pragma unroll
-                    for (int k = 0; k < BPT; ++k) {
-                        FFPair w;
-                        ff_pair<false>(a, am, b, pxh[k], pxm[k], pxl[k], pyh[k], pym[k], pyl[k], pzh[k], pzm[k],
-                                       pzl[k], 0.f, 0.f, eh, el, w);
-                        ff_acc(Axh[k], Axl[k], w.rxh, w.rxl, w.wjh, w.wjl);
-                        ff_acc(Ayh[k], Ayl[k], w.ryh, w.ryl, w.wjh, w.wjl);
-                        ff_acc(Azh[k], Azl[k], w.rzh, w.rzl, w.wjh, w.wjl);
-                        if (PHI && jb + j != tbase + lane + 32 * k) {  // no self term
-                            float vh, vl;
-                            ff_mul(a.w, am.w, w.yh, w.yl, vh, vl);
-                            ff_add(Aph[k], Apl[k], vh, vl);
-                        }
-                    }
-                }
-            } else {
-                float Fxh = 0.f, Fxl = 0.f, Fyh = 0.f, Fyl = 0.f, Fzh = 0.f, Fzl = 0.f, Fph = 0.f, Fpl = 0.f;
-#pragma unroll 1
-                for (int r = 0; r < 32; ++r) {
-                    const int idx = (lane + r) & 31;
-                    const float4 a = sH[idx], am = sM[idx], b = sL[idx];
-#pragma unroll
-                    for (int k = 0; k < BPT; ++k) {
-                        FFPair w;
-                        ff_pair<true>(a, am, b, pxh[k], pxm[k], pxl[k], pyh[k], pym[k], pyl[k], pzh[k], pzm[k],
-                                      pzl[k], nmh[k], nml[k], eh, el, w);
-                        ff_acc(Axh[k], Axl[k], w.rxh, w.rxl, w.wjh, w.wjl);
-                        ff_acc(Ayh[k], Ayl[k], w.ryh, w.ryl, w.wjh, w.wjl);
-                        ff_acc(Azh[k], Azl[k], w.rzh, w.rzl, w.wjh, w.wjl);
-                        ff_acc(Fxh, Fxl, w.rxh, w.rxl, w.wih, w.wil);
-                        ff_acc(Fyh, Fyl, w.ryh, w.ryl, w.wih, w.wil);
-                        ff_acc(Fzh, Fzl, w.rzh, w.rzl, w.wih, w.wil);
-                        if (PHI) {
-                            float vh, vl;
-                            ff_mul(a.w, am.w, w.yh, w.yl, vh, vl);
-                            ff_add(Aph[k], Apl[k], vh, vl);
-                            ff_mul(-nmh[k], -nml[k], w.yh, w.yl, vh, vl);
-                            ff_add(Fph, Fpl, vh, vl);
-                        }
-                    }
-                    const int from = (lane + 1) & 31;
-                    Fxh = __shfl_sync(0xffffffffu, Fxh, from);
-                    Fxl = __shfl_sync(0xffffffffu, Fxl, from);
-                    Fyh = __shfl_sync(0xffffffffu, Fyh, from);
-                    Fyl = __shfl_sync(0xffffffffu, Fyl, from);
-                    Fzh = __shfl_sync(0xffffffffu, Fzh, from);
-                    Fzl = __shfl_sync(0xffffffffu, Fzl, from);
-                    if (PHI) {
-                        Fph = __shfl_sync(0xffffffffu, Fph, from);
-                        Fpl = __shfl_sync(0xffffffffu, Fpl, from);
-                    }
-                }
-                // lane l now holds the reaction on chunk body l from this warp
-                const double fx = (double)Fxh + (double)Fxl, fy = (double)Fyh + (double)Fyl,
-                             fz = (double)Fzh + (double)Fzl, fp = PHI ? (double)Fph + (double)Fpl : 0.0;
-                long long so = sym_soff(I, n, RB) + (jb + lane - (I + 1) * RB);
-                if constexpr (BAND) so -= soff0;
-                if (W == 1) {
-                    if (in) spart[so] = make_double4(fx, fy, fz, fp);
-                } else {
-                    sF[0][wid][lane] = fx;
-                    sF[1][wid][lane] = fy;
-                    sF[2][wid][lane] = fz;
-                    sF[3][wid][lane] = fp;
-                    __syncthreads();
-                    if (wid == 0 && in) {
-                        double sx = 0.0, sy = 0.0, sz = 0.0, sp = 0.0;
-#pragma unroll
-                        for (int w = 0; w < W; ++w) {
-                            sx += sF[0][w][lane];
-                            sy += sF[1][w][lane];
-                            sz += sF[2][w][lane];
-                            sp += sF[3][w][lane];
-                        }
-                        spart[so] = make_double4(sx, sy, sz, sp);
-                    }
-                }
-            }
-            // fold the chunk's sums into FP64
-#pragma unroll
-            for (int k = 0; k < BPT; ++k) {
-                ax[k] += (double)Axh[k] + (double)Axl[k];
-                ay[k] += (double)Ayh[k] + (double)Ayl[k];
-                az[k] += (double)Azh[k] + (double)Azl[k];
-                if (PHI) aphi[k] += (double)Aph[k] + (double)Apl[k];
-            }
-        }
-        double4 *dst = tpart + (size_t)(c + I - (BAND ? r0 : 0)) * RB + wid * WB;
-#pragma unroll
-        for (int k = 0; k < BPT; ++k) dst[lane + 32 * k] = make_double4(ax[k], ay[k], az[k], aphi[k]);
+        symff_row_segment<W, BPT, PHI>(H, Mi, Lo, n, eh, el, tpart + (size_t)(c + I - (BAND ? r0 : 0)) * RB, spart,
+                                       sym_soff(I, n, RB) - (BAND ? soff0 : 0), I, I * RC + (int)(it - rfirst),
+                                       I * RC + (int)(seg_end - rfirst));
         it = seg_end;
     }
 }
