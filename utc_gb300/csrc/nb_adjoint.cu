@@ -26,7 +26,7 @@
 // chunks, the chunk rotating through the warp with its accumulated reaction):
 // 18 shared operations + 8 per side = 34 FP32 operations and one rsqrt per
 // pair, 17 per ordered interaction instead of 26.
-#include "nb_internal.cuh"
+#include "nb_vjp.cuh"
 
 namespace nb {
 
@@ -120,13 +120,14 @@ __global__ void __launch_bounds__(NT) vjp_pair_kernel(const float4 *__restrict__
     }
 }
 
-template <int W, int BPT, int MINB, int U = 2>
-__global__ void __launch_bounds__(32 * W, MINB) sym_vjp_kernel(const float4 *__restrict__ pos,
-                                                               const float4 *__restrict__ gbuf, int n,
-                                                               float eps2, float4 *__restrict__ tpart,
-                                                               float4 *__restrict__ spart,
-                                                               long long total, int nc, int nrb)
+// One CTA's share of a row: row block I's targets against the chunks
+// [kc0, kc1), target-side sums to dst, reactions to sp.  Not inlined into the
+// loop over rows, as sym_row_segment of nb_sym.cu.
+template <int W, int BPT>
+__device__ __noinline__ void sym_vjp_segment(const float4 *__restrict__ pos, const float4 *__restrict__ gbuf, int n,
+                                             float eps2, float4 *dst, float4 *sp, int I, int kc0, int kc1)
 {
+    constexpr int NP = BPT / 2;
     constexpr int WB = 32 * BPT;
     constexpr int RB = W * WB;
     constexpr int RC = RB / 32;
@@ -135,162 +136,80 @@ __global__ void __launch_bounds__(32 * W, MINB) sym_vjp_kernel(const float4 *__r
     __shared__ float sF[8][W][32];
     const int lane = threadIdx.x & 31;
     const int wid = threadIdx.x >> 5;
+    const int tbase = I * RB + wid * WB;
+    const float4 pad = make_float4(kPadCoord, kPadCoord, kPadCoord, 0.f);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const f2 EPS2 = f2_pack(eps2, eps2);
+
+    VjpTargets<NP> T;
+    auto idx = [&](int t) { return tbase + lane + 32 * t; };
+    T.load([&](int t) { return idx(t) < n ? pos[idx(t)] : zero; }, [&](int t) { return idx(t) < n ? gbuf[idx(t)] : zero; });
+    // the next chunk is read ahead
+    float4 nxc = kc0 * 32 + lane < n ? pos[kc0 * 32 + lane] : pad;
+    float4 nxg = kc0 * 32 + lane < n ? gbuf[kc0 * 32 + lane] : zero;
+#pragma unroll 1
+    for (int kc = kc0; kc < kc1; ++kc) {
+        const int jb = kc * 32;
+        __syncthreads();  // previous chunk: sC/sG and sF reads are done
+        if (wid == 0) {
+            sC[lane] = nxc;
+            sG[lane] = nxg;
+        }
+        __syncthreads();
+        if (wid == 0) {
+            nxc = jb + 32 + lane < n ? pos[jb + 32 + lane] : pad;
+            nxg = jb + 32 + lane < n ? gbuf[jb + 32 + lane] : zero;
+        }
+        if (kc < (I + 1) * RC) {
+            vjp_chunk_pull(T, sC, sG, EPS2);  // chunk inside the own row block: target side only
+            continue;
+        }
+        float r8[8];
+        vjp_chunk_react(T, sC, sG, lane, EPS2, r8);
+        if constexpr (W > 1) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) sF[k][wid][lane] = r8[k];
+            __syncthreads();
+            if (wid == 0) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    r8[k] = 0.f;
+#pragma unroll
+                    for (int w = 0; w < W; ++w) r8[k] += sF[k][w][lane];
+                }
+            }
+        }
+        if (wid == 0 && jb + lane < n) sp[jb + lane - (I + 1) * RB] = vjp_reaction(sC[lane], sG[lane], r8);
+    }
+    dst += wid * WB + lane;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        float4 a, b;
+        T.out(p, a, b);
+        dst[64 * p] = a;
+        dst[64 * p + 32] = b;
+    }
+}
+
+template <int W, int BPT, int MINB>
+__global__ void __launch_bounds__(32 * W, MINB) sym_vjp_kernel(const float4 *__restrict__ pos,
+                                                               const float4 *__restrict__ gbuf, int n,
+                                                               float eps2, float4 *__restrict__ tpart,
+                                                               float4 *__restrict__ spart,
+                                                               long long total, int nc, int nrb)
+{
+    constexpr int RB = W * 32 * BPT;
+    constexpr int RC = RB / 32;
     const int c = blockIdx.x;
     long long it = sk_start(c, total, gridDim.x);
     const long long end = sk_start(c + 1, total, gridDim.x);
-    const float4 pad = make_float4(kPadCoord, kPadCoord, kPadCoord, 0.f);
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-
     while (it < end) {
         const int I = sym_row_of(it, nc, RC, nrb);
         const long long rfirst = sym_prefix(I, nc, RC);
         const long long rend = sym_prefix(I + 1, nc, RC);
         const long long seg_end = end < rend ? end : rend;
-        const int kc0 = I * RC + (int)(it - rfirst);
-        const int kc1 = I * RC + (int)(seg_end - rfirst);
-        const int tbase = I * RB + wid * WB;
-
-        // missing targets: zero mass and zero g, so every term they give is 0
-        float px[BPT], py[BPT], pz[BPT], pm[BPT], gx[BPT], gy[BPT], gz[BPT];
-        float Px[BPT], Py[BPT], Pz[BPT], Q0[BPT], Q1[BPT], Q2[BPT], q[BPT], dm[BPT];
-#pragma unroll
-        for (int k = 0; k < BPT; ++k) {
-            const int i = tbase + lane + 32 * k;
-            const float4 a = i < n ? pos[i] : zero;
-            const float4 g = i < n ? gbuf[i] : zero;
-            px[k] = a.x; py[k] = a.y; pz[k] = a.z; pm[k] = a.w;
-            gx[k] = g.x; gy[k] = g.y; gz[k] = g.z;
-            Px[k] = Py[k] = Pz[k] = Q0[k] = Q1[k] = Q2[k] = q[k] = dm[k] = 0.f;
-        }
-        for (int kc = kc0; kc < kc1; ++kc) {
-            const int jb = kc * 32;
-            __syncthreads();  // previous chunk: sC/sG and sF reads are done
-            if (wid == 0) {
-                sC[lane] = (jb + lane < n) ? pos[jb + lane] : pad;
-                sG[lane] = (jb + lane < n) ? gbuf[jb + lane] : zero;
-            }
-            __syncthreads();
-            if (kc < (I + 1) * RC) {
-                // chunk inside the own row block: directed, target side only
-#pragma unroll 2
-                for (int j = 0; j < 32; ++j) {
-                    const float4 s = sC[j];
-                    const float4 g = sG[j];
-#pragma unroll
-                    for (int k = 0; k < BPT; ++k) {
-                        const float rx = s.x - px[k], ry = s.y - py[k], rz = s.z - pz[k];
-                        float d2 = fmaf(rx, rx, eps2);
-                        d2 = fmaf(ry, ry, d2);
-                        d2 = fmaf(rz, rz, d2);
-                        const float inv = rsqrt_approx(d2);
-                        const float inv2 = inv * inv;
-                        const float inv3 = inv2 * inv;
-                        const float inv5 = inv3 * inv2;
-                        Px[k] = fmaf(inv3, g.x, Px[k]);
-                        Py[k] = fmaf(inv3, g.y, Py[k]);
-                        Pz[k] = fmaf(inv3, g.z, Pz[k]);
-                        q[k] = fmaf(inv3, s.w, q[k]);
-                        const float rgj = fmaf(rz, g.z, fmaf(ry, g.y, rx * g.x));
-                        const float rgk = fmaf(rz, gz[k], fmaf(ry, gy[k], rx * gx[k]));
-                        const float cc = inv5 * fmaf(pm[k], rgj, -(s.w * rgk));
-                        Q0[k] = fmaf(cc, rx, Q0[k]);
-                        Q1[k] = fmaf(cc, ry, Q1[k]);
-                        Q2[k] = fmaf(cc, rz, Q2[k]);
-                        dm[k] = fmaf(inv3, rgj, dm[k]);
-                    }
-                }
-            } else {
-                // reaction on the rotating chunk body: P, q, Q of its own sum
-                // and its mass gradient w = sum inv^3 r.g_k
-                float rPx = 0.f, rPy = 0.f, rPz = 0.f, rq = 0.f, rQ0 = 0.f, rQ1 = 0.f, rQ2 = 0.f, rw = 0.f;
-#pragma unroll(U)
-                for (int r = 0; r < 32; ++r) {
-                    const int idx = (lane + r) & 31;
-                    const float4 s = sC[idx];
-                    const float4 g = sG[idx];
-#pragma unroll
-                    for (int k = 0; k < BPT; ++k) {
-                        const float rx = s.x - px[k], ry = s.y - py[k], rz = s.z - pz[k];
-                        float d2 = fmaf(rx, rx, eps2);
-                        d2 = fmaf(ry, ry, d2);
-                        d2 = fmaf(rz, rz, d2);
-                        const float inv = rsqrt_approx(d2);
-                        const float inv2 = inv * inv;
-                        const float inv3 = inv2 * inv;
-                        const float inv5 = inv3 * inv2;
-                        const float rgj = fmaf(rz, g.z, fmaf(ry, g.y, rx * g.x));
-                        const float rgk = fmaf(rz, gz[k], fmaf(ry, gy[k], rx * gx[k]));
-                        const float cc = inv5 * fmaf(pm[k], rgj, -(s.w * rgk));
-                        Px[k] = fmaf(inv3, g.x, Px[k]);
-                        Py[k] = fmaf(inv3, g.y, Py[k]);
-                        Pz[k] = fmaf(inv3, g.z, Pz[k]);
-                        q[k] = fmaf(inv3, s.w, q[k]);
-                        Q0[k] = fmaf(cc, rx, Q0[k]);
-                        Q1[k] = fmaf(cc, ry, Q1[k]);
-                        Q2[k] = fmaf(cc, rz, Q2[k]);
-                        dm[k] = fmaf(inv3, rgj, dm[k]);
-                        rPx = fmaf(inv3, gx[k], rPx);
-                        rPy = fmaf(inv3, gy[k], rPy);
-                        rPz = fmaf(inv3, gz[k], rPz);
-                        rq = fmaf(inv3, pm[k], rq);
-                        rQ0 = fmaf(-cc, rx, rQ0);
-                        rQ1 = fmaf(-cc, ry, rQ1);
-                        rQ2 = fmaf(-cc, rz, rQ2);
-                        rw = fmaf(inv3, rgk, rw);
-                    }
-                    const int from = (lane + 1) & 31;
-                    rPx = __shfl_sync(0xffffffffu, rPx, from);
-                    rPy = __shfl_sync(0xffffffffu, rPy, from);
-                    rPz = __shfl_sync(0xffffffffu, rPz, from);
-                    rq = __shfl_sync(0xffffffffu, rq, from);
-                    rQ0 = __shfl_sync(0xffffffffu, rQ0, from);
-                    rQ1 = __shfl_sync(0xffffffffu, rQ1, from);
-                    rQ2 = __shfl_sync(0xffffffffu, rQ2, from);
-                    rw = __shfl_sync(0xffffffffu, rw, from);
-                }
-                // lane l now holds chunk body l's reaction from this warp
-                if (W > 1) {
-                    sF[0][wid][lane] = rPx;
-                    sF[1][wid][lane] = rPy;
-                    sF[2][wid][lane] = rPz;
-                    sF[3][wid][lane] = rq;
-                    sF[4][wid][lane] = rQ0;
-                    sF[5][wid][lane] = rQ1;
-                    sF[6][wid][lane] = rQ2;
-                    sF[7][wid][lane] = rw;
-                    __syncthreads();
-                    if (wid == 0) {
-                        rPx = rPy = rPz = rq = rQ0 = rQ1 = rQ2 = rw = 0.f;
-#pragma unroll
-                        for (int w = 0; w < W; ++w) {
-                            rPx += sF[0][w][lane];
-                            rPy += sF[1][w][lane];
-                            rPz += sF[2][w][lane];
-                            rq += sF[3][w][lane];
-                            rQ0 += sF[4][w][lane];
-                            rQ1 += sF[5][w][lane];
-                            rQ2 += sF[6][w][lane];
-                            rw += sF[7][w][lane];
-                        }
-                    }
-                }
-                if (wid == 0 && jb + lane < n) {
-                    const float4 sb = sC[lane], gb = sG[lane];
-                    const float ox = fmaf(sb.w, rPx, fmaf(-rq, gb.x, -3.f * rQ0));
-                    const float oy = fmaf(sb.w, rPy, fmaf(-rq, gb.y, -3.f * rQ1));
-                    const float oz = fmaf(sb.w, rPz, fmaf(-rq, gb.z, -3.f * rQ2));
-                    spart[sym_soff(I, n, RB) + (jb + lane - (I + 1) * RB)] = make_float4(ox, oy, oz, rw);
-                }
-            }
-        }
-        float4 *dst = tpart + (size_t)(c + I) * RB + wid * WB;
-#pragma unroll
-        for (int k = 0; k < BPT; ++k) {
-            const float ox = fmaf(pm[k], Px[k], fmaf(-q[k], gx[k], -3.f * Q0[k]));
-            const float oy = fmaf(pm[k], Py[k], fmaf(-q[k], gy[k], -3.f * Q1[k]));
-            const float oz = fmaf(pm[k], Pz[k], fmaf(-q[k], gz[k], -3.f * Q2[k]));
-            dst[lane + 32 * k] = make_float4(ox, oy, oz, -dm[k]);
-        }
+        sym_vjp_segment<W, BPT>(pos, gbuf, n, eps2, tpart + (size_t)(c + I) * RB, spart + sym_soff(I, n, RB), I,
+                                I * RC + (int)(it - rfirst), I * RC + (int)(seg_end - rfirst));
         it = seg_end;
     }
 }
