@@ -38,7 +38,7 @@
 #include <vector>
 
 #include "nb_ff.cuh"
-#include "nb_internal.cuh"
+#include "nb_vjp.cuh"
 
 namespace nb {
 
@@ -201,23 +201,63 @@ struct BatchSymDev {
     int nsys;
 };
 
+// A warp's share of a row of one system (its bodies at pos): row block I's
+// targets against the chunks [kc0, kc1), target-side sums to dst, reactions to
+// sp.  As sym_row_segment of nb_sym.cu, and like it not inlined.
 template <int WPB, int BPT>
-__global__ void __launch_bounds__(32 * WPB) bks_force_kernel(const float4 *__restrict__ pos, BatchSymDev bd,
+__device__ __noinline__ void bks_row_segment(const float4 *__restrict__ pos, int ns, float eps2, float4 *dst,
+                                             float4 *sp, int I, int kc0, int kc1)
+{
+    constexpr int RB = 32 * BPT;
+    constexpr int RC = BPT;
+    __shared__ __align__(16) float4 sCb[WPB][32];
+    const int lane = WPB == 1 ? threadIdx.x : threadIdx.x & 31;
+    float4 *sC = sCb[WPB == 1 ? 0 : threadIdx.x >> 5];
+    const int tbase = I * RB;
+    const float4 pad = make_float4(kPadCoord, kPadCoord, kPadCoord, 0.f);
+    const f2 EPS2 = f2_pack(eps2, eps2);
+    PairTargets<BPT / 2> T;
+    T.load([&](int t) {
+        const int li = tbase + lane + 32 * t;
+        return li < ns ? pos[li] : make_float4(0.f, 0.f, 0.f, 0.f);
+    });
+    float4 nxt = kc0 * 32 + lane < ns ? pos[kc0 * 32 + lane] : pad;
+#pragma unroll 1
+    for (int kc = kc0; kc < kc1; ++kc) {
+        const int jb = kc * 32;
+        __syncwarp();  // previous chunk's reads are done
+        sC[lane] = nxt;
+        __syncwarp();
+        nxt = jb + 32 + lane < ns ? pos[jb + 32 + lane] : pad;
+        if (kc < (I + 1) * RC) {
+            chunk_pull(T, sC, EPS2);  // chunk inside the own row block: target side only
+        } else {
+            const float3 f = chunk_react(T, sC, lane, EPS2);
+            if (jb + lane < ns) sp[jb + lane - (I + 1) * RB] = make_float4(f.x, f.y, f.z, 0.f);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < BPT; ++t) dst[lane + 32 * t] = T.sum(t);
+}
+
+// Eight warps an SM are asked for, so that a lane may keep up to 255 registers
+// (without that ptxas held 16 targets to 168 and spilled the schedule: 4246
+// against 3821 us a step on 512 systems, N in [128, 16384]).  Step time of
+// the scalar loop that this replaces: 4341 us with 12 targets per lane, 4409
+// with 16; now 3828 and 3821.
+template <int WPB, int BPT>
+__global__ void __launch_bounds__(32 * WPB, 8 / WPB) bks_force_kernel(const float4 *__restrict__ pos, BatchSymDev bd,
                                                              float eps2, float4 *__restrict__ tpart,
                                                              float4 *__restrict__ spart, long long total,
                                                              int workers)
 {
     constexpr int RB = 32 * BPT;
     constexpr int RC = BPT;
-    __shared__ __align__(16) float4 sC[WPB][32];
-    const int lane = threadIdx.x & 31;
-    const int wid = threadIdx.x >> 5;
-    const int w = blockIdx.x * WPB + wid;
+    const int w = blockIdx.x * WPB + (threadIdx.x >> 5);
     if (w >= workers) return;
     long long it = sk_start(w, total, workers);
     const long long end = sk_start(w + 1, total, workers);
     if (it >= end) return;
-    const float4 pad = make_float4(kPadCoord, kPadCoord, kPadCoord, 0.f);
     int s = find_sys(bd.it_off, bd.nsys, it);
     while (it < end) {
         while (it >= bd.it_off[s + 1]) ++s;
@@ -229,81 +269,9 @@ __global__ void __launch_bounds__(32 * WPB) bks_force_kernel(const float4 *__res
         const long long rfirst = base + sym_prefix(I, nc, RC);
         const long long rend = base + sym_prefix(I + 1, nc, RC);
         const long long seg_end = end < rend ? end : rend;
-        const int kc0 = I * RC + (int)(it - rfirst);
-        const int kc1 = I * RC + (int)(seg_end - rfirst);
-        const int tbase = I * RB;
-
-        float px[BPT], py[BPT], pz[BPT], nm[BPT], ax[BPT], ay[BPT], az[BPT];
-#pragma unroll
-        for (int k = 0; k < BPT; ++k) {
-            const int li = tbase + lane + 32 * k;
-            // missing targets get zero mass: their reactions on the chunk are 0
-            const float4 q = li < ns ? pos[o + li] : make_float4(0.f, 0.f, 0.f, 0.f);
-            px[k] = q.x;
-            py[k] = q.y;
-            pz[k] = q.z;
-            nm[k] = -q.w;
-            ax[k] = ay[k] = az[k] = 0.f;
-        }
-        for (int kc = kc0; kc < kc1; ++kc) {
-            const int jb = kc * 32;
-            __syncwarp();  // previous chunk's reads are done
-            sC[wid][lane] = (jb + lane < ns) ? pos[o + jb + lane] : pad;
-            __syncwarp();
-            if (kc < (I + 1) * RC) {
-                // chunk inside the own row block: directed, target side only
-#pragma unroll 4
-                for (int j = 0; j < 32; ++j) {
-                    const float4 q = sC[wid][j];
-#pragma unroll
-                    for (int k = 0; k < BPT; ++k) {
-                        const float rx = q.x - px[k], ry = q.y - py[k], rz = q.z - pz[k];
-                        float d2 = fmaf(rx, rx, eps2);
-                        d2 = fmaf(ry, ry, d2);
-                        d2 = fmaf(rz, rz, d2);
-                        const float inv = rsqrt_approx(d2);
-                        const float sc = (q.w * inv) * (inv * inv);
-                        ax[k] = fmaf(rx, sc, ax[k]);
-                        ay[k] = fmaf(ry, sc, ay[k]);
-                        az[k] = fmaf(rz, sc, az[k]);
-                    }
-                }
-            } else {
-                float fx = 0.f, fy = 0.f, fz = 0.f;
-#pragma unroll 2
-                for (int r = 0; r < 32; ++r) {
-                    const float4 q = sC[wid][(lane + r) & 31];
-#pragma unroll
-                    for (int k = 0; k < BPT; ++k) {
-                        const float rx = q.x - px[k], ry = q.y - py[k], rz = q.z - pz[k];
-                        float d2 = fmaf(rx, rx, eps2);
-                        d2 = fmaf(ry, ry, d2);
-                        d2 = fmaf(rz, rz, d2);
-                        const float inv = rsqrt_approx(d2);
-                        const float inv3 = inv * (inv * inv);
-                        const float st = q.w * inv3;
-                        const float ss = nm[k] * inv3;
-                        ax[k] = fmaf(rx, st, ax[k]);
-                        ay[k] = fmaf(ry, st, ay[k]);
-                        az[k] = fmaf(rz, st, az[k]);
-                        fx = fmaf(rx, ss, fx);
-                        fy = fmaf(ry, ss, fy);
-                        fz = fmaf(rz, ss, fz);
-                    }
-                    const int from = (lane + 1) & 31;
-                    fx = __shfl_sync(0xffffffffu, fx, from);
-                    fy = __shfl_sync(0xffffffffu, fy, from);
-                    fz = __shfl_sync(0xffffffffu, fz, from);
-                }
-                // lane l holds the reaction on chunk body l
-                if (jb + lane < ns)
-                    spart[bd.sp_off[s] + sym_soff(I, ns, RB) + (jb + lane - (I + 1) * RB)] =
-                        make_float4(fx, fy, fz, 0.f);
-            }
-        }
-        float4 *dst = tpart + ((long long)w + bd.row_off[s] + I) * RB;
-#pragma unroll
-        for (int k = 0; k < BPT; ++k) dst[lane + 32 * k] = make_float4(ax[k], ay[k], az[k], 0.f);
+        bks_row_segment<WPB, BPT>(pos + o, ns, eps2, tpart + ((long long)w + bd.row_off[s] + I) * RB,
+                                  spart + bd.sp_off[s] + sym_soff(I, ns, RB), I, I * RC + (int)(it - rfirst),
+                                  I * RC + (int)(seg_end - rfirst));
         it = seg_end;
     }
 }
@@ -359,8 +327,8 @@ __device__ __noinline__ void bksff_row_segment(const float4 *__restrict__ H, con
     constexpr int RB = 32 * BPT;
     constexpr int RC = BPT;
     __shared__ __align__(16) float4 sHb[WPB][32], sMb[WPB][32], sLb[WPB][32];
-    const int lane = threadIdx.x & 31;
-    const int wid = threadIdx.x >> 5;
+    const int lane = WPB == 1 ? threadIdx.x : threadIdx.x & 31;
+    const int wid = WPB == 1 ? 0 : threadIdx.x >> 5;
     float4 *sH = sHb[wid], *sM = sMb[wid], *sL = sLb[wid];
     const int tbase = I * RB;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -672,7 +640,57 @@ __global__ void bk_adj_update_kernel(const float4 *__restrict__ partial, BatchDe
 // unordered pair once, the chunk body's eight reaction sums rotating through
 // the warp) on the symmetric batched layout of bks_force_kernel.
 template <int WPB, int BPT>
-__global__ void __launch_bounds__(32 * WPB) bks_vjp_kernel(const float4 *__restrict__ pos,
+__device__ __noinline__ void bks_vjp_segment(const float4 *__restrict__ pos, const float4 *__restrict__ gbuf, int ns,
+                                             float eps2, float4 *dst, float4 *sp, int I, int kc0, int kc1)
+{
+    constexpr int NP = BPT / 2;
+    constexpr int RB = 32 * BPT;
+    constexpr int RC = BPT;
+    __shared__ __align__(16) float4 sCb[WPB][32];
+    __shared__ __align__(16) float4 sGb[WPB][32];
+    const int lane = WPB == 1 ? threadIdx.x : threadIdx.x & 31;
+    const int wid = WPB == 1 ? 0 : threadIdx.x >> 5;
+    float4 *sC = sCb[wid], *sG = sGb[wid];
+    const int tbase = I * RB;
+    const float4 pad = make_float4(kPadCoord, kPadCoord, kPadCoord, 0.f);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const f2 EPS2 = f2_pack(eps2, eps2);
+
+    VjpTargets<NP> T;
+    auto idx = [&](int t) { return tbase + lane + 32 * t; };
+    T.load([&](int t) { return idx(t) < ns ? pos[idx(t)] : zero; },
+           [&](int t) { return idx(t) < ns ? gbuf[idx(t)] : zero; });
+    float4 nxc = kc0 * 32 + lane < ns ? pos[kc0 * 32 + lane] : pad;
+    float4 nxg = kc0 * 32 + lane < ns ? gbuf[kc0 * 32 + lane] : zero;
+#pragma unroll 1
+    for (int kc = kc0; kc < kc1; ++kc) {
+        const int jb = kc * 32;
+        __syncwarp();  // previous chunk's reads are done
+        sC[lane] = nxc;
+        sG[lane] = nxg;
+        __syncwarp();
+        nxc = jb + 32 + lane < ns ? pos[jb + 32 + lane] : pad;
+        nxg = jb + 32 + lane < ns ? gbuf[jb + 32 + lane] : zero;
+        if (kc < (I + 1) * RC) {
+            vjp_chunk_pull(T, sC, sG, EPS2);  // chunk inside the own row block: target side only
+        } else {
+            float r8[8];
+            vjp_chunk_react(T, sC, sG, lane, EPS2, r8);
+            if (jb + lane < ns) sp[jb + lane - (I + 1) * RB] = vjp_reaction(sC[lane], sG[lane], r8);
+        }
+    }
+    dst += lane;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        float4 a, b;
+        T.out(p, a, b);
+        dst[64 * p] = a;
+        dst[64 * p + 32] = b;
+    }
+}
+
+template <int WPB, int BPT>
+__global__ void __launch_bounds__(32 * WPB, 8 / WPB) bks_vjp_kernel(const float4 *__restrict__ pos,
                                                            const float4 *__restrict__ gbuf, BatchSymDev bd,
                                                            float eps2, float4 *__restrict__ tpart,
                                                            float4 *__restrict__ spart, long long total,
@@ -680,17 +698,11 @@ __global__ void __launch_bounds__(32 * WPB) bks_vjp_kernel(const float4 *__restr
 {
     constexpr int RB = 32 * BPT;
     constexpr int RC = BPT;
-    __shared__ __align__(16) float4 sC[WPB][32];
-    __shared__ __align__(16) float4 sG[WPB][32];
-    const int lane = threadIdx.x & 31;
-    const int wid = threadIdx.x >> 5;
-    const int w = blockIdx.x * WPB + wid;
+    const int w = blockIdx.x * WPB + (threadIdx.x >> 5);
     if (w >= workers) return;
     long long it = sk_start(w, total, workers);
     const long long end = sk_start(w + 1, total, workers);
     if (it >= end) return;
-    const float4 pad = make_float4(kPadCoord, kPadCoord, kPadCoord, 0.f);
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     int s = find_sys(bd.it_off, bd.nsys, it);
     while (it < end) {
         while (it >= bd.it_off[s + 1]) ++s;
@@ -702,123 +714,9 @@ __global__ void __launch_bounds__(32 * WPB) bks_vjp_kernel(const float4 *__restr
         const long long rfirst = base + sym_prefix(I, nc, RC);
         const long long rend = base + sym_prefix(I + 1, nc, RC);
         const long long seg_end = end < rend ? end : rend;
-        const int kc0 = I * RC + (int)(it - rfirst);
-        const int kc1 = I * RC + (int)(seg_end - rfirst);
-        const int tbase = I * RB;
-
-        // missing targets: zero mass and zero g, so every term they give is 0
-        float px[BPT], py[BPT], pz[BPT], pm[BPT], gx[BPT], gy[BPT], gz[BPT];
-        float Px[BPT], Py[BPT], Pz[BPT], Q0[BPT], Q1[BPT], Q2[BPT], q[BPT], dm[BPT];
-#pragma unroll
-        for (int k = 0; k < BPT; ++k) {
-            const int li = tbase + lane + 32 * k;
-            const float4 a = li < ns ? pos[o + li] : zero;
-            const float4 g = li < ns ? gbuf[o + li] : zero;
-            px[k] = a.x; py[k] = a.y; pz[k] = a.z; pm[k] = a.w;
-            gx[k] = g.x; gy[k] = g.y; gz[k] = g.z;
-            Px[k] = Py[k] = Pz[k] = Q0[k] = Q1[k] = Q2[k] = q[k] = dm[k] = 0.f;
-        }
-        for (int kc = kc0; kc < kc1; ++kc) {
-            const int jb = kc * 32;
-            __syncwarp();  // previous chunk's reads are done
-            sC[wid][lane] = (jb + lane < ns) ? pos[o + jb + lane] : pad;
-            sG[wid][lane] = (jb + lane < ns) ? gbuf[o + jb + lane] : zero;
-            __syncwarp();
-            if (kc < (I + 1) * RC) {
-                // chunk inside the own row block: directed, target side only
-#pragma unroll 2
-                for (int j = 0; j < 32; ++j) {
-                    const float4 sb = sC[wid][j];
-                    const float4 g = sG[wid][j];
-#pragma unroll
-                    for (int k = 0; k < BPT; ++k) {
-                        const float rx = sb.x - px[k], ry = sb.y - py[k], rz = sb.z - pz[k];
-                        float d2 = fmaf(rx, rx, eps2);
-                        d2 = fmaf(ry, ry, d2);
-                        d2 = fmaf(rz, rz, d2);
-                        const float inv = rsqrt_approx(d2);
-                        const float inv2 = inv * inv;
-                        const float inv3 = inv2 * inv;
-                        const float inv5 = inv3 * inv2;
-                        Px[k] = fmaf(inv3, g.x, Px[k]);
-                        Py[k] = fmaf(inv3, g.y, Py[k]);
-                        Pz[k] = fmaf(inv3, g.z, Pz[k]);
-                        q[k] = fmaf(inv3, sb.w, q[k]);
-                        const float rgj = fmaf(rz, g.z, fmaf(ry, g.y, rx * g.x));
-                        const float rgk = fmaf(rz, gz[k], fmaf(ry, gy[k], rx * gx[k]));
-                        const float cc = inv5 * fmaf(pm[k], rgj, -(sb.w * rgk));
-                        Q0[k] = fmaf(cc, rx, Q0[k]);
-                        Q1[k] = fmaf(cc, ry, Q1[k]);
-                        Q2[k] = fmaf(cc, rz, Q2[k]);
-                        dm[k] = fmaf(inv3, rgj, dm[k]);
-                    }
-                }
-            } else {
-                float rPx = 0.f, rPy = 0.f, rPz = 0.f, rq = 0.f, rQ0 = 0.f, rQ1 = 0.f, rQ2 = 0.f, rw = 0.f;
-#pragma unroll 2
-                for (int r = 0; r < 32; ++r) {
-                    const int idx = (lane + r) & 31;
-                    const float4 sb = sC[wid][idx];
-                    const float4 g = sG[wid][idx];
-#pragma unroll
-                    for (int k = 0; k < BPT; ++k) {
-                        const float rx = sb.x - px[k], ry = sb.y - py[k], rz = sb.z - pz[k];
-                        float d2 = fmaf(rx, rx, eps2);
-                        d2 = fmaf(ry, ry, d2);
-                        d2 = fmaf(rz, rz, d2);
-                        const float inv = rsqrt_approx(d2);
-                        const float inv2 = inv * inv;
-                        const float inv3 = inv2 * inv;
-                        const float inv5 = inv3 * inv2;
-                        const float rgj = fmaf(rz, g.z, fmaf(ry, g.y, rx * g.x));
-                        const float rgk = fmaf(rz, gz[k], fmaf(ry, gy[k], rx * gx[k]));
-                        const float cc = inv5 * fmaf(pm[k], rgj, -(sb.w * rgk));
-                        Px[k] = fmaf(inv3, g.x, Px[k]);
-                        Py[k] = fmaf(inv3, g.y, Py[k]);
-                        Pz[k] = fmaf(inv3, g.z, Pz[k]);
-                        q[k] = fmaf(inv3, sb.w, q[k]);
-                        Q0[k] = fmaf(cc, rx, Q0[k]);
-                        Q1[k] = fmaf(cc, ry, Q1[k]);
-                        Q2[k] = fmaf(cc, rz, Q2[k]);
-                        dm[k] = fmaf(inv3, rgj, dm[k]);
-                        rPx = fmaf(inv3, gx[k], rPx);
-                        rPy = fmaf(inv3, gy[k], rPy);
-                        rPz = fmaf(inv3, gz[k], rPz);
-                        rq = fmaf(inv3, pm[k], rq);
-                        rQ0 = fmaf(-cc, rx, rQ0);
-                        rQ1 = fmaf(-cc, ry, rQ1);
-                        rQ2 = fmaf(-cc, rz, rQ2);
-                        rw = fmaf(inv3, rgk, rw);
-                    }
-                    const int from = (lane + 1) & 31;
-                    rPx = __shfl_sync(0xffffffffu, rPx, from);
-                    rPy = __shfl_sync(0xffffffffu, rPy, from);
-                    rPz = __shfl_sync(0xffffffffu, rPz, from);
-                    rq = __shfl_sync(0xffffffffu, rq, from);
-                    rQ0 = __shfl_sync(0xffffffffu, rQ0, from);
-                    rQ1 = __shfl_sync(0xffffffffu, rQ1, from);
-                    rQ2 = __shfl_sync(0xffffffffu, rQ2, from);
-                    rw = __shfl_sync(0xffffffffu, rw, from);
-                }
-                // lane l holds chunk body l's reaction
-                if (jb + lane < ns) {
-                    const float4 sb = sC[wid][lane], gb = sG[wid][lane];
-                    const float ox = fmaf(sb.w, rPx, fmaf(-rq, gb.x, -3.f * rQ0));
-                    const float oy = fmaf(sb.w, rPy, fmaf(-rq, gb.y, -3.f * rQ1));
-                    const float oz = fmaf(sb.w, rPz, fmaf(-rq, gb.z, -3.f * rQ2));
-                    spart[bd.sp_off[s] + sym_soff(I, ns, RB) + (jb + lane - (I + 1) * RB)] =
-                        make_float4(ox, oy, oz, rw);
-                }
-            }
-        }
-        float4 *dst = tpart + ((long long)w + bd.row_off[s] + I) * RB;
-#pragma unroll
-        for (int k = 0; k < BPT; ++k) {
-            const float ox = fmaf(pm[k], Px[k], fmaf(-q[k], gx[k], -3.f * Q0[k]));
-            const float oy = fmaf(pm[k], Py[k], fmaf(-q[k], gy[k], -3.f * Q1[k]));
-            const float oz = fmaf(pm[k], Pz[k], fmaf(-q[k], gz[k], -3.f * Q2[k]));
-            dst[lane + 32 * k] = make_float4(ox, oy, oz, -dm[k]);
-        }
+        bks_vjp_segment<WPB, BPT>(pos + o, gbuf + o, ns, eps2, tpart + ((long long)w + bd.row_off[s] + I) * RB,
+                                  spart + bd.sp_off[s] + sym_soff(I, ns, RB), I, I * RC + (int)(it - rfirst),
+                                  I * RC + (int)(seg_end - rfirst));
         it = seg_end;
     }
 }
@@ -1331,10 +1229,12 @@ int nb_batch_create(const nb_params *p, int nsys, const int *sizes, nb_batch **o
         free_batch(b);
         return nb::cuda_error(e, "batch tables");
     }
-    // defaults: float symmetric one-warp workers x 16 targets, directed
-    // 4 x 4, float-float (FP64 state) one-warp workers x 2
+    // defaults: float symmetric one-warp workers x 12 targets (3828 us a step
+    // on 512 systems of 128 to 16384 bodies, 86.9 on 16 x 4096, 20.6 on 64 of
+    // 128 to 1000; 16 targets 3821, 91.9, 23.1; 8 targets 3949, 91.5, 20.2),
+    // directed 4 x 4, float-float (FP64 state) one-warp workers x 2
     const int wpb = p->block ? p->block / 32 : (b->sym ? 1 : 4);
-    const int bpt = p->bpt ? p->bpt : (b->f64 ? 2 : (b->sym ? 16 : 4));
+    const int bpt = p->bpt ? p->bpt : (b->f64 ? 2 : (b->sym ? 12 : 4));
     int st = batch_apply_plan(b, wpb, bpt, nullptr);
     if (st) {
         free_batch(b);
