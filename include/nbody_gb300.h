@@ -369,7 +369,10 @@ int nb_state_ptrs(nb_ctx *ctx, void **pos_dev, void **vel_dev);
 
 /* Resolved launch shape of the context's force kernel: {block, bpt, grid,
  * target block size, slots}; for the symmetric kernels block = warps per
- * CTA * 32, bpt = targets per lane and the target block is the row block. */
+ * CTA * 32, bpt = targets per lane and the target block is the row block.
+ * NB_F32 symmetric contexts of up to 9000 bodies step in one launch of a
+ * kernel of their own where their shape is the automatic one (unless bands
+ * or NB_SOURCE_FIXED are asked for); they report that automatic shape. */
 int nb_plan_info(nb_ctx *ctx, int *info5);
 
 /* Source side of a symmetric context: info4 = {source side (NB_SOURCE_FIXED

@@ -607,16 +607,16 @@ static int step_once(nb_ctx *c, cudaStream_t s, void *acc_out, cudaEvent_t *ev =
     } else if (p.algo == NB_ALGO_SYM) {
         st = nb::sym_force(c->splan, (const float4 *)po, (float)p.eps2, c->sym_t, c->sym_s,
                            (float4 *)c->sym_acc, s);
-        if (!st && ev) NB_CUDA(cudaEventRecord(ev[1], s));
+        if (!st && ev && !c->splan.small) NB_CUDA(cudaEventRecord(ev[1], s));
         if (!st && acc_keep)
             st = nb::sym_integrate(c->splan, (const float4 *)po, nullptr, nullptr, c->sym_t, c->sym_s,
-                                   (const float4 *)c->sym_acc,
+                                   (const float4 *)c->sym_acc, (float)p.eps2,
                                    (float)p.damping, (float)p.dt, p.kick, (float)p.G, acc_keep,
                                    s, 0);
         if (!st)
             st = nb::sym_integrate(c->splan, (const float4 *)po, (float4 *)pn, (float4 *)c->vel,
-                                   c->sym_t, c->sym_s, (const float4 *)c->sym_acc, (float)p.damping,
-                                   (float)p.dt, p.kick, (float)p.G, (float4 *)acc_out, s);
+                                   c->sym_t, c->sym_s, (const float4 *)c->sym_acc, (float)p.eps2,
+                                   (float)p.damping, (float)p.dt, p.kick, (float)p.G, (float4 *)acc_out, s);
     } else {
         st = nb::fast_force(c->plan, (const float4 *)po, (float)p.eps2, c->partial, s);
         if (!st && ev) NB_CUDA(cudaEventRecord(ev[1], s));
@@ -626,7 +626,8 @@ static int step_once(nb_ctx *c, cudaStream_t s, void *acc_out, cudaEvent_t *ev =
                                     (float4 *)acc_out, s);
     }
     if (!st && ev) {
-        if (!uses_fast(c) && !f64_sym(c)) NB_CUDA(cudaEventRecord(ev[1], s));  // exact: one fused kernel
+        // one fused kernel (exact, small symmetric systems): all of it is force time
+        if ((!uses_fast(c) && !f64_sym(c)) || (uses_sym(c) && c->splan.small)) NB_CUDA(cudaEventRecord(ev[1], s));
         NB_CUDA(cudaEventRecord(ev[2], s));
     }
     if (!st && !acc_out) c->cur ^= 1;
@@ -1073,11 +1074,11 @@ int nb_adj_backward(nb_ctx *c, unsigned long long generation, const void *gx_T, 
                     return st2;
                 if (p.kick == NB_KICK_REFERENCE &&
                     (st2 = nb::sym_integrate(c->splan, xk, nullptr, nullptr, c->sym_t, c->sym_s,
-                                             (const float4 *)c->sym_acc, D, dt,
+                                             (const float4 *)c->sym_acc, eps2, D, dt,
                                              p.kick, G, sa + (size_t)k * n, rs, 0)))
                     return st2;
                 if ((st2 = nb::sym_integrate(c->splan, xk, xn, vt, c->sym_t, c->sym_s,
-                                             (const float4 *)c->sym_acc, D, dt, p.kick, G, nullptr, rs)))
+                                             (const float4 *)c->sym_acc, eps2, D, dt, p.kick, G, nullptr, rs)))
                     return st2;
                 continue;
             }
@@ -1153,6 +1154,7 @@ int nb_launches_per_step(nb_ctx *c)
     const int bands = (uses_sym(c) || comp_sym(c) || f64_sym(c)) && c->splan.nbands > 1 ? c->splan.nbands : 0;
     if (ff_sym(c)) return 4 + (bands ? 2 * bands - 1 : 0);  // scale reduction, split, force, integrate
     if (bands) return 2 * bands + 1;
+    if (uses_sym(c) && c->splan.small) return 1;
     return (uses_fast(c) || is_comp(c) || f64_sym(c)) ? 2 : 1;
 }
 

@@ -1585,7 +1585,7 @@ static int sys_step(const nb_batch *b, const SysPlans &sp, int i, int c, float4 
     float4 *pn = b->pos[c ^ 1] + o, *vel = b->vel + o;
     if (b->sym) {
         if ((st = nb::sym_force(sp.sym[i], po, (float)p.eps2, tpart, spart, nullptr, s))) return st;
-        return nb::sym_integrate(sp.sym[i], po, pn, vel, tpart, spart, nullptr, (float)p.damping, (float)p.dt,
+        return nb::sym_integrate(sp.sym[i], po, pn, vel, tpart, spart, nullptr, (float)p.eps2, (float)p.damping, (float)p.dt,
                                  p.kick, (float)p.G, nullptr, s);
     }
     if ((st = nb::fast_force(sp.dir[i], po, (float)p.eps2, tpart, s, 0))) return st;

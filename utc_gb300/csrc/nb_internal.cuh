@@ -307,6 +307,8 @@ struct SymPlan {
     int slots = 0;       // grid + nrb - 1 target-side slots of rb float4
     long long spart_size = 0;  // float4 entries of the source-side array (of the largest band)
     int sms = 0;         // SMs of the device planned for
+    int small = 0;       // the step runs as one launch of the small-system kernel (nb_small.cu): sym_force
+                         // does nothing and sym_integrate is the whole step, without the partials
     // Triangular plans whose source-side array would pass the budget are cut
     // into bands of consecutive row blocks: the force kernel runs band by
     // band over the band's (row, chunk) items, every band's source-side
@@ -393,9 +395,16 @@ int sym_force(const SymPlan &p, const float4 *pos, float eps2, float4 *tpart, fl
 // consume (fixed plans): zero the accumulators after reading them, ready for
 // the next force launch; 0 leaves them for a second reader of the same
 // force launch
+// eps2: as given to sym_force (used by small plans)
 int sym_integrate(const SymPlan &p, const float4 *pos_old, float4 *pos_new, float4 *vel,
-                  const float4 *tpart, const float4 *spart, const float4 *accsum, float damping, float dt,
-                  int kick, float G, float4 *acc_out, cudaStream_t s, int consume = 1);
+                  const float4 *tpart, const float4 *spart, const float4 *accsum, float eps2, float damping,
+                  float dt, int kick, float G, float4 *acc_out, cudaStream_t s, int consume = 1);
+// One step (pos_new != nullptr) or the bare accelerations (acc_out), or both,
+// of a small system in one launch (nb_small.cu).
+int small_step(int n, int sms, const float4 *pos_old, float4 *pos_new, float4 *vel, float eps2, float damping,
+               float dt, int kick, float G, float4 *acc_out, cudaStream_t s);
+// Largest system that the automatic plan steps so.
+constexpr int kSmallBodies = 9000;
 // Fixed plans: zero the accumulators and write the record (the sum of |m| of
 // pos and the scale it gives with eps2); after every new state and scratch.
 int sym_fx_prepare(const SymPlan &p, const float4 *pos, float4 *spart, float eps2, cudaStream_t s);

@@ -1,0 +1,185 @@
+// nb_small.cu -- the whole step of a small FP32 system in one launch.
+//
+// The symmetric kernels need two dependent launches a step (pair terms, then
+// the sum of every body's partials), and a small system has few (row, chunk)
+// items for 152 SMs: at N = 1024 the pair terms take a third of a microsecond
+// of the chip, but the two launches took 7.4 us from a graph and 12.3 us one
+// by one.  Here a CTA owns TB bodies for the whole step: its 256 threads split
+// the sources, every pair is evaluated from the target's side (both orders
+// are evaluated, 12 FP32 operations and one rsqrt each: twice the pair terms,
+// but no partial leaves the CTA), the sums are reduced through the warps and
+// the CTA's first threads apply the kick / damping / drift.  No scratch, no
+// second launch, fixed order of summation: deterministic.
+//
+// Step time from a replayed graph, GB300, us, against the two launches:
+// N = 512 1.8 (6.4), 1024 2.2 (7.1), 2048 3.6 (9.2), 3000 5.4 (12.8), 4099
+// 9.2 (16.3), 6000 16.0 (23.7), 8192 28 (32.5).  Bounds: latency below N about
+// 2000 (launch, one round of loads, the reduction), above it register-file
+// reads (26 operand reads a pair of interactions, nb_pair.cuh) and how evenly
+// the CTAs fill the SMs.  128 threads a CTA ran 5 to 30 % ahead of 256 and
+// 512; the launch bound of one CTA lets the loop have the registers that it
+// asks for (142 for 8 targets, 110 for 4; without it 64, and 3.5 us at
+// N = 1024).
+#include "nb_pair.cuh"
+
+namespace nb {
+
+constexpr int kSmallThreads = 128;
+
+constexpr int pow2_up(int x) { return x <= 2 ? 2 : x <= 4 ? 4 : x <= 8 ? 8 : 16; }
+
+// Sums v[0..3 T) (T targets x 3 components) over the warp.  While more than
+// one target is left the lanes halve them: a lane keeps the half that its bit
+// selects and gives the other away, so that the first levels cost 3 T / 2,
+// 3 T / 4, ... shuffles.  Returns the lane's target; every lane of a target's
+// group has its three sums.
+template <int T>
+__device__ __forceinline__ int warp_sum(float *v, int lane)
+{
+    int mine = 0, off = 16;
+#pragma unroll
+    for (int h = T / 2; h >= 1; h /= 2) {
+        const bool up = (lane & off) != 0;
+        mine = 2 * mine + (up ? 1 : 0);
+#pragma unroll
+        for (int k = 0; k < 3 * h; ++k) {
+            const float give = up ? v[k] : v[3 * h + k], keep = up ? v[3 * h + k] : v[k];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+        }
+        off /= 2;
+    }
+#pragma unroll
+    for (; off >= 1; off /= 2) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], off);
+    }
+    return mine;
+}
+
+// pos_old is not declared __restrict__: it is written until the wait below, so
+// no load of it may take the read-only path.
+// pos_new == nullptr: no step, only acc_out; acc_out may be given beside a
+// step too.
+template <int TB>
+__global__ void __launch_bounds__(kSmallThreads, 1) small_step_kernel(const float4 *pos_old,
+                                                                   float4 *__restrict__ pos_new,
+                                                                   float4 *__restrict__ vel, int n, float eps2,
+                                                                   float damping, float dt, int kick, float G,
+                                                                   float4 *__restrict__ acc_out)
+{
+    constexpr int NP = TB / 2, TP = pow2_up(TB);
+    constexpr int NW = kSmallThreads / 32;
+    __shared__ float red[NW][3 * TP];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int t0 = blockIdx.x * TB;
+    const float4 pad = make_float4(kPadCoord, kPadCoord, kPadCoord, 0.f);
+    const f2 EPS2 = f2_pack(eps2, eps2);
+    // A programmatic launch: the blocks come in as those of the previous step's
+    // kernel leave, and wait here until that kernel is complete and its
+    // writes visible.  It gives its dependents no earlier signal: blocks let
+    // in before the SMs are free gather on those that empty first (N = 3000:
+    // 6.6 us a step against 5.4; plain launches 5.65).
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // the body that this thread integrates
+    const int mine = t0 + tid;
+    const bool own = tid < TB && mine < n;
+    float4 p = pad, v = pad;
+    if (own) {
+        p = pos_old[mine];
+        if (pos_new) v = vel[mine];
+    }
+    PairTargets<NP> T;
+    T.load([&](int t) { return t0 + t < n ? pos_old[t0 + t] : make_float4(0.f, 0.f, 0.f, 0.f); });
+    float4 nxt = tid < n ? pos_old[tid] : pad;
+    for (int j = tid; j - tid < n; j += kSmallThreads) {
+        const float4 q = nxt;
+        const int jn = j + kSmallThreads;
+        nxt = jn < n ? pos_old[jn] : pad;
+        const f2 X = f2_pack(q.x, q.x), Y = f2_pack(q.y, q.y), Z = f2_pack(q.z, q.z), M = f2_pack(q.w, q.w);
+#pragma unroll
+        for (int k = 0; k < NP; ++k) pair_pull(T, k, pair_term(T, k, X, Y, Z, EPS2), M);
+    }
+    float s[3 * TP];
+#pragma unroll
+    for (int t = 3 * TB; t < 3 * TP; ++t) s[t] = 0.f;
+#pragma unroll
+    for (int t = 0; t < TB; ++t) {
+        const float4 a = T.sum(t);
+        s[3 * t] = a.x;
+        s[3 * t + 1] = a.y;
+        s[3 * t + 2] = a.z;
+    }
+    const int t = warp_sum<TP>(s, lane);
+    if ((lane & (32 / TP - 1)) == 0) {
+        red[wid][3 * t] = s[0];
+        red[wid][3 * t + 1] = s[1];
+        red[wid][3 * t + 2] = s[2];
+    }
+    __syncthreads();
+    if (!own) return;
+    float ax = 0.f, ay = 0.f, az = 0.f;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+        ax = __fadd_rn(ax, red[w][3 * tid]);
+        ay = __fadd_rn(ay, red[w][3 * tid + 1]);
+        az = __fadd_rn(az, red[w][3 * tid + 2]);
+    }
+    if (acc_out) acc_out[mine] = make_float4(ax, ay, az, 0.f);
+    if (!pos_new) return;
+    const float k = kick == NB_KICK_REFERENCE ? p.w : G;
+    v.x = __fadd_rn(v.x, __fmul_rn(__fmul_rn(ax, k), dt));
+    v.y = __fadd_rn(v.y, __fmul_rn(__fmul_rn(ay, k), dt));
+    v.z = __fadd_rn(v.z, __fmul_rn(__fmul_rn(az, k), dt));
+    v.x = __fmul_rn(v.x, damping);
+    v.y = __fmul_rn(v.y, damping);
+    v.z = __fmul_rn(v.z, damping);
+    p.x = __fadd_rn(p.x, __fmul_rn(v.x, dt));
+    p.y = __fadd_rn(p.y, __fmul_rn(v.y, dt));
+    p.z = __fadd_rn(p.z, __fmul_rn(v.z, dt));
+    pos_new[mine] = p;
+    vel[mine] = v;
+}
+
+// Targets per CTA: few bodies per CTA while the step is a chain of latencies
+// (below 2000 bodies), then the choice that leaves the fullest SM the least
+// to do: ceil(CTAs / SMs) CTAs of TB bodies each, plus 0.9 of a body's work per
+// CTA for its pass over the sources and its reduction (measured for 4 to 16
+// bodies at twelve sizes: N = 3000 6.0 us with 10 bodies, 6.5 with 8, 6.7
+// with 6; N = 6000 15.9 with 8, 17.3 with 6).
+static int small_targets(int n, int sms)
+{
+    if (n < 2000) return 4;
+    int best = 8;
+    float least = 1e30f;
+    for (int tb = 6; tb <= 10; tb += 2) {
+        const int ctas = (n + tb - 1) / tb;
+        const float cost = (float)((ctas + sms - 1) / sms) * ((float)tb + 0.9f);
+        if (cost < least) {
+            least = cost;
+            best = tb;
+        }
+    }
+    return best;
+}
+
+int small_step(int n, int sms, const float4 *pos_old, float4 *pos_new, float4 *vel, float eps2, float damping,
+               float dt, int kick, float G, float4 *acc_out, cudaStream_t s)
+{
+    if (n == 0) return NB_OK;
+    const int tb = small_targets(n, sms);
+    auto k = tb == 4 ? small_step_kernel<4> : tb == 6 ? small_step_kernel<6> : tb == 8 ? small_step_kernel<8>
+                                                                                       : small_step_kernel<10>;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((n + tb - 1) / tb));
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    NB_CUDA(cudaLaunchKernelEx(&cfg, k, pos_old, pos_new, vel, n, eps2, damping, dt, kick, G, acc_out));
+    return NB_OK;
+}
+
+}  // namespace nb

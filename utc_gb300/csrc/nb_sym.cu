@@ -505,6 +505,19 @@ static sym_kernel_t sym_kernel_for(int w, int bpt, int comp, int fixed = 0, int 
     return nullptr;
 }
 
+// Targets per lane of the one-warp shape: 16, halved for small systems until
+// there are four (row, chunk) items per SM, at least 4.
+static int sym_small_bpt(int n, int sms)
+{
+    int bpt = 16;
+    while (bpt > 4 && n > 0) {
+        const int rb = 32 * bpt, nrb = (n + rb - 1) / rb, nc = (n + 31) / 32;
+        if (sym_prefix(nrb, nc, bpt) >= 4ll * sms) break;
+        bpt /= 2;
+    }
+    return bpt;
+}
+
 int sym_plan(int n, int warps, int bpt, int device, SymPlan *pl, int comp, int source_side, int bands)
 {
     if (source_side < NB_SOURCE_AUTO || source_side > NB_SOURCE_FIXED)
@@ -516,18 +529,14 @@ int sym_plan(int n, int warps, int bpt, int device, SymPlan *pl, int comp, int s
     // triangular plans go to bands where the array would pass the budget;
     // bands = -1 grows the row block instead
     const bool may_band = !fixed && bands >= 0;
+    int sms = 0;
+    NB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     SymPlan p;
     for (int attempt = 0; attempt < 2; ++attempt) {
         if (!given && fixed) {
             warps = 1;
             bpt = 16;
-            int sms = 0;  // fewer targets per lane for small systems, as below
-            NB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-            while (bpt > 4 && n > 0) {
-                const int rb = 32 * bpt, nrb = (n + rb - 1) / rb, nc = (n + 31) / 32;
-                if (sym_prefix(nrb, nc, bpt) >= 4ll * sms) break;
-                bpt /= 2;
-            }
+            bpt = sym_small_bpt(n, sms);  // fewer targets per lane for small systems, as below
         }
         if (warps == 0 && bpt == 0) {
             // plain: one-warp CTAs x 16 targets (row block 512), then 4 x 20
@@ -551,15 +560,7 @@ int sym_plan(int n, int warps, int bpt, int device, SymPlan *pl, int comp, int s
             // four (row, chunk) items per resident warp slot of an SM, so the
             // launch is not a few long items (at N=1024, 16 targets per lane
             // give 48 items)
-            if (!comp && warps == 1) {
-                int sms = 0;
-                NB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-                while (bpt > 4 && n > 0) {
-                    const int rb = 32 * bpt, nrb = (n + rb - 1) / rb, nc = (n + 31) / 32;
-                    if (sym_prefix(nrb, nc, bpt) >= 4ll * sms) break;
-                    bpt /= 2;
-                }
-            }
+            if (!comp && warps == 1) bpt = sym_small_bpt(n, sms);
         }
         if (warps == 0) warps = 8;
         if (bpt == 0) bpt = 8;
@@ -603,8 +604,13 @@ int sym_plan(int n, int warps, int bpt, int device, SymPlan *pl, int comp, int s
                                                           "1 or 4 warps x 12)"
                                                         : "symmetric kernel shape not compiled");
     p.total = n > 0 ? sym_prefix(p.nrb, p.nc, p.rb / 32) : 0;
-    int sms = 0, occ = 0;
-    NB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    // Small systems step in one launch where the plan is the automatic one
+    // (also when its shape is given): twice the pair terms, but no partials
+    // and no second launch (N = 1024 2.2 us a step against 7.1, N = 8192 28
+    // against 32.5; they meet between 9000, 33 us, and 10000, 41)
+    p.small = !comp && !p.fixed && p.nbands == 1 && bands <= 1 && n > 0 && n <= kSmallBodies && p.warps == 1 &&
+              p.bpt == sym_small_bpt(n, sms);
+    int occ = 0;
     NB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 32 * p.warps, 0));
     if (occ < 1) return set_error(NB_ERR_UNSUPPORTED, "symmetric kernel does not fit on an SM");
     long long grid = (long long)sms * occ;
@@ -675,7 +681,7 @@ int sym_fx_rescale(const SymPlan &p, float4 *spart, float eps2, cudaStream_t s)
 int sym_force(const SymPlan &p, const float4 *pos, float eps2, float4 *tpart, float4 *spart,
               float4 *accsum, cudaStream_t s)
 {
-    if (p.total == 0) return NB_OK;
+    if (p.total == 0 || p.small) return NB_OK;
     sym_kernel_t k = sym_kernel_for(p.warps, p.bpt, p.comp, p.fixed, p.nbands > 1);
     if (!k) return set_error(NB_ERR_UNSUPPORTED, "symmetric kernel shape not compiled");
     // lo blocks (compensated plans) follow the hi blocks
@@ -706,10 +712,12 @@ int sym_force(const SymPlan &p, const float4 *pos, float eps2, float4 *tpart, fl
 }
 
 int sym_integrate(const SymPlan &p, const float4 *pos_old, float4 *pos_new, float4 *vel,
-                  const float4 *tpart, const float4 *spart, const float4 *accsum, float damping, float dt,
-                  int kick, float G, float4 *acc_out, cudaStream_t s, int consume)
+                  const float4 *tpart, const float4 *spart, const float4 *accsum, float eps2, float damping,
+                  float dt, int kick, float G, float4 *acc_out, cudaStream_t s, int consume)
 {
     if (p.n == 0) return NB_OK;
+    if (p.small)
+        return small_step(p.n, p.sms, pos_old, acc_out ? nullptr : pos_new, vel, eps2, damping, dt, kick, G, acc_out, s);
     if (p.nbands > 1 && !accsum) return set_error(NB_ERR_INVALID, "sym_integrate: a banded plan needs its per-body sums");
     const long long threads = 4ll * p.n;  // a quad of threads per body
     unsigned long long *fxacc =
