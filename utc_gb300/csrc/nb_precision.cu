@@ -259,13 +259,26 @@ __global__ void energy_partial_kernel(int n, const float4 *__restrict__ pos32,
     if (threadIdx.x < 5) block_out[(size_t)blockIdx.x * 5 + threadIdx.x] = red[threadIdx.x][0];
 }
 
-__global__ void energy_final_kernel(const double *__restrict__ block_out, int nblocks,
-                                    double *__restrict__ out)
+// One block sums the block partials in a fixed order: thread (q, j) takes
+// partials j, j + 128, ..., then a tree over j.  (One thread per quantity took
+// 256 dependent additions at N = 65536.)
+constexpr int kEnergyFinal = 128;
+
+__global__ void __launch_bounds__(5 * kEnergyFinal)
+    energy_final_kernel(const double *__restrict__ block_out, int nblocks, double *__restrict__ out)
 {
-    if (threadIdx.x >= 5) return;
+    __shared__ double red[5][kEnergyFinal];
+    const int q = threadIdx.x / kEnergyFinal, j = threadIdx.x % kEnergyFinal;
     double s = 0;
-    for (int b = 0; b < nblocks; ++b) s += block_out[(size_t)b * 5 + threadIdx.x];
-    out[threadIdx.x] = s;
+#pragma unroll 4
+    for (int b = j; b < nblocks; b += kEnergyFinal) s += block_out[(size_t)b * 5 + q];
+    red[q][j] = s;
+    __syncthreads();
+    for (int w = kEnergyFinal / 2; w > 0; w >>= 1) {
+        if (j < w) red[q][j] += red[q][j + w];
+        __syncthreads();
+    }
+    if (j == 0) out[q] = red[q][0];
 }
 
 int comp_split(const double4 *pin, const double4 *vin, double4 *pos64, float4 *pos32,
@@ -428,7 +441,7 @@ int energy_reduce(int n, const float4 *pos32, const double4 *pos64, const float4
                                                           G, block_tmp, vel64);
         NB_LAUNCH_CHECK("energy_partial_kernel launch");
     }
-    energy_final_kernel<<<1, 32, 0, s>>>(block_tmp, nb, out_dev);
+    energy_final_kernel<<<1, 5 * kEnergyFinal, 0, s>>>(block_tmp, nb, out_dev);
     NB_LAUNCH_CHECK("energy_final_kernel launch");
     return NB_OK;
 }
