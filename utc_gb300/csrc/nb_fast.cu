@@ -14,8 +14,9 @@
 //    1-10 % slower.)
 //  * Sources are staged through shared memory with each component stored
 //    twice, (x, x, y, y) and (z, z, m, m), so one LDS.128 broadcast yields the
-//    two packed operands a source contributes to a target pair.  The next
-//    tile is prefetched into registers while the current one is consumed.
+//    two packed operands a source contributes to a target pair (once in the
+//    potential pass).  The next tile is prefetched into registers while the
+//    current one is consumed.
 //  * Work is split stream-K style: the (target block, 32-source group)
 //    iteration space is cut into `grid` equal contiguous ranges, one per
 //    persistent CTA, so all SMs finish together at any N (no wave
@@ -27,6 +28,145 @@
 #include "nb_pair.cuh"
 
 namespace nb {
+
+// A CTA's share of one target block: its targets against the sources
+// [j0, j1), sums to dst.  Not inlined into the loop over target blocks: as in
+// sym_row_segment of nb_sym.cu, ptxas otherwise moves the target pairs around
+// (4.5 moves a packed pair term).  N = 65536, one launch: plain 1527 us
+// against 1787, with the potential 1632 against 2044, compensated 1668 against
+// 1962 (2812 G interactions/s; 26 register operands a packed pair term, two
+// a cycle, allow 3100, see nb_pair.cuh).  The potential pass holds each source
+// once in shared memory and takes eight a turn (with pairs and four 1700 us);
+// for the plain pass that is slower (1598 us).
+template <int NT, int NPAIR, int FLAGS>
+__device__ __noinline__ void sk_segment(const float4 *__restrict__ pos, int n, float eps2, float4 *dst,
+                                        long long lo_offset, int tb, int j0, int j1)
+{
+    constexpr bool COMP = (FLAGS & SK_COMP) != 0;
+    constexpr bool PHI = (FLAGS & SK_PHI) != 0;
+    constexpr int TB = NT * 2 * NPAIR;
+    constexpr bool TWICE = !PHI || COMP;  // sources stored as pairs
+    constexpr int U = TWICE ? 4 : 8;      // sources per turn of the inner loop
+    constexpr int CP_ = COMP ? NPAIR : 1;
+    __shared__ __align__(16) float4 sA[NT];              // (x, x, y, y), or (x, y, z, m)
+    __shared__ __align__(16) float4 sB[TWICE ? NT : 1];  // (z, z, m, m)
+    const int t = threadIdx.x;
+    const f2 EPS2 = f2_pack(eps2, eps2);
+    const f2 ZERO = f2_pack(0.f, 0.f);
+    const float4 pad = make_float4(kPadCoord, kPadCoord, kPadCoord, 0.f);
+
+    f2 PX[NPAIR], PY[NPAIR], PZ[NPAIR], AX[NPAIR], AY[NPAIR], AZ[NPAIR], AP[NPAIR];
+    f2 SX[CP_], SY[CP_], SZ[CP_], SP[CP_], CX[CP_], CY[CP_], CZ[CP_], CPh[CP_];
+#pragma unroll
+    for (int p = 0; p < NPAIR; ++p) {
+        const int i0 = tb * TB + t + (2 * p) * NT;
+        const int i1 = i0 + NT;
+        const float4 q0 = i0 < n ? pos[i0] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 q1 = i1 < n ? pos[i1] : make_float4(0.f, 0.f, 0.f, 0.f);
+        PX[p] = f2_pack(q0.x, q1.x);
+        PY[p] = f2_pack(q0.y, q1.y);
+        PZ[p] = f2_pack(q0.z, q1.z);
+        AX[p] = AY[p] = AZ[p] = AP[p] = ZERO;
+        if constexpr (COMP) SX[p] = SY[p] = SZ[p] = SP[p] = CX[p] = CY[p] = CZ[p] = CPh[p] = ZERO;
+    }
+
+    float4 nxt = (j0 + t < j1) ? pos[j0 + t] : pad;
+#pragma unroll 1
+    for (int jt = j0; jt < j1; jt += NT) {
+        __syncthreads();  // the previous tile has been consumed by all warps
+        if constexpr (TWICE) {
+            sA[t] = make_float4(nxt.x, nxt.x, nxt.y, nxt.y);
+            sB[t] = make_float4(nxt.z, nxt.z, nxt.w, nxt.w);
+        } else {
+            sA[t] = nxt;
+        }
+        __syncthreads();
+        if (jt + NT < j1) {
+            const int jn = jt + NT + t;
+            nxt = jn < j1 ? pos[jn] : pad;
+        }
+        const int cnt = min(NT, j1 - jt);
+        const int cnt_u = (cnt + U - 1) / U * U;  // entries past cnt are zero-mass pads
+#pragma unroll 1
+        for (int j = 0; j < cnt_u; j += U) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const float4 a = sA[j + u];
+                f2 X2, Y2, Z2, M2;
+                if constexpr (TWICE) {
+                    const float4 b = sB[j + u];
+                    X2 = f2_pack(a.x, a.y), Y2 = f2_pack(a.z, a.w);
+                    Z2 = f2_pack(b.x, b.y), M2 = f2_pack(b.z, b.w);
+                } else {
+                    X2 = f2_pack(a.x, a.x), Y2 = f2_pack(a.y, a.y);
+                    Z2 = f2_pack(a.z, a.z), M2 = f2_pack(a.w, a.w);
+                }
+#pragma unroll
+                for (int p = 0; p < NPAIR; ++p) {
+                    const f2 rx = f2_sub(X2, PX[p]);
+                    const f2 ry = f2_sub(Y2, PY[p]);
+                    const f2 rz = f2_sub(Z2, PZ[p]);
+                    f2 d2 = f2_fma(rx, rx, EPS2);
+                    d2 = f2_fma(ry, ry, d2);
+                    d2 = f2_fma(rz, rz, d2);
+                    float dlo, dhi;
+                    f2_unpack(d2, dlo, dhi);
+                    const f2 inv = f2_pack(rsqrt_approx(dlo), rsqrt_approx(dhi));
+                    const f2 inv2 = f2_mul(inv, inv);
+                    const f2 mi = f2_mul(M2, inv);
+                    const f2 s = f2_mul(mi, inv2);
+                    AX[p] = f2_fma(rx, s, AX[p]);
+                    AY[p] = f2_fma(ry, s, AY[p]);
+                    AZ[p] = f2_fma(rz, s, AZ[p]);
+                    if constexpr (PHI) AP[p] = f2_add(AP[p], mi);
+                }
+            }
+        }
+        if constexpr (COMP) {
+#pragma unroll
+            for (int p = 0; p < NPAIR; ++p) {
+                f2 e;
+                f2_two_sum(SX[p], AX[p], SX[p], e);
+                CX[p] = f2_add(CX[p], e);
+                f2_two_sum(SY[p], AY[p], SY[p], e);
+                CY[p] = f2_add(CY[p], e);
+                f2_two_sum(SZ[p], AZ[p], SZ[p], e);
+                CZ[p] = f2_add(CZ[p], e);
+                if constexpr (PHI) {
+                    f2_two_sum(SP[p], AP[p], SP[p], e);
+                    CPh[p] = f2_add(CPh[p], e);
+                }
+                AX[p] = AY[p] = AZ[p] = AP[p] = ZERO;
+            }
+        }
+    }
+
+#pragma unroll
+    for (int p = 0; p < NPAIR; ++p) {
+        float x0, x1, y0, y1, z0, z1, w0 = 0.f, w1 = 0.f;
+        if constexpr (COMP) {
+            f2_unpack(SX[p], x0, x1);
+            f2_unpack(SY[p], y0, y1);
+            f2_unpack(SZ[p], z0, z1);
+            if constexpr (PHI) f2_unpack(SP[p], w0, w1);
+        } else {
+            f2_unpack(AX[p], x0, x1);
+            f2_unpack(AY[p], y0, y1);
+            f2_unpack(AZ[p], z0, z1);
+            if constexpr (PHI) f2_unpack(AP[p], w0, w1);
+        }
+        dst[t + (2 * p) * NT] = make_float4(x0, y0, z0, w0);
+        dst[t + (2 * p + 1) * NT] = make_float4(x1, y1, z1, w1);
+        if constexpr (COMP) {
+            f2_unpack(CX[p], x0, x1);
+            f2_unpack(CY[p], y0, y1);
+            f2_unpack(CZ[p], z0, z1);
+            if constexpr (PHI) f2_unpack(CPh[p], w0, w1);
+            dst[lo_offset + t + (2 * p) * NT] = make_float4(x0, y0, z0, w0);
+            dst[lo_offset + t + (2 * p + 1) * NT] = make_float4(x1, y1, z1, w1);
+        }
+    }
+}
 
 // Each thread owns 2*NPAIR targets held as packed pairs (t + 2p*NT,
 // t + (2p+1)*NT).  FLAGS: SK_COMP -- fold each tile's partial sums into a
@@ -44,129 +184,18 @@ __global__ void __launch_bounds__(NT) sk_force_kernel(const float4 *__restrict__
                                                       long long lo_offset, int cta_base, int grid_full,
                                                       long long it_lo, long long it_hi)
 {
-    constexpr bool COMP = (FLAGS & SK_COMP) != 0;
-    constexpr bool PHI = (FLAGS & SK_PHI) != 0;
     constexpr int TB = NT * 2 * NPAIR;
-    constexpr int CP_ = COMP ? NPAIR : 1;
-    __shared__ __align__(16) float4 sA[NT];  // (x, x, y, y)
-    __shared__ __align__(16) float4 sB[NT];  // (z, z, m, m)
-    const int t = threadIdx.x;
     const int c = cta_base + blockIdx.x;
     long long it = sk_start(c, total, grid_full);
     long long end = sk_start(c + 1, total, grid_full);
     if (it < it_lo) it = it_lo;
     if (end > it_hi) end = it_hi;
-    const f2 EPS2 = f2_pack(eps2, eps2);
-    const f2 ZERO = f2_pack(0.f, 0.f);
-    const float4 pad = make_float4(kPadCoord, kPadCoord, kPadCoord, 0.f);
-
     while (it < end) {
         const int tb = (int)(it / ngroups);
         const long long tb_first = (long long)tb * ngroups;
         const long long seg_end = end < tb_first + ngroups ? end : tb_first + ngroups;
-        const int j0 = (int)(it - tb_first) * kGroup;
-        const int j1 = min((int)(seg_end - tb_first) * kGroup, n);
-
-        f2 PX[NPAIR], PY[NPAIR], PZ[NPAIR], AX[NPAIR], AY[NPAIR], AZ[NPAIR], AP[NPAIR];
-        f2 SX[CP_], SY[CP_], SZ[CP_], SP[CP_], CX[CP_], CY[CP_], CZ[CP_], CPh[CP_];
-#pragma unroll
-        for (int p = 0; p < NPAIR; ++p) {
-            const int i0 = tb * TB + t + (2 * p) * NT;
-            const int i1 = i0 + NT;
-            const float4 q0 = i0 < n ? pos[i0] : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float4 q1 = i1 < n ? pos[i1] : make_float4(0.f, 0.f, 0.f, 0.f);
-            PX[p] = f2_pack(q0.x, q1.x);
-            PY[p] = f2_pack(q0.y, q1.y);
-            PZ[p] = f2_pack(q0.z, q1.z);
-            AX[p] = AY[p] = AZ[p] = AP[p] = ZERO;
-            if constexpr (COMP) SX[p] = SY[p] = SZ[p] = SP[p] = CX[p] = CY[p] = CZ[p] = CPh[p] = ZERO;
-        }
-
-        float4 nxt = (j0 + t < j1) ? pos[j0 + t] : pad;
-        for (int jt = j0; jt < j1; jt += NT) {
-            __syncthreads();  // the previous tile has been consumed by all warps
-            sA[t] = make_float4(nxt.x, nxt.x, nxt.y, nxt.y);
-            sB[t] = make_float4(nxt.z, nxt.z, nxt.w, nxt.w);
-            __syncthreads();
-            if (jt + NT < j1) {
-                const int jn = jt + NT + t;
-                nxt = jn < j1 ? pos[jn] : pad;
-            }
-            const int cnt = min(NT, j1 - jt);
-            const int cnt4 = (cnt + 3) & ~3;  // entries past cnt are zero-mass pads
-            for (int j = 0; j < cnt4; j += 4) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const float4 a = sA[j + u];
-                    const float4 b = sB[j + u];
-                    const f2 X2 = f2_pack(a.x, a.y), Y2 = f2_pack(a.z, a.w);
-                    const f2 Z2 = f2_pack(b.x, b.y), M2 = f2_pack(b.z, b.w);
-#pragma unroll
-                    for (int p = 0; p < NPAIR; ++p) {
-                        const f2 rx = f2_sub(X2, PX[p]);
-                        const f2 ry = f2_sub(Y2, PY[p]);
-                        const f2 rz = f2_sub(Z2, PZ[p]);
-                        f2 d2 = f2_fma(rx, rx, EPS2);
-                        d2 = f2_fma(ry, ry, d2);
-                        d2 = f2_fma(rz, rz, d2);
-                        float dlo, dhi;
-                        f2_unpack(d2, dlo, dhi);
-                        const f2 inv = f2_pack(rsqrt_approx(dlo), rsqrt_approx(dhi));
-                        const f2 inv2 = f2_mul(inv, inv);
-                        const f2 mi = f2_mul(M2, inv);
-                        const f2 s = f2_mul(mi, inv2);
-                        AX[p] = f2_fma(rx, s, AX[p]);
-                        AY[p] = f2_fma(ry, s, AY[p]);
-                        AZ[p] = f2_fma(rz, s, AZ[p]);
-                        if constexpr (PHI) AP[p] = f2_add(AP[p], mi);
-                    }
-                }
-            }
-            if constexpr (COMP) {
-#pragma unroll
-                for (int p = 0; p < NPAIR; ++p) {
-                    f2 e;
-                    f2_two_sum(SX[p], AX[p], SX[p], e);
-                    CX[p] = f2_add(CX[p], e);
-                    f2_two_sum(SY[p], AY[p], SY[p], e);
-                    CY[p] = f2_add(CY[p], e);
-                    f2_two_sum(SZ[p], AZ[p], SZ[p], e);
-                    CZ[p] = f2_add(CZ[p], e);
-                    if constexpr (PHI) {
-                        f2_two_sum(SP[p], AP[p], SP[p], e);
-                        CPh[p] = f2_add(CPh[p], e);
-                    }
-                    AX[p] = AY[p] = AZ[p] = AP[p] = ZERO;
-                }
-            }
-        }
-
-        float4 *dst = partial + (size_t)(c + tb) * TB;
-#pragma unroll
-        for (int p = 0; p < NPAIR; ++p) {
-            float x0, x1, y0, y1, z0, z1, w0 = 0.f, w1 = 0.f;
-            if constexpr (COMP) {
-                f2_unpack(SX[p], x0, x1);
-                f2_unpack(SY[p], y0, y1);
-                f2_unpack(SZ[p], z0, z1);
-                if constexpr (PHI) f2_unpack(SP[p], w0, w1);
-            } else {
-                f2_unpack(AX[p], x0, x1);
-                f2_unpack(AY[p], y0, y1);
-                f2_unpack(AZ[p], z0, z1);
-                if constexpr (PHI) f2_unpack(AP[p], w0, w1);
-            }
-            dst[t + (2 * p) * NT] = make_float4(x0, y0, z0, w0);
-            dst[t + (2 * p + 1) * NT] = make_float4(x1, y1, z1, w1);
-            if constexpr (COMP) {
-                f2_unpack(CX[p], x0, x1);
-                f2_unpack(CY[p], y0, y1);
-                f2_unpack(CZ[p], z0, z1);
-                if constexpr (PHI) f2_unpack(CPh[p], w0, w1);
-                dst[lo_offset + t + (2 * p) * NT] = make_float4(x0, y0, z0, w0);
-                dst[lo_offset + t + (2 * p + 1) * NT] = make_float4(x1, y1, z1, w1);
-            }
-        }
+        sk_segment<NT, NPAIR, FLAGS>(pos, n, eps2, partial + (size_t)(c + tb) * TB, lo_offset, tb,
+                                     (int)(it - tb_first) * kGroup, min((int)(seg_end - tb_first) * kGroup, n));
         it = seg_end;
     }
 }
