@@ -86,7 +86,7 @@ __device__ __noinline__ void sk_segment(const float4 *__restrict__ pos, int n, f
             nxt = jn < j1 ? pos[jn] : pad;
         }
         const int cnt = min(NT, j1 - jt);
-        const int cnt_u = (cnt + U - 1) / U * U;  // entries past cnt are zero-mass pads
+        const int cnt_u = (cnt + U - 1) & ~(U - 1);  // entries past cnt are zero-mass pads
 #pragma unroll 1
         for (int j = 0; j < cnt_u; j += U) {
 #pragma unroll
@@ -178,7 +178,7 @@ __device__ __noinline__ void sk_segment(const float4 *__restrict__ pos, int n, f
 // that cover a range of target blocks computes those blocks' partial slots
 // exactly as the full launch does (a shard of the targets, same bits).
 template <int NT, int NPAIR, int FLAGS>
-__global__ void __launch_bounds__(NT) sk_force_kernel(const float4 *__restrict__ pos, int n,
+__global__ void __launch_bounds__(NT, NPAIR == 1 ? 1024 / NT : 0) sk_force_kernel(const float4 *__restrict__ pos, int n,
                                                       float eps2, float4 *__restrict__ partial,
                                                       long long total, int ngroups,
                                                       long long lo_offset, int cta_base, int grid_full,
