@@ -216,7 +216,10 @@ int nb_energy(nb_ctx *ctx, double *out5, void *accphi_dev, void *stream);
 
 /* Adjoint (reverse mode) of `steps` steps; no counterpart in the reference.
  * nb_adj_forward advances the state like nb_step and keeps a checkpoint
- * (positions and velocities) every ckpt_every steps.  nb_adj_backward then
+ * (positions and velocities) every ckpt_every steps; where the positions of
+ * all steps (and, with the reference kick, the accelerations: 16 or 32 B per
+ * body and step) come to at most 1 GiB it keeps those instead, and nothing
+ * below is recomputed (the gradients have the same bits).  nb_adj_backward then
  * takes the cotangents of the final positions gx_T and velocities gv_T
  * (device, n float4, xyz used; gv_T may be NULL for zero) and writes
  * dL/dx0, dL/dv0 (device n float4, w = 0) and dL/dm (device n float),

@@ -135,6 +135,12 @@ struct nb_ctx {
         unsigned long long generation = 0;
         // the forward pass left the last segment's states in seg_pos/seg_acc
         bool live_last = false;
+        // every state of the recorded forward pass, [steps + 1][n], and its
+        // accelerations (reference kick), [steps][n]: nothing is recomputed
+        // where they fit kAdjTapeBytes
+        bool taped = false;
+        float4 *tape_pos = nullptr, *tape_acc = nullptr;
+        size_t cap_tape_pos = 0, cap_tape_acc = 0;  // float4 entries
         // second segment buffer: segment s-1 is recomputed on rstream while
         // the reverse pass runs through segment s on the caller's stream
         float4 *seg_pos2 = nullptr, *seg_acc2 = nullptr, *vel_tmp2 = nullptr;
@@ -216,6 +222,8 @@ static void free_ctx(nb_ctx *c)
     nb::dfree(c->adj.seg_pos2);
     nb::dfree(c->adj.seg_acc2);
     nb::dfree(c->adj.vel_tmp2);
+    nb::dfree(c->adj.tape_pos);
+    nb::dfree(c->adj.tape_acc);
     if (c->adj.rstream) cudaStreamDestroy(c->adj.rstream);
     for (auto &e : c->adj.ev_rec)
         if (e) cudaEventDestroy(e);
@@ -907,6 +915,37 @@ int nb_energy(nb_ctx *c, double *out5, void *accphi_dev, void *stream)
 // ---------------------------------------------------------------------------
 // adjoint: forward with checkpoints, reverse pass with per-segment recompute
 // ---------------------------------------------------------------------------
+// Most that the states of a forward pass may take for all of them to be kept.
+// The caller's ckpt_every bounds the memory of long trajectories of large
+// systems; below this size the recomputation that it costs (a forward step per
+// reverse step: 85 of 350 us at N = 16384) buys less than a hundredth of the
+// GPU's memory.
+constexpr size_t kAdjTapeBytes = (size_t)1 << 30;
+
+// Room for a tape of `steps` steps; false when it would be too large or the
+// device has none left (the checkpoints then serve).
+static bool adj_reserve_tape(nb_ctx *c, int steps)
+{
+    auto &A = c->adj;
+    const size_t n = (size_t)c->p.n, np = n * ((size_t)steps + 1);
+    const size_t na = c->p.kick == NB_KICK_REFERENCE ? n * (size_t)steps : 0;
+    if (n == 0 || (np + na) * sizeof(float4) > kAdjTapeBytes) return false;
+    auto grow = [](float4 **buf, size_t *cap, size_t need) {
+        if (need <= *cap) return true;
+        nb::dfree(*buf);
+        *buf = nullptr;
+        *cap = 0;
+        if (nb::dmalloc((void **)buf, need * sizeof(float4)) != cudaSuccess) {
+            *buf = nullptr;
+            (void)cudaGetLastError();
+            return false;
+        }
+        *cap = need;
+        return true;
+    };
+    return grow(&A.tape_pos, &A.cap_tape_pos, np) && grow(&A.tape_acc, &A.cap_tape_acc, na);
+}
+
 static int adj_reserve(nb_ctx *c, int nckpt, int every)
 {
     const size_t n = (size_t)c->p.n;
@@ -947,7 +986,7 @@ static int adj_reserve(nb_ctx *c, int nckpt, int every)
             (st = dev_alloc((void **)&A.gm, n * sizeof(float), "adjoint allocation")))
             return st;
     }
-    if (nckpt > A.cap_ckpt) {
+    if (nckpt > A.cap_ckpt) {  // (0 for a taped pass)
         nb::dfree(A.ckpt_pos);
         nb::dfree(A.ckpt_vel);
         A.ckpt_pos = A.ckpt_vel = nullptr;
@@ -974,6 +1013,39 @@ static int adj_reserve(nb_ctx *c, int nckpt, int every)
     return NB_OK;
 }
 
+// `len` steps from x[0], states to x[1], x[2], ... (n float4 each), the
+// velocities vel updated in place, with the reference kick the accelerations
+// to acc[0], acc[1], ...: the kernels, and so the bits, of nb_step.
+static int adj_steps(nb_ctx *c, float4 *x, float4 *vel, float4 *acc, int len, cudaStream_t s)
+{
+    const nb_params &p = c->p;
+    const size_t n = (size_t)p.n;
+    const float eps2 = (float)p.eps2, D = (float)p.damping, dt = (float)p.dt, G = (float)p.G;
+    const bool ref = p.kick == NB_KICK_REFERENCE;
+    int st = NB_OK;
+    for (int k = 0; k < len && !st; ++k) {
+        const float4 *xk = x + (size_t)k * n;
+        float4 *xn = x + (size_t)(k + 1) * n, *ak = ref ? acc + (size_t)k * n : nullptr;
+        if (uses_sym(c) && c->splan.small) {
+            st = nb::small_step(p.n, c->splan.sms, xk, xn, vel, eps2, D, dt, p.kick, G, ak, s);
+        } else if (uses_sym(c)) {
+            const float4 *sum = (const float4 *)c->sym_acc;
+            st = nb::sym_force(c->splan, xk, eps2, c->sym_t, c->sym_s, (float4 *)c->sym_acc, s);
+            if (!st && ak)
+                st = nb::sym_integrate(c->splan, xk, nullptr, nullptr, c->sym_t, c->sym_s, sum, eps2, D, dt, p.kick,
+                                       G, ak, s, 0);
+            if (!st)
+                st = nb::sym_integrate(c->splan, xk, xn, vel, c->sym_t, c->sym_s, sum, eps2, D, dt, p.kick, G,
+                                       nullptr, s);
+        } else {
+            st = nb::fast_force(c->plan, xk, eps2, c->partial, s);
+            if (!st && ak) st = nb::fast_reduce(c->plan, c->partial, 0, xk, eps2, ak, nullptr, s);
+            if (!st) st = nb::fast_integrate(c->plan, xk, xn, vel, c->partial, D, dt, p.kick, G, nullptr, s);
+        }
+    }
+    return st;
+}
+
 int nb_adj_forward(nb_ctx *c, int steps, int ckpt_every, void *stream, unsigned long long *generation)
 {
     if (generation) *generation = 0;
@@ -984,20 +1056,37 @@ int nb_adj_forward(nb_ctx *c, int steps, int ckpt_every, void *stream, unsigned 
     if (steps < 1 || ckpt_every < 1) return set_error(NB_ERR_INVALID, "steps and ckpt_every must be >= 1");
     if (ckpt_every > steps) ckpt_every = steps;
     const int nckpt = (steps + ckpt_every - 1) / ckpt_every;
-    int st = adj_reserve(c, nckpt, ckpt_every);
+    auto &A = c->adj;
+    A.ready = false;  // what it holds may go from here on
+    A.live_last = false;
+    const bool taped = adj_reserve_tape(c, steps);
+    int st = taped ? adj_reserve(c, 0, 0) : adj_reserve(c, nckpt, ckpt_every);
     if (st) return st;
     cudaStream_t s = (cudaStream_t)stream;
     if ((st = fx_refresh(c, s))) return st;
     const size_t n = (size_t)c->p.n;
-    auto &A = c->adj;
+    if (taped) {
+        // every state stays where it is computed
+        NB_CUDA(cudaMemcpyAsync(A.tape_pos, c->pos[c->cur], n * sizeof(float4), cudaMemcpyDeviceToDevice, s));
+        if ((st = adj_steps(c, A.tape_pos, (float4 *)c->vel, A.tape_acc, steps, s))) return st;
+        NB_CUDA(cudaMemcpyAsync(c->pos[c->cur], A.tape_pos + (size_t)steps * n, n * sizeof(float4),
+                                cudaMemcpyDeviceToDevice, s));
+        A.steps = steps;
+        A.every = steps;
+        A.nckpt = 1;
+        A.taped = true;
+        A.ready = true;
+        A.generation += 1;
+        if (generation) *generation = A.generation;
+        return NB_OK;
+    }
+    A.taped = false;
     const nb_params &p = c->p;
     // The last segment is the first one the reverse pass needs: its states
     // (and, for the reference kick, its accelerations) are kept in the
     // segment buffers as they are computed, so that segment is not
     // recomputed.  Same kernels, same bits as a recompute.
     const int t_last = (nckpt - 1) * ckpt_every;
-    A.ready = false;
-    A.live_last = false;
     for (int t = 0; t < steps; ++t) {
         if (t % ckpt_every == 0 && n) {
             const size_t k = (size_t)(t / ckpt_every) * n;
@@ -1065,31 +1154,7 @@ int nb_adj_backward(nb_ctx *c, unsigned long long generation, const void *gx_T, 
         const int len = (A.steps - t0) < A.every ? (A.steps - t0) : A.every;
         NB_CUDA(cudaMemcpyAsync(sp, A.ckpt_pos + (size_t)seg * n, n * sizeof(float4), cudaMemcpyDeviceToDevice, rs));
         NB_CUDA(cudaMemcpyAsync(vt, A.ckpt_vel + (size_t)seg * n, n * sizeof(float4), cudaMemcpyDeviceToDevice, rs));
-        int st2;
-        for (int k = 0; k < len; ++k) {
-            const float4 *xk = sp + (size_t)k * n;
-            float4 *xn = sp + (size_t)(k + 1) * n;
-            if (uses_sym(c)) {
-                if ((st2 = nb::sym_force(c->splan, xk, eps2, c->sym_t, c->sym_s, (float4 *)c->sym_acc, rs)))
-                    return st2;
-                if (p.kick == NB_KICK_REFERENCE &&
-                    (st2 = nb::sym_integrate(c->splan, xk, nullptr, nullptr, c->sym_t, c->sym_s,
-                                             (const float4 *)c->sym_acc, eps2, D, dt,
-                                             p.kick, G, sa + (size_t)k * n, rs, 0)))
-                    return st2;
-                if ((st2 = nb::sym_integrate(c->splan, xk, xn, vt, c->sym_t, c->sym_s,
-                                             (const float4 *)c->sym_acc, eps2, D, dt, p.kick, G, nullptr, rs)))
-                    return st2;
-                continue;
-            }
-            if ((st2 = nb::fast_force(c->plan, xk, eps2, c->partial, rs))) return st2;
-            if (p.kick == NB_KICK_REFERENCE &&
-                (st2 = nb::fast_reduce(c->plan, c->partial, 0, xk, eps2, sa + (size_t)k * n, nullptr, rs)))
-                return st2;
-            if ((st2 = nb::fast_integrate(c->plan, xk, xn, vt, c->partial, D, dt, p.kick, G, nullptr, rs)))
-                return st2;
-        }
-        return NB_OK;
+        return adj_steps(c, sp, vt, sa, len, rs);
     };
     // Segments alternate between the two buffers, the last one in buffer 0
     // (where the forward pass leaves it).  While the reverse pass runs through
@@ -1102,7 +1167,7 @@ int nb_adj_backward(nb_ctx *c, unsigned long long generation, const void *gx_T, 
     if (last > 0 && !A.rstream &&
         (st = nb::create_recompute_stream(&A.rstream, A.ev_rec, &A.ev_go)))
         return st;
-    if (!live && (st = recompute(last, buf_of(last), s))) return st;
+    if (!A.taped && !live && (st = recompute(last, buf_of(last), s))) return st;
     bool have_g = false;
     for (int seg = last; seg >= 0; --seg) {
         const int b = buf_of(seg);
@@ -1115,13 +1180,14 @@ int nb_adj_backward(nb_ctx *c, unsigned long long generation, const void *gx_T, 
             if ((st = recompute(seg - 1, buf_of(seg - 1), A.rstream))) return st;
             NB_CUDA(cudaEventRecord(A.ev_rec[buf_of(seg - 1)], A.rstream));
         }
-        const float4 *sp = b ? A.seg_pos2 : A.seg_pos, *sa = b ? A.seg_acc2 : A.seg_acc;
+        const float4 *sp = A.taped ? A.tape_pos : b ? A.seg_pos2 : A.seg_pos;
+        const float4 *sa = A.taped ? A.tape_acc : b ? A.seg_acc2 : A.seg_acc;
         const int t0 = seg * A.every;
         const int len = (A.steps - t0) < A.every ? (A.steps - t0) : A.every;
-        // reverse through the segment
+        // reverse through the segment (a taped pass is one)
         for (int k = len - 1; k >= 0; --k) {
             const float4 *xk = sp + (size_t)k * n;
-            const float4 *ak = sa + (size_t)k * n;
+            const float4 *ak = sa ? sa + (size_t)k * n : nullptr;  // read with the reference kick only
             if (!have_g) {
                 if ((st = nb::adj_g(p.n, xk, A.lx, A.lv, A.gbuf, D, dt, p.kick, G, s))) return st;
                 have_g = true;
