@@ -497,6 +497,54 @@ int nb_destroy(nb_ctx *c)
     return NB_OK;
 }
 
+}  // extern "C"
+
+// dst <- src for two buffers of `n` float4 each (pos, vel).
+static __global__ void state_copy_kernel(float4 *d0, const float4 *s0, float4 *d1, const float4 *s1, size_t n)
+{
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n)
+        d0[i] = s0[i];
+    else if (i < 2 * n)
+        d1[i - n] = s1[i - n];
+}
+
+// Both arrays of the state between this context and a caller, `sb` bytes each,
+// in one launch where the caller's pointers are memory of this device that a
+// kernel may read 16 bytes at a time, otherwise (host memory, another device,
+// odd addresses, buffers that cross) as two copies in order.  The two copies
+// on either side of a small system's step cost the host 5.9 us each time, the
+// one launch 2.5, the step 2.0.
+static cudaError_t copy_state(const nb_ctx *c, void *d0, const void *s0, void *d1, const void *s1, size_t sb,
+                              const void *user0, const void *user1, cudaStream_t s)
+{
+    int dev = -1;
+    auto here = [&](const void *q) {
+        cudaPointerAttributes at;
+        if ((uintptr_t)q % 16 || cudaPointerGetAttributes(&at, q) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        return at.type == cudaMemoryTypeDevice && at.device == c->device;
+    };
+    auto cross = [&](const void *a, const void *b) {
+        const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+        return x < y + sb && y < x + sb;
+    };
+    if (c->p.memtype != NB_MEM_UNIFIED && cudaGetDevice(&dev) == cudaSuccess && dev == c->device && !cross(d0, s1) &&
+        !cross(d1, s0) && !cross(d0, d1) && here(user0) && here(user1)) {
+        const size_t n = sb / sizeof(float4);
+        state_copy_kernel<<<(unsigned)((2 * n + 255) / 256), 256, 0, s>>>((float4 *)d0, (const float4 *)s0,
+                                                                         (float4 *)d1, (const float4 *)s1, n);
+        if (cudaGetLastError() == cudaSuccess) return cudaSuccess;
+        // not launched (a stream of another device): the copies
+    }
+    cudaError_t e = cudaMemcpyAsync(d0, s0, sb, cudaMemcpyDefault, s);
+    return e == cudaSuccess ? cudaMemcpyAsync(d1, s1, sb, cudaMemcpyDefault, s) : e;
+}
+
+extern "C" {
+
 int nb_set_state(nb_ctx *c, const void *pos, const void *vel, int where, void *stream)
 {
     if (!c) return set_error(NB_ERR_INVALID, "ctx is NULL");
@@ -513,8 +561,12 @@ int nb_set_state(nb_ctx *c, const void *pos, const void *vel, int where, void *s
         if (st) return st;
         if (where == NB_HOST) NB_CUDA(cudaStreamSynchronize(s));
     } else if (sb) {
-        NB_CUDA(cudaMemcpyAsync(c->pos[0], pos, sb, cudaMemcpyDefault, s));
-        NB_CUDA(cudaMemcpyAsync(c->vel, vel, sb, cudaMemcpyDefault, s));
+        if (where == NB_DEVICE) {
+            NB_CUDA(copy_state(c, c->pos[0], pos, c->vel, vel, sb, pos, vel, s));
+        } else {
+            NB_CUDA(cudaMemcpyAsync(c->pos[0], pos, sb, cudaMemcpyDefault, s));
+            NB_CUDA(cudaMemcpyAsync(c->vel, vel, sb, cudaMemcpyDefault, s));
+        }
         // symmetric contexts: zeroed source-side accumulators and the sum of
         // |m| their scale comes from
         if (uses_sym(c)) {
@@ -542,6 +594,8 @@ int nb_get_state(nb_ctx *c, void *pos, void *vel, int where, void *stream)
         if (pos) NB_CUDA(cudaMemcpyAsync(pos, c->tmpA, sb, cudaMemcpyDefault, s));
         if (vel) NB_CUDA(cudaMemcpyAsync(vel, c->tmpB, sb, cudaMemcpyDefault, s));
         if (where == NB_HOST) NB_CUDA(cudaStreamSynchronize(s));
+    } else if (sb && pos && vel && where == NB_DEVICE) {
+        NB_CUDA(copy_state(c, pos, c->pos[c->cur], vel, c->vel, sb, pos, vel, s));
     } else if (sb) {
         if (pos) NB_CUDA(cudaMemcpyAsync(pos, c->pos[c->cur], sb, cudaMemcpyDefault, s));
         if (vel) NB_CUDA(cudaMemcpyAsync(vel, c->vel, sb, cudaMemcpyDefault, s));

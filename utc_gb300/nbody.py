@@ -19,17 +19,30 @@ _ALGO = {"fast": N.NB_ALGO_FAST, "exact": N.NB_ALGO_EXACT, "sym": N.NB_ALGO_SYM,
 _KICK = {"reference": N.NB_KICK_REFERENCE, "physical": N.NB_KICK_PHYSICAL}
 
 
+_torch_module = None
+_raw_stream = None  # (device) -> cudaStream_t of torch's current stream
+
+
 def _torch():
-    import torch
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        _torch_module = torch
+    return _torch_module
 
 
 def current_stream_handle():
-    """cudaStream_t of torch's current stream as an int (0 = legacy default)."""
-    torch = _torch()
-    if torch.cuda.is_available():
-        return int(torch.cuda.current_stream().cuda_stream)
-    return 0
+    """cudaStream_t of torch's current stream as an int (0 = legacy default).
+    Asked for on every call: torch's raw getter where it has one (a tenth of
+    the host time of building a Stream object)."""
+    global _raw_stream
+    torch = _torch_module or _torch()
+    if not torch.cuda.is_initialized() and not torch.cuda.is_available():
+        return 0
+    if _raw_stream is None:
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+            lambda device: torch.cuda.current_stream(device).cuda_stream)
+    return int(_raw_stream(torch.cuda.current_device()))
 
 
 def _is_torch(x):
@@ -41,11 +54,12 @@ def _device_buffer(x, shape, dtype, name):
     if only the dtype or the layout differ).  The C ABI copies whole buffers
     by the context's size: a tensor of another size would be read or written
     past its end, so that is refused here."""
-    torch = _torch()
     if not _is_torch(x) or not x.is_cuda:
         raise ValueError(f"{name}: needs a CUDA tensor")
-    if tuple(x.shape) != tuple(shape):
+    if x.shape != shape:
         raise ValueError(f"{name}: needs shape {tuple(shape)}, got {tuple(x.shape)}")
+    if x.dtype is dtype and x.is_contiguous():
+        return x
     return x.to(dtype).contiguous()
 
 
@@ -73,6 +87,7 @@ class NBodySystem:
         self.precision = precision
         # host-side state type: double4 for f64 and for the compensated mode
         self.dtype = np.float64 if precision in ("f64", "f32comp") else np.float32
+        self._shape = (self.n, 4)
         h = C.c_void_p()
         N.check(self.lib.nb_create(C.byref(p), C.byref(h)), "nb_create")
         self.handle = h
@@ -104,8 +119,8 @@ class NBodySystem:
 
     def _buf(self, x, name):
         if _is_torch(x):
-            t = _device_buffer(x, (self.n, 4), self._torch_dtype(), name)
-            return C.c_void_p(t.data_ptr()), N.NB_DEVICE, t
+            t = _device_buffer(x, self._shape, self._torch_dtype(), name)
+            return t.data_ptr(), N.NB_DEVICE, t
         a = np.ascontiguousarray(x, dtype=self.dtype).reshape(self.n, 4)
         return a.ctypes.data_as(C.c_void_p), N.NB_HOST, a
 
@@ -115,7 +130,7 @@ class NBodySystem:
         if wp != wv:
             raise ValueError("pos and vel must both be host or both be device buffers")
         s = current_stream_handle() if stream is None else stream
-        N.check(self.lib.nb_set_state(self.handle, pp, vp, wp, C.c_void_p(s)), "nb_set_state")
+        N.check(self.lib.nb_set_state(self.handle, pp, vp, wp, s), "nb_set_state")
         if wp == N.NB_DEVICE and (keep_p is not pos or keep_v is not vel):
             _torch().cuda.synchronize()  # the copies read converted temporaries
         del keep_p, keep_v
@@ -132,19 +147,19 @@ class NBodySystem:
     def get_state_device(self, pos_t, vel_t, stream=None):
         """Copy the state into the CUDA tensors pos_t, vel_t ((n, 4), the
         context's host dtype, contiguous: they are written in place)."""
+        dtype = self._torch_dtype()
         for t, name in ((pos_t, "pos_t"), (vel_t, "vel_t")):
-            if not (_is_torch(t) and t.is_cuda and t.is_contiguous() and tuple(t.shape) == (self.n, 4)
-                    and t.dtype == self._torch_dtype()):
+            if not (_is_torch(t) and t.is_cuda and t.is_contiguous() and t.shape == self._shape
+                    and t.dtype is dtype):
                 raise ValueError(f"{name}: needs a contiguous CUDA tensor of shape ({self.n}, 4) "
-                                 f"and dtype {self._torch_dtype()}")
+                                 f"and dtype {dtype}")
         s = current_stream_handle() if stream is None else stream
-        N.check(self.lib.nb_get_state(self.handle, C.c_void_p(pos_t.data_ptr()),
-                                      C.c_void_p(vel_t.data_ptr()), N.NB_DEVICE, C.c_void_p(s)),
+        N.check(self.lib.nb_get_state(self.handle, pos_t.data_ptr(), vel_t.data_ptr(), N.NB_DEVICE, s),
                 "nb_get_state")
 
     def step(self, steps=1, stream=None):
         s = current_stream_handle() if stream is None else stream
-        N.check(self.lib.nb_step(self.handle, int(steps), C.c_void_p(s)), "nb_step")
+        N.check(self.lib.nb_step(self.handle, int(steps), s), "nb_step")
 
     def set_params(self, eps2, damping, dt, G=1.0):
         """New eps2 (softening squared), damping, dt and G for the next steps
