@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(32 * WPB)
     const long long end = sk_start(w + 1, total, workers);
     if (it >= end) return;
     // eps2 in the scaled units (x 2^(2 kx)), as a float-float
-    const double e2s = ldexp(eps2, -2 * ff_exponent(range[0]));
+    const double e2s = mul_pow2(eps2, -2 * ff_exponent(range[0]));
     const float eh = __double2float_rn(e2s), el = __double2float_rn(e2s - (double)eh);
     int s = find_sys(bd.it_off, bd.nsys, it);
     while (it < end) {
@@ -461,9 +461,9 @@ __global__ void bksff_integrate_kernel(const double4 *__restrict__ pos_old, doub
         az = __dadd_rn(az, q.z);
     }
     const int k2 = ff_exponent(range[1]) - 2 * ff_exponent(range[0]);
-    ax = ldexp(ax, k2);
-    ay = ldexp(ay, k2);
-    az = ldexp(az, k2);
+    ax = mul_pow2(ax, k2);
+    ay = mul_pow2(ay, k2);
+    az = mul_pow2(az, k2);
     if (acc_out) {
         acc_out[i] = make_double4(ax, ay, az, 0.0);
         return;

@@ -217,8 +217,20 @@ __host__ __device__ __forceinline__ long long sk_start(long long c, long long to
 // CTA that owns iteration `it`: the largest c with start(c) <= it.
 __host__ __device__ __forceinline__ int sk_owner(long long it, long long total, int grid)
 {
-    return (int)(((it + 1) * (long long)grid - 1) / total);
+    const unsigned long long v = (unsigned long long)((it + 1) * (long long)grid - 1);
+    // 32-bit division where it will do: the 64-bit one is a dependent chain of
+    // more than a hundred instructions at the head of every integrator
+    if (((v | (unsigned long long)total) >> 32) == 0) return (int)((unsigned)v / (unsigned)total);
+    return (int)(v / (unsigned long long)total);
 }
+#ifdef __CUDACC__
+// ldexp(a, k), by one product with an exact power of two wherever that is a
+// normal number
+__device__ __forceinline__ double mul_pow2(double a, int k)
+{
+    return k >= -1022 && k <= 1023 ? a * __longlong_as_double((long long)(1023 + k) << 52) : ldexp(a, k);
+}
+#endif
 
 // Force-kernel variants: compensated (two-sum) tile accumulation writing
 // (hi, lo) partials, and the potential sum carried in w.

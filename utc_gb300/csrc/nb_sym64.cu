@@ -142,7 +142,10 @@ __global__ void __launch_bounds__(32 * W, MINB) sym64_force_kernel(const double4
 // in w when the force pass recorded it: the float-float energy pass).
 //
 // Reads all partials once (N^2 / (2 rb) double4), so memory and the narrow
-// FP64 pipe's additions bound it.  A block takes 32 bodies x 8 slices: slice
+// FP64 pipe's additions bound it; for small systems the chain of FP64
+// operations after the sums, which is why each component has a warp of its
+// own and fetches its old state first (N = 1000: 9.2 us with one warp doing
+// all of it and 64-bit divisions for the slots, now 6.5).  A block takes 32 bodies x 8 slices: slice
 // q sums slots c0 + q, c0 + q + 8, ... and rows q, q + 8, ... in order, and the
 // slices are added in slice order (fixed order: deterministic); the w sums
 // only where they are asked for.  With one thread per body the walk over up to
@@ -162,6 +165,21 @@ __global__ void __launch_bounds__(32 * kSym64Slices)
     // bodies from the last one down: the longest row walks start first
     const int i = n - 1 - (int)(blockIdx.x * 32 + lane);
     const bool want_w = acc_out != nullptr;
+    // what the warp's component q needs after the sums, fetched ahead of them
+    const size_t e = 4 * (size_t)(i < 0 ? 0 : i) + q;
+    unsigned long long scale[2] = {0, 0};
+    double xo = 0.0, m = 0.0, v = 0.0;
+    if (q < 4 && i >= 0) {
+        if (ffrange) {
+            scale[0] = ffrange[0];
+            scale[1] = ffrange[1];
+        }
+        if (!acc_out) {
+            xo = reinterpret_cast<const double *>(pos_old)[e];
+            m = pos_old[i].w;
+            if (q < 3) v = reinterpret_cast<const double *>(vel)[e];
+        }
+    }
     double ax = 0.0, ay = 0.0, az = 0.0, aw = 0.0;
     auto add = [&](const double4 &v) {
         ax = __dadd_rn(ax, v.x);
@@ -186,14 +204,12 @@ __global__ void __launch_bounds__(32 * kSym64Slices)
     red[2][q][lane] = az;
     red[3][q][lane] = aw;
     __syncthreads();
-    if (q != 0 || i < 0) return;
+    // warp q goes on with component q of the 32 bodies: x, y, z, and w (the
+    // potential, or what the step carries along)
+    if (q > 3 || i < 0) return;
+    double a = red[q][0][lane];
 #pragma unroll
-    for (int k = 1; k < kSym64Slices; ++k) {
-        ax = __dadd_rn(ax, red[0][k][lane]);
-        ay = __dadd_rn(ay, red[1][k][lane]);
-        az = __dadd_rn(az, red[2][k][lane]);
-        aw = __dadd_rn(aw, red[3][k][lane]);
-    }
+    for (int k = 1; k < kSym64Slices; ++k) a = __dadd_rn(a, red[q][k][lane]);
     if (ffrange) {
         // float-float path: its sums are in units scaled by 2^kx (positions)
         // and 2^km (masses), kx = -e(max |x|), km = -e(max m) with
@@ -203,31 +219,22 @@ __global__ void __launch_bounds__(32 * kSym64Slices)
             const int f = (int)((b >> 52) & 0x7ff);
             return (f == 0 || f == 0x7ff) ? 0 : f - 1022;
         };
-        const int em = ex(ffrange[1]), ex0 = ex(ffrange[0]);
-        const int k = em - 2 * ex0;
-        ax = ldexp(ax, k);
-        ay = ldexp(ay, k);
-        az = ldexp(az, k);
-        aw = ldexp(aw, em - ex0);
+        const int em = ex(scale[1]), ex0 = ex(scale[0]);
+        const int k = q < 3 ? em - 2 * ex0 : em - ex0;
+        a = mul_pow2(a, k);
     }
     if (acc_out) {
-        acc_out[i] = make_double4(ax, ay, az, aw);
+        reinterpret_cast<double *>(acc_out)[e] = a;
         return;
     }
-    double4 p = pos_old[i];
-    double4 v = vel[i];
-    const double k = kick == NB_KICK_REFERENCE ? p.w : G;
-    v.x = __dadd_rn(v.x, __dmul_rn(__dmul_rn(ax, k), dt));
-    v.y = __dadd_rn(v.y, __dmul_rn(__dmul_rn(ay, k), dt));
-    v.z = __dadd_rn(v.z, __dmul_rn(__dmul_rn(az, k), dt));
-    v.x = __dmul_rn(v.x, damping);
-    v.y = __dmul_rn(v.y, damping);
-    v.z = __dmul_rn(v.z, damping);
-    p.x = __dadd_rn(p.x, __dmul_rn(v.x, dt));
-    p.y = __dadd_rn(p.y, __dmul_rn(v.y, dt));
-    p.z = __dadd_rn(p.z, __dmul_rn(v.z, dt));
-    pos_new[i] = p;
-    vel[i] = v;
+    if (q < 3) {
+        const double k = kick == NB_KICK_REFERENCE ? m : G;
+        v = __dadd_rn(v, __dmul_rn(__dmul_rn(a, k), dt));
+        v = __dmul_rn(v, damping);
+        reinterpret_cast<double *>(vel)[e] = v;
+        xo = __dadd_rn(xo, __dmul_rn(v, dt));
+    }
+    reinterpret_cast<double *>(pos_new)[e] = xo;  // component 3: the mass
 }
 
 typedef void (*sym64_kernel_t)(const double4 *, int, double, double4 *, double4 *, long long, int, int);

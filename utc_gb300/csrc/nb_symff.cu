@@ -82,35 +82,95 @@ __global__ void ff_range_kernel(const double4 *__restrict__ pos, int n, unsigned
     }
 }
 
-// Scaled split: coordinates x * 2^kx (below 1 in magnitude) on the grids
-// H: 2^-20, M: 2^-44, L: 2^-68 (H + M + L == x * 2^kx exactly when
+// Scaled split of one body: coordinates x * 2^kx (below 1 in magnitude) on the
+// grids H: 2^-20, M: 2^-44, L: 2^-68 (H + M + L == x * 2^kx exactly when
 // |x * 2^kx| >= 2^-16, otherwise to 2^-69); the mass m * 2^km as the
-// float-float H + M (L unused).
-__global__ void ff_split_kernel(const double4 *__restrict__ pos, int n, const unsigned long long *__restrict__ range,
-                                float4 *__restrict__ H, float4 *__restrict__ M, float4 *__restrict__ L)
+// float-float H + M (L unused).  ex = -kx, em = -km; a sum with 1.5 * 2^(52 - g) leaves v rounded to the grid 2^-g.
+__device__ __forceinline__ void ff_split_body(const double4 &q, int ex, int em, float4 *H, float4 *M, float4 *L)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int kx = -ff_exponent(range[0]), km = -ff_exponent(range[1]);
-    const double4 q = pos[i];
-    const double v[4] = {ldexp(q.x, kx), ldexp(q.y, kx), ldexp(q.z, kx), ldexp(q.w, km)};
+    auto grid = [](double v, double c) { return __dsub_rn(__dadd_rn(v, c), c); };
+    const double v[4] = {mul_pow2(q.x, -ex), mul_pow2(q.y, -ex), mul_pow2(q.z, -ex), mul_pow2(q.w, -em)};
     float h[4], m[4], l[4];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const double gh = ldexp(rint(ldexp(v[k], 20)), -20);  // |gh| <= 1: 21 bits
-        const double r1 = v[k] - gh;                              // exact, |r1| <= 2^-21
-        const double gm = ldexp(rint(ldexp(r1, 44)), -44);       // 24 bits
-        const double r2 = r1 - gm;                                // exact, |r2| <= 2^-45
+        const double gh = grid(v[k], 0x1.8p32);   // |gh| <= 1: 21 bits
+        const double r1 = v[k] - gh;              // exact, |r1| <= 2^-21
+        const double gm = grid(r1, 0x1.8p8);      // 24 bits
+        const double r2 = r1 - gm;                // exact, |r2| <= 2^-45
         h[k] = (float)gh;
         m[k] = (float)gm;
-        l[k] = (float)ldexp(rint(ldexp(r2, 68)), -68);            // 24 bits
+        l[k] = (float)grid(r2, 0x1.8p-16);        // 24 bits
     }
     h[3] = __double2float_rn(v[3]);
     m[3] = __double2float_rn(v[3] - (double)h[3]);
     l[3] = 0.f;
-    H[i] = make_float4(h[0], h[1], h[2], h[3]);
-    M[i] = make_float4(m[0], m[1], m[2], m[3]);
-    L[i] = make_float4(l[0], l[1], l[2], l[3]);
+    *H = make_float4(h[0], h[1], h[2], h[3]);
+    *M = make_float4(m[0], m[1], m[2], m[3]);
+    *L = make_float4(l[0], l[1], l[2], l[3]);
+}
+
+// Latency bounds these two (some 40 dependent operations of the narrow FP64
+// pipe a body): small blocks, so that a small system spreads over many SMs.
+// With ldexp and rint in place of the products and sums, in blocks of 256, the
+// split took 10.8 us at N = 1000 to 8192; now 4.1 to 4.7.
+constexpr int kFFSplitBlock = 64;
+
+__global__ void __launch_bounds__(kFFSplitBlock) ff_split_kernel(const double4 *__restrict__ pos, int n,
+                                                                 const unsigned long long *__restrict__ range,
+                                                                 float4 *__restrict__ H, float4 *__restrict__ M,
+                                                                 float4 *__restrict__ L)
+{
+    const int i = blockIdx.x * kFFSplitBlock + threadIdx.x;
+    if (i >= n) return;
+    ff_split_body(pos[i], ff_exponent(range[0]), ff_exponent(range[1]), H + i, M + i, L + i);
+}
+
+// Range and split in one launch for small systems: every block finds the
+// largest coordinate and mass of all bodies for itself (only their exponents
+// are used, so the upper words do), instead of a memset and a reduction of
+// their own.  The redundant pass over the bodies costs 0.6 us per 1000 of them
+// against 3 us and two launches: 4.8 us at N = 1000, 6.7 at N = 4096, 10.1
+// at N = 8192, where the three launches take 3.0 + 4.1 us and the gaps between.
+constexpr int kFFFusedBlock = 256;
+constexpr int kFFFusedBodies = 6144;
+
+__global__ void __launch_bounds__(kFFFusedBlock) ff_range_split_kernel(const double4 *__restrict__ pos, int n,
+                                                                       unsigned long long *__restrict__ range,
+                                                                       float4 *__restrict__ H, float4 *__restrict__ M,
+                                                                       float4 *__restrict__ L)
+{
+    __shared__ unsigned red[2][kFFFusedBlock / 32];
+    const int i = blockIdx.x * kFFSplitBlock + threadIdx.x;
+    const bool own = threadIdx.x < kFFSplitBlock && i < n;
+    const double4 mine = own ? pos[i] : make_double4(0.0, 0.0, 0.0, 0.0);
+    auto top = [](double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; };
+    unsigned mc = 0, mm = 0;
+    for (int j = threadIdx.x; j < n; j += 8 * kFFFusedBlock) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const double4 q = pos[min(j + k * kFFFusedBlock, n - 1)];  // the last body again past the end
+            mc = max(mc, max(top(q.x), max(top(q.y), top(q.z))));
+            mm = max(mm, top(q.w));
+        }
+    }
+    mc = __reduce_max_sync(0xffffffffu, mc);
+    mm = __reduce_max_sync(0xffffffffu, mm);
+    if ((threadIdx.x & 31) == 0) {
+        red[0][threadIdx.x >> 5] = mc;
+        red[1][threadIdx.x >> 5] = mm;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kFFFusedBlock / 32; ++w) {
+        mc = max(mc, red[0][w]);
+        mm = max(mm, red[1][w]);
+    }
+    const unsigned long long rc = (unsigned long long)mc << 32, rm = (unsigned long long)mm << 32;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        range[0] = rc;
+        range[1] = rm;
+    }
+    if (own) ff_split_body(mine, ff_exponent(rc), ff_exponent(rm), H + i, M + i, L + i);
 }
 
 // One CTA's share of a row: row block I's targets against the chunks
@@ -222,7 +282,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
     constexpr int RC = RB / 32;
     const int c = blockIdx.x;
     // eps2 in the scaled units (x 2^(2 kx)), as a float-float
-    const double e2s = ldexp(eps2, -2 * ff_exponent(range[0]));
+    const double e2s = mul_pow2(eps2, -2 * ff_exponent(range[0]));
     const float eh = __double2float_rn(e2s), el = __double2float_rn(e2s - (double)eh);
     long long it = sk_start(c, total, gridDim.x);
     long long end = sk_start(c + 1, total, gridDim.x);
@@ -366,12 +426,17 @@ int ff_scale_split(const double4 *pos, int n, int sms, float4 *H, float4 *M, flo
                    cudaStream_t s)
 {
     if (n == 0) return NB_OK;
+    if (n <= kFFFusedBodies) {
+        ff_range_split_kernel<<<(n + kFFSplitBlock - 1) / kFFSplitBlock, kFFFusedBlock, 0, s>>>(pos, n, range, H, M, L);
+        NB_LAUNCH_CHECK("ff_range_split_kernel launch");
+        return NB_OK;
+    }
     NB_CUDA(cudaMemsetAsync(range, 0, 2 * sizeof(unsigned long long), s));
     const long long want = (n + 255) / 256, cap = 4ll * (sms > 0 ? sms : 1);
     const long long blocks = want < cap ? want : cap;
     ff_range_kernel<<<(unsigned)blocks, 256, 0, s>>>(pos, n, range);
     NB_LAUNCH_CHECK("ff_range_kernel launch");
-    ff_split_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(pos, n, range, H, M, L);
+    ff_split_kernel<<<(unsigned)((n + kFFSplitBlock - 1) / kFFSplitBlock), kFFSplitBlock, 0, s>>>(pos, n, range, H, M, L);
     NB_LAUNCH_CHECK("ff_split_kernel launch");
     return NB_OK;
 }
