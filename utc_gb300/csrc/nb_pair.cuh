@@ -68,9 +68,9 @@ struct PairTargets {
     }
 };
 
-// r = q - p and 1 / (|r|^2 + eps2)^(3/2) for a pair of targets
+// r = q - p, inv = 1 / (|r|^2 + eps2)^(1/2) and its cube for a pair of targets
 struct PairTerm {
-    f2 rx, ry, rz, inv3;
+    f2 rx, ry, rz, inv, inv3;
 };
 
 template <int NP>
@@ -85,23 +85,24 @@ __device__ __forceinline__ PairTerm pair_term(const PairTargets<NP> &t, int p, f
     d2 = f2_fma(o.rz, o.rz, d2);
     float lo, hi;
     f2_unpack(d2, lo, hi);
-    const f2 inv = f2_pack(rsqrt_approx(lo), rsqrt_approx(hi));
-    o.inv3 = f2_mul(inv, f2_mul(inv, inv));
+    o.inv = f2_pack(rsqrt_approx(lo), rsqrt_approx(hi));
+    o.inv3 = f2_mul(o.inv, f2_mul(o.inv, o.inv));
     return o;
 }
 
-template <int NP>
+template <int NP, bool ORDERED = false>
 __device__ __forceinline__ void pair_pull(PairTargets<NP> &t, int p, const PairTerm &r, f2 M)
 {
-    const f2 st = f2_mul(M, r.inv3);
+    const f2 st = ORDERED ? f2_mul(f2_mul(M, r.inv), f2_mul(r.inv, r.inv)) : f2_mul(M, r.inv3);
     t.ax[p] = f2_fma(r.rx, st, t.ax[p]);
     t.ay[p] = f2_fma(r.ry, st, t.ay[p]);
     t.az[p] = f2_fma(r.rz, st, t.az[p]);
 }
 
 // The pull of the 32 chunk bodies in sC on the lane's targets (a chunk inside
-// the targets' own row block: both orders of each pair occur there).
-template <int NP>
+// the targets' own row block: both orders of each pair occur there).  ORDERED: see
+// chunk_react; the weight is (m inv) inv^2.
+template <int NP, bool ORDERED = false>
 __device__ __forceinline__ void chunk_pull(PairTargets<NP> &t, const float4 *sC, f2 EPS2)
 {
 #pragma unroll 1
@@ -109,7 +110,7 @@ __device__ __forceinline__ void chunk_pull(PairTargets<NP> &t, const float4 *sC,
         const float4 q = sC[j];
         const f2 X = f2_pack(q.x, q.x), Y = f2_pack(q.y, q.y), Z = f2_pack(q.z, q.z), M = f2_pack(q.w, q.w);
 #pragma unroll
-        for (int p = 0; p < NP; ++p) pair_pull(t, p, pair_term(t, p, X, Y, Z, EPS2), M);
+        for (int p = 0; p < NP; ++p) pair_pull<NP, ORDERED>(t, p, pair_term(t, p, X, Y, Z, EPS2), M);
     }
 }
 
@@ -132,10 +133,19 @@ __device__ __forceinline__ float f2_fold(f2 v)
 // that body's reaction (one half per target of a pair, folded at the end),
 // passed on to lane l - 1 after the step.  Returns the reaction on chunk body
 // l from the warp's targets.
-template <int NP>
+//
+// ORDERED (the compensated kernel): the reaction is one sum over the targets in
+// their order.  A compensated step's state has twice the digits of its pair
+// terms, so the rounding of a 384-term sum in FP32 shows in its results: the
+// order is part of them (two chains folded at the end moved them by 1e-8 where
+// the forces are large).  Six scalar FMAs take the place of three packed
+// ones: two steps at N = 131071 take 10196 us, 10029 with the two chains, 11490
+// with the scalar loop.
+template <int NP, bool ORDERED = false>
 __device__ __forceinline__ float3 chunk_react(PairTargets<NP> &t, const float4 *sC, int lane, f2 EPS2)
 {
     f2 fx = f2_pack(0.f, 0.f), fy = fx, fz = fx;
+    float3 f = make_float3(0.f, 0.f, 0.f);  // ORDERED
     const int from = (lane + 1) & 31;
 #pragma unroll 8
     for (int r = 0; r < 32; ++r) {
@@ -146,15 +156,32 @@ __device__ __forceinline__ float3 chunk_react(PairTargets<NP> &t, const float4 *
             const PairTerm o = pair_term(t, p, X, Y, Z, EPS2);
             pair_pull(t, p, o, M);
             const f2 ss = f2_mul(t.nm[p], o.inv3);
-            fx = f2_fma(o.rx, ss, fx);
-            fy = f2_fma(o.ry, ss, fy);
-            fz = f2_fma(o.rz, ss, fz);
+            if constexpr (ORDERED) {
+                float s0, s1, r0, r1;
+                f2_unpack(ss, s0, s1);
+                f2_unpack(o.rx, r0, r1);
+                f.x = __fmaf_rn(r1, s1, __fmaf_rn(r0, s0, f.x));
+                f2_unpack(o.ry, r0, r1);
+                f.y = __fmaf_rn(r1, s1, __fmaf_rn(r0, s0, f.y));
+                f2_unpack(o.rz, r0, r1);
+                f.z = __fmaf_rn(r1, s1, __fmaf_rn(r0, s0, f.z));
+            } else {
+                fx = f2_fma(o.rx, ss, fx);
+                fy = f2_fma(o.ry, ss, fy);
+                fz = f2_fma(o.rz, ss, fz);
+            }
         }
-        fx = f2_shfl(fx, from);
-        fy = f2_shfl(fy, from);
-        fz = f2_shfl(fz, from);
+        if constexpr (ORDERED) {
+            f.x = __shfl_sync(0xffffffffu, f.x, from);
+            f.y = __shfl_sync(0xffffffffu, f.y, from);
+            f.z = __shfl_sync(0xffffffffu, f.z, from);
+        } else {
+            fx = f2_shfl(fx, from);
+            fy = f2_shfl(fy, from);
+            fz = f2_shfl(fz, from);
+        }
     }
-    return make_float3(f2_fold(fx), f2_fold(fy), f2_fold(fz));
+    return ORDERED ? f : make_float3(f2_fold(fx), f2_fold(fy), f2_fold(fz));
 }
 
 // Packed two-sum (Knuth): s + e == a + b exactly, s = fl(a + b).
