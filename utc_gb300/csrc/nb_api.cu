@@ -646,7 +646,11 @@ static int step_once(nb_ctx *c, cudaStream_t s, void *acc_out, cudaEvent_t *ev =
         if (!st && ev) NB_CUDA(cudaEventRecord(ev[2], s));
         return st;  // positions are updated in place: no ping-pong
     }
-    if (f64_sym(c)) {
+    if (ff_sym(c) && c->splan.small) {
+        st = nb::symff_small_step(c->splan, (const double4 *)po, acc_out ? nullptr : (double4 *)pn, (double4 *)c->vel,
+                                  p.eps2, p.damping, p.dt, p.kick, p.G, (double4 *)acc_out, c->ff_split, c->ff_range,
+                                  s);
+    } else if (f64_sym(c)) {
         st = ff_sym(c) ? nb::symff_force(c->splan, (const double4 *)po, p.eps2, c->ff_split, c->ff_range,
                                          (double4 *)c->sym_t, (double4 *)c->sym_s, (double4 *)c->sym_acc, s)
                        : nb::sym64_force(c->splan, (const double4 *)po, p.eps2, (double4 *)c->sym_t,
@@ -689,7 +693,7 @@ static int step_once(nb_ctx *c, cudaStream_t s, void *acc_out, cudaEvent_t *ev =
     }
     if (!st && ev) {
         // one fused kernel (exact, small symmetric systems): all of it is force time
-        if ((!uses_fast(c) && !f64_sym(c)) || (uses_sym(c) && c->splan.small)) NB_CUDA(cudaEventRecord(ev[1], s));
+        if ((!uses_fast(c) && !f64_sym(c)) || ((uses_sym(c) || ff_sym(c)) && c->splan.small)) NB_CUDA(cudaEventRecord(ev[1], s));
         NB_CUDA(cudaEventRecord(ev[2], s));
     }
     if (!st && !acc_out) c->cur ^= 1;
@@ -1272,7 +1276,11 @@ int nb_launches_per_step(nb_ctx *c)
     if (c->p.n == 0) return 0;
     // a banded symmetric plan: a force and a fold launch per band
     const int bands = (uses_sym(c) || comp_sym(c) || f64_sym(c)) && c->splan.nbands > 1 ? c->splan.nbands : 0;
-    if (ff_sym(c)) return 4 + (bands ? 2 * bands - 1 : 0);  // scale reduction, split, force, integrate
+    if (ff_sym(c)) {
+        // scale reduction and split (one launch for small systems), then force and integrate (likewise)
+        const int prep = c->p.n <= nb::kFFFusedBodies ? 1 : 2;
+        return prep + (c->splan.small ? 1 : 2) + (bands ? 2 * bands - 1 : 0);
+    }
     if (bands) return 2 * bands + 1;
     if (uses_sym(c) && c->splan.small) return 1;
     return (uses_fast(c) || is_comp(c) || f64_sym(c)) ? 2 : 1;

@@ -1575,6 +1575,9 @@ static int sys_step(const nb_batch *b, const SysPlans &sp, int i, int c, float4 
     if (b->f64) {
         const double4 *po = (const double4 *)b->pos[c] + o;
         double4 *pn = (double4 *)b->pos[c ^ 1] + o, *vel = (double4 *)b->vel + o;
+        if (sp.sym[i].small)
+            return nb::symff_small_step(sp.sym[i], po, pn, vel, p.eps2, p.damping, p.dt, p.kick, p.G, nullptr,
+                                        b->ff_split + 3 * (size_t)o, range, s);
         if ((st = nb::symff_force(sp.sym[i], po, p.eps2, b->ff_split + 3 * (size_t)o, range, (double4 *)tpart,
                                   (double4 *)spart, nullptr, s)))
             return st;

@@ -224,6 +224,29 @@ __host__ __device__ __forceinline__ int sk_owner(long long it, long long total, 
     return (int)(v / (unsigned long long)total);
 }
 #ifdef __CUDACC__
+// Launch of a kernel that begins with pdl_wait(): its blocks come in as those of
+// the stream's kernel before it leave, and wait there until that kernel is
+// complete and its writes are visible (0.4 us a launch less than a plain one).
+// No argument that the kernel before writes may be read through const
+// __restrict__: read-only loads may be moved ahead of the wait.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+int pdl_launch(const char *what, void (*k)(P...), unsigned grid, unsigned block, cudaStream_t s, A... a)
+{
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k, static_cast<P>(a)...);
+    return e == cudaSuccess ? NB_OK : cuda_error(e, what);
+}
+
 // ldexp(a, k), by one product with an exact power of two wherever that is a
 // normal number
 __device__ __forceinline__ double mul_pow2(double a, int k)
@@ -443,6 +466,15 @@ int sym64_integrate(const SymPlan &p, const double4 *pos_old, double4 *pos_new, 
 int symff_plan(int n, int warps, int bpt, int device, SymPlan *pl, int bands = 0);
 int symff_force(const SymPlan &p, const double4 *pos, double eps2, float4 *split, unsigned long long *range,
                 double4 *tpart, double4 *spart, double4 *accsum, cudaStream_t s, int phi = 0);
+// The step of a plan with `small` set: the preparation and one kernel for pairs,
+// sums and integration, or (pos_new == nullptr) only acc_out.  Its
+// potential pass is symff_force's.
+int symff_small_step(const SymPlan &p, const double4 *pos_old, double4 *pos_new, double4 *vel, double eps2,
+                     double damping, double dt, int kick, double G, double4 *acc_out, float4 *split,
+                     unsigned long long *range, cudaStream_t s);
+// Largest system whose preparation is one launch, and whose whole step is small
+constexpr int kFFFusedBodies = 6144;
+constexpr int kFFSmallBodies = 2400;
 // The float-float paths' per-step preparation: range (2 unsigned long long)
 // <- bits of the largest |coordinate| and |mass|; H + M + L <- the positions
 // and masses scaled by those powers of two, split into three floats.

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_step_kernel(const floa
     // writes visible.  It gives its dependents no earlier signal: blocks let
     // in before the SMs are free gather on those that empty first (N = 3000:
     // 6.6 us a step against 5.4; plain launches 5.65).
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_wait();
     // the body that this thread integrates
     const int mine = t0 + tid;
     const bool own = tid < TB && mine < n;
@@ -169,17 +169,8 @@ int small_step(int n, int sms, const float4 *pos_old, float4 *pos_new, float4 *v
     const int tb = small_targets(n, sms);
     auto k = tb == 4 ? small_step_kernel<4> : tb == 6 ? small_step_kernel<6> : tb == 8 ? small_step_kernel<8>
                                                                                        : small_step_kernel<10>;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((n + tb - 1) / tb));
-    cfg.blockDim = dim3(kSmallThreads);
-    cfg.stream = s;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    NB_CUDA(cudaLaunchKernelEx(&cfg, k, pos_old, pos_new, vel, n, eps2, damping, dt, kick, G, acc_out));
-    return NB_OK;
+    return pdl_launch("small_step_kernel launch", k, (unsigned)((n + tb - 1) / tb), kSmallThreads, s, pos_old, pos_new,
+                      vel, n, eps2, damping, dt, kick, G, acc_out);
 }
 
 }  // namespace nb

@@ -132,16 +132,14 @@ __global__ void __launch_bounds__(kFFSplitBlock) ff_split_kernel(const double4 *
 // against 3 us and two launches: 4.8 us at N = 1000, 6.7 at N = 4096, 10.1
 // at N = 8192, where the three launches take 3.0 + 4.1 us and the gaps between.
 constexpr int kFFFusedBlock = 256;
-constexpr int kFFFusedBodies = 6144;
 
-__global__ void __launch_bounds__(kFFFusedBlock) ff_range_split_kernel(const double4 *__restrict__ pos, int n,
-                                                                       unsigned long long *__restrict__ range,
-                                                                       float4 *__restrict__ H, float4 *__restrict__ M,
-                                                                       float4 *__restrict__ L)
+__global__ void __launch_bounds__(kFFFusedBlock) ff_range_split_kernel(const double4 *pos, int n, unsigned long long *range,
+                                                                       float4 *H, float4 *M, float4 *L)
 {
     __shared__ unsigned red[2][kFFFusedBlock / 32];
     const int i = blockIdx.x * kFFSplitBlock + threadIdx.x;
     const bool own = threadIdx.x < kFFSplitBlock && i < n;
+    pdl_wait();
     const double4 mine = own ? pos[i] : make_double4(0.0, 0.0, 0.0, 0.0);
     auto top = [](double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; };
     unsigned mc = 0, mm = 0;
@@ -380,6 +378,7 @@ int symff_plan(int n, int warps, int bpt, int device, SymPlan *pl, int bands)
     p.grid = p.total > 0 ? (int)grid : 0;
     p.slots = p.total > 0 ? p.grid + p.nrb - 1 : 0;
     p.sms = sms;
+    p.small = p.nbands == 1 && bands <= 1 && n > 0 && n <= kFFSmallBodies && warps == 1 && bpt == 2;
     *pl = p;
     return NB_OK;
 }
@@ -426,11 +425,9 @@ int ff_scale_split(const double4 *pos, int n, int sms, float4 *H, float4 *M, flo
                    cudaStream_t s)
 {
     if (n == 0) return NB_OK;
-    if (n <= kFFFusedBodies) {
-        ff_range_split_kernel<<<(n + kFFSplitBlock - 1) / kFFSplitBlock, kFFFusedBlock, 0, s>>>(pos, n, range, H, M, L);
-        NB_LAUNCH_CHECK("ff_range_split_kernel launch");
-        return NB_OK;
-    }
+    if (n <= kFFFusedBodies)
+        return pdl_launch("ff_range_split_kernel launch", ff_range_split_kernel,
+                          (unsigned)((n + kFFSplitBlock - 1) / kFFSplitBlock), kFFFusedBlock, s, pos, n, range, H, M, L);
     NB_CUDA(cudaMemsetAsync(range, 0, 2 * sizeof(unsigned long long), s));
     const long long want = (n + 255) / 256, cap = 4ll * (sms > 0 ? sms : 1);
     const long long blocks = want < cap ? want : cap;
@@ -439,6 +436,169 @@ int ff_scale_split(const double4 *pos, int n, int sms, float4 *H, float4 *M, flo
     ff_split_kernel<<<(unsigned)((n + kFFSplitBlock - 1) / kFFSplitBlock), kFFSplitBlock, 0, s>>>(pos, n, range, H, M, L);
     NB_LAUNCH_CHECK("ff_split_kernel launch");
     return NB_OK;
+}
+
+// ---------------------------------------------------------------------------
+// Small systems: the preparation, then the rest of the step in one launch (the
+// layout of nb_small.cu).  A CTA owns two bodies (a pair of the f32x2
+// arithmetic), its 128 threads split the sources, every pair is evaluated from
+// the target's side (140 operations, 1.5 times the work of the symmetric kernel
+// a pair of bodies, but no partial leaves the CTA and no item of 64 x 32 pairs
+// has to be found for every warp); the sums are reduced through the warps in
+// float-float and across them in FP64.
+//
+// Step time from a replayed graph, GB300, us, against the symmetric kernels:
+// N = 300 5.9 (17.4), 1000 11.8 (19.8), 1500 16.8 (20.8), 2000 25.8 (28.1),
+// 2300 31.9 (35.6), 2500 37.7 (36.4), 3000 47.5 (44.2): the line is at 2400.
+// Bounds: the chain preparation (3 us) - first loads - reduction while small,
+// then the FMA pipe and whole CTAs per SM (1000 bodies: 3.3 CTAs an SM on
+// average, 4 on most).  4 bodies a CTA: within 6 % either way; 256 threads: 4
+// to 15 % slower.
+constexpr int kFFSmallThreads = 128;
+constexpr int kFFSmallTargets = 2;
+
+__device__ __forceinline__ void ff_add1(float &h, float &l, float gh, float gl)
+{
+    float s, e;
+    two_sum(h, gh, s, e);
+    const float t = __fadd_rn(__fadd_rn(l, gl), e);
+    h = __fadd_rn(s, t);
+    l = __fsub_rn(t, __fsub_rn(h, s));
+}
+
+// Sums (h, l)[0..3 T) over the warp as warp_sum of nb_small.cu does: the lanes
+// halve the targets while there is more than one, and the lane's target is
+// returned.
+template <int T>
+__device__ __forceinline__ int ff_warp_sum(float *h, float *l, int lane)
+{
+    int mine = 0, off = 16;
+#pragma unroll
+    for (int half = T / 2; half >= 1; half /= 2) {
+        const bool up = (lane & off) != 0;
+        mine = 2 * mine + (up ? 1 : 0);
+#pragma unroll
+        for (int k = 0; k < 3 * half; ++k) {
+            const int o = 3 * half + k;
+            const float gh = up ? h[k] : h[o], gl = up ? l[k] : l[o];
+            h[k] = up ? h[o] : h[k];
+            l[k] = up ? l[o] : l[k];
+            ff_add1(h[k], l[k], __shfl_xor_sync(0xffffffffu, gh, off), __shfl_xor_sync(0xffffffffu, gl, off));
+        }
+        off /= 2;
+    }
+#pragma unroll
+    for (; off >= 1; off /= 2) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            ff_add1(h[k], l[k], __shfl_xor_sync(0xffffffffu, h[k], off), __shfl_xor_sync(0xffffffffu, l[k], off));
+    }
+    return mine;
+}
+
+template <int TB>
+__global__ void __launch_bounds__(kFFSmallThreads, 8 / TB)
+    symff_small_kernel(const float4 *H, const float4 *M, const float4 *L, const unsigned long long *range,
+                       const double *pos_old, double *pos_new, double *vel, int n, double eps2, double damping,
+                       double dt, int kick, double G, double *acc_out)
+{
+    constexpr int NP = TB / 2, NW = kFFSmallThreads / 32;
+    __shared__ double red[NW][3 * TB];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int t0 = blockIdx.x * TB;
+    // the component that this thread integrates
+    const int body = t0 + (tid >> 2), q = tid & 3;
+    const bool own = tid < 4 * TB && body < n;
+    const size_t e = 4 * (size_t)body + q;
+    pdl_wait();
+    const int ex = ff_exponent(range[0]), em = ff_exponent(range[1]);
+    double x = 0.0, m = 0.0, v = 0.0;
+    if (own && pos_new) {
+        x = pos_old[e];
+        m = pos_old[e - q + 3];
+        if (q < 3) v = vel[e];
+    }
+    const double e2s = mul_pow2(eps2, -2 * ex);
+    const float eh = __double2float_rn(e2s), el = __double2float_rn(e2s - (double)eh);
+    const f2 EH = ff_pack1(eh), EL = ff_pack1(el);
+    FFTargets<NP, false> T;
+    T.load(H, M, L, [&](int k) { return t0 + k < n ? t0 + k : -1; });
+    T.clear();
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 h = zero, mi = zero, lo = zero;
+    if (tid < n) {
+        h = H[tid];
+        mi = M[tid];
+        lo = L[tid];
+    }
+    bool odd = false;
+#pragma unroll 2
+    for (int j = tid; j < n; j += kFFSmallThreads) {
+        FFSource s;
+        s.load(h, mi, lo);
+        const int jn = j + kFFSmallThreads;
+        if (jn < n) {
+            h = H[jn];
+            mi = M[jn];
+            lo = L[jn];
+        }
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            FFPair w;
+            ff_pair<false>(s, T.t[p], EH, EL, w);
+            T.pull(p, w);
+        }
+        if (odd) T.norm();
+        odd = !odd;
+    }
+    T.norm();
+    float sh[3 * TB], sl[3 * TB];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        f2_unpack(T.ax[p].h, sh[6 * p], sh[6 * p + 3]);
+        f2_unpack(T.ax[p].l, sl[6 * p], sl[6 * p + 3]);
+        f2_unpack(T.ay[p].h, sh[6 * p + 1], sh[6 * p + 4]);
+        f2_unpack(T.ay[p].l, sl[6 * p + 1], sl[6 * p + 4]);
+        f2_unpack(T.az[p].h, sh[6 * p + 2], sh[6 * p + 5]);
+        f2_unpack(T.az[p].l, sl[6 * p + 2], sl[6 * p + 5]);
+    }
+    const int t = ff_warp_sum<TB>(sh, sl, lane);
+    if ((lane & (32 / TB - 1)) == 0) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) red[wid][3 * t + k] = (double)sh[k] + (double)sl[k];
+    }
+    __syncthreads();
+    if (!own) return;
+    double a = 0.0;
+    if (q < 3) {
+        a = red[0][3 * (tid >> 2) + q];
+#pragma unroll
+        for (int w = 1; w < NW; ++w) a = __dadd_rn(a, red[w][3 * (tid >> 2) + q]);
+        a = mul_pow2(a, em - 2 * ex);
+    }
+    if (acc_out) acc_out[e] = a;
+    if (!pos_new) return;
+    if (q < 3) {
+        const double k = kick == NB_KICK_REFERENCE ? m : G;
+        v = __dadd_rn(v, __dmul_rn(__dmul_rn(a, k), dt));
+        v = __dmul_rn(v, damping);
+        vel[e] = v;
+        x = __dadd_rn(x, __dmul_rn(v, dt));
+    }
+    pos_new[e] = x;
+}
+
+int symff_small_step(const SymPlan &p, const double4 *pos_old, double4 *pos_new, double4 *vel, double eps2,
+                     double damping, double dt, int kick, double G, double4 *acc_out, float4 *split,
+                     unsigned long long *range, cudaStream_t s)
+{
+    if (p.n == 0) return NB_OK;
+    float4 *H = split, *M = split + p.n, *L = split + 2 * (size_t)p.n;
+    if (int st = ff_scale_split(pos_old, p.n, p.sms, H, M, L, range, s)) return st;
+    return pdl_launch("symff_small_kernel launch", symff_small_kernel<kFFSmallTargets>,
+                      (unsigned)((p.n + kFFSmallTargets - 1) / kFFSmallTargets), kFFSmallThreads, s, H, M, L, range,
+                      (const double *)pos_old, (double *)pos_new, (double *)vel, p.n, eps2, damping, dt, kick, G,
+                      (double *)acc_out);
 }
 
 int symff_force(const SymPlan &p, const double4 *pos, double eps2, float4 *split, unsigned long long *range,
