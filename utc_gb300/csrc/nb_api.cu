@@ -1085,7 +1085,7 @@ static int adj_steps(nb_ctx *c, float4 *x, float4 *vel, float4 *acc, int len, cu
         const float4 *xk = x + (size_t)k * n;
         float4 *xn = x + (size_t)(k + 1) * n, *ak = ref ? acc + (size_t)k * n : nullptr;
         if (uses_sym(c) && c->splan.small) {
-            st = nb::small_step(p.n, c->splan.sms, xk, xn, vel, eps2, D, dt, p.kick, G, ak, s);
+            st = nb::small_step(p.n, 0, p.n, c->splan.sms, xk, xn, vel, eps2, D, dt, p.kick, G, ak, s);
         } else if (uses_sym(c)) {
             const float4 *sum = (const float4 *)c->sym_acc;
             st = nb::sym_force(c->splan, xk, eps2, c->sym_t, c->sym_s, (float4 *)c->sym_acc, s);

@@ -23,6 +23,7 @@
 //    quantisation).  A CTA writes one partial acceleration per target block
 //    it touches; a second, bandwidth-bound kernel sums the partials of each
 //    target in CTA order (deterministic) and applies the kick/drift update.
+//  * Systems too small for that to fill 152 SMs evenly run direct (kDirectBodies).
 #include <algorithm>
 
 #include "nb_pair.cuh"
@@ -203,13 +204,13 @@ __global__ void __launch_bounds__(NT, NPAIR == 1 ? 1024 / NT : 0) sk_force_kerne
 // Sum the partial slots of each target in CTA order, then the reference's
 // kick / damping / drift with unfused IEEE operations in its order
 // (bodysystem_kernel.cu:115-126).  Targets i_begin <= i < i_end.
-__global__ void sk_integrate_kernel(const float4 *__restrict__ pos_old, float4 *__restrict__ pos_new,
-                                    float4 *__restrict__ vel, const float4 *__restrict__ partial,
+__global__ void sk_integrate_kernel(const float4 *pos_old, float4 *pos_new, float4 *vel, const float4 *partial,
                                     int i_begin, int i_end, int tbsize, long long total, int ngroups,
                                     int grid, float damping, float dt, int kick, float G,
-                                    float4 *__restrict__ acc_out)
+                                    float4 *acc_out)
 {
     const int i = i_begin + blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
     if (i >= i_end) return;
     const int tb = i / tbsize;
     const int li = i - tb * tbsize;
@@ -217,6 +218,7 @@ __global__ void sk_integrate_kernel(const float4 *__restrict__ pos_old, float4 *
     const int c0 = sk_owner(first, total, grid);
     const int c1 = sk_owner(first + ngroups - 1, total, grid);
     float ax = 0.f, ay = 0.f, az = 0.f;
+#pragma unroll 8
     for (int c = c0; c <= c1; ++c) {
         const float4 q = partial[(size_t)(c + tb) * tbsize + li];
         ax = __fadd_rn(ax, q.x);
@@ -242,6 +244,16 @@ __global__ void sk_integrate_kernel(const float4 *__restrict__ pos_old, float4 *
     pos_new[i] = p;
     vel[i] = v;
 }
+
+// Largest system of the automatic shape that runs direct: the force launch is the
+// kernel of nb_small.cu, which sums each target in one CTA, so that the
+// integrator reads one partial per body in place of up to 60.  Graph-replayed
+// step, GB300, us, against the stream-K kernel: N = 300 3.5 (5.1), 1000 3.7 (7.3),
+// 4099 10.8 (22.7), 8192 29.7 (40.0), 12345 64 (70.5), 16384 105 (110), 24000 216
+// (224).  At 32768, with blocks of 256 threads, stream-K is ahead (387 against
+// 393): it pads targets less there, and its CTAs end together, while the
+// CTAs of a direct launch leave a ragged last wave.
+constexpr int kDirectBodies = 24576;
 
 // ---------------------------------------------------------------------------
 // dispatch over the compiled (threads per CTA, target pairs per thread) shapes
@@ -277,11 +289,10 @@ bool fast_shape_supported(int block, int bpt, int flags)
 int fast_plan(int n, int block, int bpt, int ctas_per_sm, int device, SkPlan *pl, int flags)
 {
     if (n < 0) return set_error(NB_ERR_INVALID, "n must be >= 0");
-    if (block == 0 || bpt == 0) {
-        // default shape: wide blocks for large N, finer granularity below
-        if (block == 0) block = n >= 32768 ? 256 : 128;
-        if (bpt == 0) bpt = n >= 8192 ? 8 : (n >= 2048 ? 4 : 2);
-    }
+    // default shape: wide blocks for large N, finer granularity below
+    const int auto_block = n >= 32768 ? 256 : 128, auto_bpt = n >= 8192 ? 8 : (n >= 2048 ? 4 : 2);
+    if (block == 0) block = auto_block;
+    if (bpt == 0) bpt = auto_bpt;
     sk_kernel_t k = sk_kernel_for(block, bpt, flags);
     if (!k) return set_error(NB_ERR_UNSUPPORTED, "fast kernel shape (block, bodies per thread) not compiled");
     SkPlan p;
@@ -301,6 +312,8 @@ int fast_plan(int n, int block, int bpt, int ctas_per_sm, int device, SkPlan *pl
     if (p.total > 0 && grid > p.total) grid = p.total;
     p.grid = p.total > 0 ? (int)grid : 0;
     p.slots = p.total > 0 ? p.grid + p.ntb - 1 : 0;
+    p.sms = sms;
+    p.direct = flags == 0 && ctas_per_sm == 0 && block == auto_block && bpt == auto_bpt && n <= kDirectBodies;
     *pl = p;
     return NB_OK;
 }
@@ -327,6 +340,9 @@ int fast_force(const SkPlan &p, const float4 *pos, float eps2, float4 *partial, 
     if (p.total == 0) return NB_OK;
     sk_kernel_t k = sk_kernel_for(p.block, p.bpt, flags);
     if (!k) return set_error(NB_ERR_UNSUPPORTED, "fast kernel shape not compiled for this variant");
+    if (p.direct)
+        return small_step(p.n, p.ranged ? p.i_lo : 0, p.ranged ? p.i_hi : p.n, p.sms, pos, nullptr, nullptr, eps2, 0.f,
+                          0.f, NB_KICK_PHYSICAL, 0.f, partial, s);
     const long long lo_offset = (long long)p.slots * p.tbsize;
     long long lo = 0, hi = p.total;
     int base = 0, ctas = p.grid;
@@ -348,12 +364,10 @@ int fast_integrate(const SkPlan &p, const float4 *pos_old, float4 *pos_new, floa
 {
     const int i0 = p.ranged ? p.i_lo : 0, i1 = p.ranged ? p.i_hi : p.n;
     if (i1 <= i0) return NB_OK;
-    const int bs = 256;
-    sk_integrate_kernel<<<(i1 - i0 + bs - 1) / bs, bs, 0, s>>>(pos_old, pos_new, vel, partial, i0, i1,
-                                                               p.tbsize, p.total, p.ngroups, p.grid,
-                                                               damping, dt, kick, G, acc_out);
-    NB_LAUNCH_CHECK("sk_integrate_kernel launch");
-    return NB_OK;
+    const SkLayout l = sk_layout(p);
+    return pdl_launch("sk_integrate_kernel launch", sk_integrate_kernel, (unsigned)((i1 - i0 + 127) / 128), 128, s,
+                      pos_old, pos_new, vel, partial, i0, i1, l.tbsize, l.total, l.ngroups, l.grid, damping, dt, kick,
+                      G, acc_out);
 }
 
 // ---------------------------------------------------------------------------

@@ -208,7 +208,24 @@ struct SkPlan {
     bool ranged = false;
     long long it_lo = 0, it_hi = 0;
     int i_lo = 0, i_hi = 0;
+    // one sum per target, at partial[target]: the force launch is small_step's
+    // kernel (nb_small.cu), no CTA's partials are shared out
+    bool direct = false;
+    int sms = 0;
 };
+
+// How a plan's partials are laid out, for the kernels that sum them: slot
+// c + tb of tbsize entries for CTA c's share of target block tb.  A direct plan
+// reads as one CTA with one block of all targets.
+struct SkLayout {
+    int tbsize, ngroups, grid;
+    long long total;
+};
+inline SkLayout sk_layout(const SkPlan &p)
+{
+    if (p.direct) return {0x7fffffff, 1, 1, 1};
+    return {p.tbsize, p.ngroups, p.grid, p.total};
+}
 
 __host__ __device__ __forceinline__ long long sk_start(long long c, long long total, int grid)
 {
@@ -435,9 +452,10 @@ int sym_integrate(const SymPlan &p, const float4 *pos_old, float4 *pos_new, floa
                   const float4 *tpart, const float4 *spart, const float4 *accsum, float eps2, float damping,
                   float dt, int kick, float G, float4 *acc_out, cudaStream_t s, int consume = 1);
 // One step (pos_new != nullptr) or the bare accelerations (acc_out), or both,
-// of a small system in one launch (nb_small.cu).
-int small_step(int n, int sms, const float4 *pos_old, float4 *pos_new, float4 *vel, float eps2, float damping,
-               float dt, int kick, float G, float4 *acc_out, cudaStream_t s);
+// of the targets [lo, hi) of n bodies in one launch (nb_small.cu); the split
+// changes no bit.
+int small_step(int n, int lo, int hi, int sms, const float4 *pos_old, float4 *pos_new, float4 *vel, float eps2,
+               float damping, float dt, int kick, float G, float4 *acc_out, cudaStream_t s);
 // Largest system that the automatic plan steps so.
 constexpr int kSmallBodies = 9000;
 // Fixed plans: zero the accumulators and write the record (the sum of |m| of

@@ -304,8 +304,9 @@ int fast_reduce(const SkPlan &p, const float4 *partial, int comp, const float4 *
 {
     if (p.n == 0) return NB_OK;
     const long long lo_off = (long long)p.slots * p.tbsize;
-    sk_reduce_kernel<<<(p.n + 255) / 256, 256, 0, s>>>(partial, p.n, p.tbsize, p.total, p.ngroups,
-                                                      p.grid, lo_off, comp, pos32, eps2, out32,
+    const SkLayout l = sk_layout(p);
+    sk_reduce_kernel<<<(p.n + 255) / 256, 256, 0, s>>>(partial, p.n, l.tbsize, l.total, l.ngroups,
+                                                      l.grid, lo_off, comp, pos32, eps2, out32,
                                                       out64);
     NB_LAUNCH_CHECK("sk_reduce_kernel launch");
     return NB_OK;

@@ -9,7 +9,10 @@
 // are evaluated, 12 FP32 operations and one rsqrt each: twice the pair terms,
 // but no partial leaves the CTA), the sums are reduced through the warps and
 // the CTA's first threads apply the kick / damping / drift.  No scratch, no
-// second launch, fixed order of summation: deterministic.
+// second launch, fixed order of summation: deterministic.  A target's sum
+// depends neither on its place in a CTA nor on TB (each thread's sources and the
+// tree over the threads are the same), so shards of the targets give the same
+// bits.  Direct plans of nb_fast.cu use it for their force launch.
 //
 // Step time from a replayed graph, GB300, us, against the two launches:
 // N = 512 1.8 (6.4), 1024 2.2 (7.1), 2048 3.6 (9.2), 3000 5.4 (12.8), 4099
@@ -63,7 +66,7 @@ __device__ __forceinline__ int warp_sum(float *v, int lane)
 template <int TB>
 __global__ void __launch_bounds__(kSmallThreads, 1) small_step_kernel(const float4 *pos_old,
                                                                    float4 *__restrict__ pos_new,
-                                                                   float4 *__restrict__ vel, int n, float eps2,
+                                                                   float4 *__restrict__ vel, int n, int lo, int hi, float eps2,
                                                                    float damping, float dt, int kick, float G,
                                                                    float4 *__restrict__ acc_out)
 {
@@ -71,7 +74,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_step_kernel(const floa
     constexpr int NW = kSmallThreads / 32;
     __shared__ float red[NW][3 * TP];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int t0 = blockIdx.x * TB;
+    const int t0 = lo + blockIdx.x * TB;
     const float4 pad = make_float4(kPadCoord, kPadCoord, kPadCoord, 0.f);
     const f2 EPS2 = f2_pack(eps2, eps2);
     // A programmatic launch: the blocks come in as those of the previous step's
@@ -82,7 +85,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_step_kernel(const floa
     pdl_wait();
     // the body that this thread integrates
     const int mine = t0 + tid;
-    const bool own = tid < TB && mine < n;
+    const bool own = tid < TB && mine < hi;
     float4 p = pad, v = pad;
     if (own) {
         p = pos_old[mine];
@@ -145,10 +148,12 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_step_kernel(const floa
 // to do: ceil(CTAs / SMs) CTAs of TB bodies each, plus 0.9 of a body's work per
 // CTA for its pass over the sources and its reduction (measured for 4 to 16
 // bodies at twelve sizes: N = 3000 6.0 us with 10 bodies, 6.5 with 8, 6.7
-// with 6; N = 6000 15.9 with 8, 17.3 with 6).
+// with 6; N = 6000 15.9 with 8, 17.3 with 6).  Above kSmallBodies 8: N = 12345 62.5
+// us (6: 62.9, 10: 64.4, 12: 65.8, 16: 75.9), N = 20000 153.6 (10: 158.5).
 static int small_targets(int n, int sms)
 {
     if (n < 2000) return 4;
+    if (n > kSmallBodies) return 8;
     int best = 8;
     float least = 1e30f;
     for (int tb = 6; tb <= 10; tb += 2) {
@@ -162,15 +167,15 @@ static int small_targets(int n, int sms)
     return best;
 }
 
-int small_step(int n, int sms, const float4 *pos_old, float4 *pos_new, float4 *vel, float eps2, float damping,
-               float dt, int kick, float G, float4 *acc_out, cudaStream_t s)
+int small_step(int n, int lo, int hi, int sms, const float4 *pos_old, float4 *pos_new, float4 *vel, float eps2,
+               float damping, float dt, int kick, float G, float4 *acc_out, cudaStream_t s)
 {
-    if (n == 0) return NB_OK;
-    const int tb = small_targets(n, sms);
+    if (hi <= lo) return NB_OK;
+    const int tb = small_targets(hi - lo, sms);
     auto k = tb == 4 ? small_step_kernel<4> : tb == 6 ? small_step_kernel<6> : tb == 8 ? small_step_kernel<8>
                                                                                        : small_step_kernel<10>;
-    return pdl_launch("small_step_kernel launch", k, (unsigned)((n + tb - 1) / tb), kSmallThreads, s, pos_old, pos_new,
-                      vel, n, eps2, damping, dt, kick, G, acc_out);
+    return pdl_launch("small_step_kernel launch", k, (unsigned)((hi - lo + tb - 1) / tb), kSmallThreads, s, pos_old, pos_new,
+                      vel, n, lo, hi, eps2, damping, dt, kick, G, acc_out);
 }
 
 }  // namespace nb

@@ -717,7 +717,7 @@ int sym_integrate(const SymPlan &p, const float4 *pos_old, float4 *pos_new, floa
 {
     if (p.n == 0) return NB_OK;
     if (p.small)
-        return small_step(p.n, p.sms, pos_old, acc_out ? nullptr : pos_new, vel, eps2, damping, dt, kick, G, acc_out, s);
+        return small_step(p.n, 0, p.n, p.sms, pos_old, acc_out ? nullptr : pos_new, vel, eps2, damping, dt, kick, G, acc_out, s);
     if (p.nbands > 1 && !accsum) return set_error(NB_ERR_INVALID, "sym_integrate: a banded plan needs its per-body sums");
     const long long threads = 4ll * p.n;  // a quad of threads per body
     unsigned long long *fxacc =
