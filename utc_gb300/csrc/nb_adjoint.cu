@@ -279,21 +279,14 @@ __global__ void __launch_bounds__(kAdjUpdBlock) adj_update_sym_kernel(
         const int c0 = sk_owner(sym_prefix(I, nc, rc), total, grid);
         const int c1 = sk_owner(sym_prefix(I + 1, nc, rc) - 1, total, grid);
         const int li = i - I * rb;
-        for (int c = c0 + q; c <= c1; c += 4) {
-            const float4 v4 = tpart[(size_t)(c + I) * rb + li];
+        auto add = [&](const float4 &v4) {
             ox += v4.x;
             oy += v4.y;
             oz += v4.z;
             odm += v4.w;
-        }
-#pragma unroll 4
-        for (int r = q; r < I; r += 4) {
-            const float4 v4 = spart[sym_soff(r, n, rb) + (i - (long long)(r + 1) * rb)];
-            ox += v4.x;
-            oy += v4.y;
-            oz += v4.z;
-            odm += v4.w;
-        }
+        };
+        walk<4>(c0 + q, c1, 4, [&](int c) { return tpart[(size_t)(c + I) * rb + li]; }, add);
+        walk<4>(q, I - 1, 4, [&](int r) { return spart[sym_soff(r, n, rb) + (i - (long long)(r + 1) * rb)]; }, add);
     }
 #pragma unroll
     for (int m = 1; m <= 2; m <<= 1) {

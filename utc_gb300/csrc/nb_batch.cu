@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "nb_ff.cuh"
+#include "nb_integ.cuh"
 #include "nb_vjp.cuh"
 
 namespace nb {
@@ -182,12 +183,12 @@ __global__ void bk_integrate_kernel(const float4 *__restrict__ pos_old, float4 *
     const long long gtb = (long long)bd.tb_off[s] + tbl;
     const int lj = li - tbl * wtb;
     float ax = 0.f, ay = 0.f, az = 0.f;
-    for (int c = c0; c <= c1; ++c) {
-        const float4 q = partial[(c + gtb) * wtb + lj];
-        ax = __fadd_rn(ax, q.x);
-        ay = __fadd_rn(ay, q.y);
-        az = __fadd_rn(az, q.z);
-    }
+    walk<8>(c0, c1, 1, [&](int c) { return partial[(c + gtb) * wtb + lj]; },
+            [&](const float4 &q) {
+                ax = __fadd_rn(ax, q.x);
+                ay = __fadd_rn(ay, q.y);
+                az = __fadd_rn(az, q.z);
+            });
     batch_kick_drift(i, ax, ay, az, pos_old, pos_new, vel, damping, dt, kick, G, acc_out);
 }
 
@@ -276,16 +277,15 @@ __global__ void __launch_bounds__(32 * WPB, 8 / WPB) bks_force_kernel(const floa
     }
 }
 
-// Per body: target-side slots of its row (warp order), then the source-side
-// entries of rows 0..I-1 of its system (row order), then kick / drift.
-__global__ void bks_integrate_kernel(const float4 *__restrict__ pos_old, float4 *__restrict__ pos_new,
-                                     float4 *__restrict__ vel, const float4 *__restrict__ tpart,
-                                     const float4 *__restrict__ spart, BatchSymDev bd, int nbody, int rb,
-                                     long long total, int workers, float damping, float dt, int kick,
-                                     float G, float4 *__restrict__ acc_out)
+// The slot and source-side sums of one body by Q threads (4, as in
+// sym_integrate_kernel, or 1): thread q takes every Qth slot of the body's row
+// (warp order) and every Qth of the entries of rows 0..I-1 of its system (row
+// order); four are added pairwise.  add(v) takes a partial.
+template <int Q, class Add>
+__device__ __forceinline__ void bks_walk(int i, int q, const float4 *__restrict__ tpart,
+                                              const float4 *__restrict__ spart, const BatchSymDev &bd, int rb,
+                                              long long total, int workers, Add add)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nbody) return;
     const int s = bd.body_sys[i];
     const int o = bd.sys_off[s];
     const int ns = bd.sys_off[s + 1] - o;
@@ -298,21 +298,51 @@ __global__ void bks_integrate_kernel(const float4 *__restrict__ pos_old, float4 
     const int c1 = sk_owner(base + sym_prefix(I + 1, nc, rc) - 1, total, workers);
     const long long grow = (long long)bd.row_off[s] + I;
     const int lj = li - I * rb;
+    walk<4>(c0 + q, c1, Q, [&](int c) { return tpart[(c + grow) * rb + lj]; }, add);
+    const float4 *sp = spart + bd.sp_off[s];
+    walk<4>(q, I - 1, Q, [&](int r) { return sp[sym_soff(r, ns, rb) + (li - (long long)(r + 1) * rb)]; }, add);
+}
+
+// Batches of at most this many bodies take a quad per body, larger ones a thread:
+// 25000 bodies (18 systems) 5.8 us with quads and 7.9 without, 90000 9.6 and 5.8,
+// 716000 54 and 24.
+constexpr int kFewBodies = 32768;
+
+template <int Q>
+__device__ __forceinline__ float quad_sum(float v)
+{
+    if (Q == 1) return v;
+    v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
+    return __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 2));
+}
+
+// Per body: the sums, then kick / drift.  With one thread per body and a plain
+// loop the walk over slots and rows was a chain of loads (18 systems of 591 to
+// 2703 bodies: 13.5 us beside 20 us of force).
+template <int Q>
+__global__ void __launch_bounds__(256) bks_integrate_kernel(const float4 *__restrict__ pos_old,
+                                                            float4 *__restrict__ pos_new, float4 *__restrict__ vel,
+                                                            const float4 *__restrict__ tpart,
+                                                            const float4 *__restrict__ spart, BatchSymDev bd,
+                                                            int nbody, int rb, long long total, int workers,
+                                                            float damping, float dt, int kick, float G,
+                                                            float4 *__restrict__ acc_out)
+{
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int q = (int)(t % Q);
+    const bool live = t / Q < nbody;  // dead threads still take part in the shuffles
+    const int i = live ? (int)(t / Q) : 0;
     float ax = 0.f, ay = 0.f, az = 0.f;
-    for (int c = c0; c <= c1; ++c) {
-        const float4 q = tpart[(c + grow) * rb + lj];
-        ax = __fadd_rn(ax, q.x);
-        ay = __fadd_rn(ay, q.y);
-        az = __fadd_rn(az, q.z);
-    }
-    long long off = bd.sp_off[s] + li - rb;  // row r at soff(r) + li - (r + 1) rb
-    for (int r = 0; r < I; ++r) {
-        const float4 q = spart[off];
-        off += (long long)ns - (long long)(r + 2) * rb;
-        ax = __fadd_rn(ax, q.x);
-        ay = __fadd_rn(ay, q.y);
-        az = __fadd_rn(az, q.z);
-    }
+    if (live)
+        bks_walk<Q>(i, q, tpart, spart, bd, rb, total, workers, [&](const float4 &v) {
+            ax = __fadd_rn(ax, v.x);
+            ay = __fadd_rn(ay, v.y);
+            az = __fadd_rn(az, v.z);
+        });
+    ax = quad_sum<Q>(ax);
+    ay = quad_sum<Q>(ay);
+    az = quad_sum<Q>(az);
+    if (!live || q != 0) return;
     batch_kick_drift(i, ax, ay, az, pos_old, pos_new, vel, damping, dt, kick, G, acc_out);
 }
 
@@ -420,68 +450,46 @@ __global__ void __launch_bounds__(32 * WPB)
 }
 
 // Per body: FP64 sums of the target-side slots of its row (warp order) and
-// the source-side entries of rows 0..I-1 of its system (row order), the
-// batch's scaling undone (a = a_scaled * 2^(2 kx - km), exact), then the
-// reference's kick / damping / drift in its order with unfused IEEE
-// operations (bodysystem.cc:135-182), or the bare acceleration.
-__global__ void bksff_integrate_kernel(const double4 *__restrict__ pos_old, double4 *__restrict__ pos_new,
-                                       double4 *__restrict__ vel, const double4 *__restrict__ tpart,
-                                       const double4 *__restrict__ spart, BatchSymDev bd, int nbody, int rb,
-                                       long long total, int workers, double damping, double dt, int kick,
-                                       double G, const unsigned long long *__restrict__ range,
-                                       double4 *__restrict__ acc_out)
+// the source-side entries of rows 0..I-1 of its system (row order), every
+// eighth of them by each warp (integrate64), the batch's scaling undone (a =
+// a_scaled * 2^(2 kx - km), exact), then kick / damping / drift or the bare
+// acceleration.
+// Four warps a block: 53000 bodies 14.5 us, 150000 24.5 us (eight warps 22 and 35,
+// one thread per body 18.1 and 28.3).
+constexpr int kBatchSlices = 4;
+
+__global__ void __launch_bounds__(32 * kBatchSlices)
+    bksff_integrate_kernel(const double4 *__restrict__ pos_old, double4 *__restrict__ pos_new,
+                           double4 *__restrict__ vel, const double4 *__restrict__ tpart,
+                           const double4 *__restrict__ spart, BatchSymDev bd, int nbody, int rb, long long total,
+                           int workers, double damping, double dt, int kick, double G,
+                           const unsigned long long *__restrict__ range, double4 *__restrict__ acc_out)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nbody) return;
-    const int s = bd.body_sys[i];
-    const int o = bd.sys_off[s];
-    const int ns = bd.sys_off[s + 1] - o;
-    const int li = i - o;
-    const int rc = rb / 32;
-    const int nc = (ns + 31) / 32;
-    const int I = li / rb;
-    const long long base = bd.it_off[s];
-    const int c0 = sk_owner(base + sym_prefix(I, nc, rc), total, workers);
-    const int c1 = sk_owner(base + sym_prefix(I + 1, nc, rc) - 1, total, workers);
-    const long long grow = (long long)bd.row_off[s] + I;
-    const int lj = li - I * rb;
-    double ax = 0.0, ay = 0.0, az = 0.0;
-    for (int c = c0; c <= c1; ++c) {
-        const double4 q = tpart[(c + grow) * rb + lj];
-        ax = __dadd_rn(ax, q.x);
-        ay = __dadd_rn(ay, q.y);
-        az = __dadd_rn(az, q.z);
-    }
-    long long off = bd.sp_off[s] + li - rb;  // row r at soff(r) + li - (r + 1) rb
-    for (int r = 0; r < I; ++r) {
-        const double4 q = spart[off];
-        off += (long long)ns - (long long)(r + 2) * rb;
-        ax = __dadd_rn(ax, q.x);
-        ay = __dadd_rn(ay, q.y);
-        az = __dadd_rn(az, q.z);
-    }
+    const int b = blockIdx.x * 32 + (threadIdx.x & 31);
+    const int i = b < nbody ? b : -1;
     const int k2 = ff_exponent(range[1]) - 2 * ff_exponent(range[0]);
-    ax = mul_pow2(ax, k2);
-    ay = mul_pow2(ay, k2);
-    az = mul_pow2(az, k2);
-    if (acc_out) {
-        acc_out[i] = make_double4(ax, ay, az, 0.0);
-        return;
-    }
-    double4 p = pos_old[i];
-    double4 v = vel[i];
-    const double k = kick == NB_KICK_REFERENCE ? p.w : G;
-    v.x = __dadd_rn(v.x, __dmul_rn(__dmul_rn(ax, k), dt));
-    v.y = __dadd_rn(v.y, __dmul_rn(__dmul_rn(ay, k), dt));
-    v.z = __dadd_rn(v.z, __dmul_rn(__dmul_rn(az, k), dt));
-    v.x = __dmul_rn(v.x, damping);
-    v.y = __dmul_rn(v.y, damping);
-    v.z = __dmul_rn(v.z, damping);
-    p.x = __dadd_rn(p.x, __dmul_rn(v.x, dt));
-    p.y = __dadd_rn(p.y, __dmul_rn(v.y, dt));
-    p.z = __dadd_rn(p.z, __dmul_rn(v.z, dt));
-    pos_new[i] = p;
-    vel[i] = v;
+    integrate64<kBatchSlices>(
+        i,
+        [&](int q, auto add) {
+            const int s = bd.body_sys[i];
+            const int o = bd.sys_off[s];
+            const int ns = bd.sys_off[s + 1] - o;
+            const int li = i - o;
+            const int rc = rb / 32;
+            const int nc = (ns + 31) / 32;
+            const int I = li / rb;
+            const long long base = bd.it_off[s];
+            const int c0 = sk_owner(base + sym_prefix(I, nc, rc), total, workers);
+            const int c1 = sk_owner(base + sym_prefix(I + 1, nc, rc) - 1, total, workers);
+            const long long grow = (long long)bd.row_off[s] + I;
+            const int lj = li - I * rb;
+            for (int c = c0 + q; c <= c1; c += kBatchSlices) add(tpart[(c + grow) * rb + lj]);
+            const double4 *sp = spart + bd.sp_off[s];
+#pragma unroll 4
+            for (int r = q; r < I; r += kBatchSlices) add(sp[sym_soff(r, ns, rb) + (li - (long long)(r + 1) * rb)]);
+        },
+        [&](int q, double a) { return q < 3 ? mul_pow2(a, k2) : a; }, pos_old, pos_new, vel, damping, dt, kick, G,
+        acc_out);
 }
 
 typedef void (*bksff_kernel_t)(const float4 *, const float4 *, const float4 *, BatchSymDev, double,
@@ -721,46 +729,33 @@ __global__ void __launch_bounds__(32 * WPB, 8 / WPB) bks_vjp_kernel(const float4
     }
 }
 
-// Symmetric batched reverse-step update: target-side slots (warp order) and
-// source-side rows (row order) of the body's system, then the per-body update.
-__global__ void bks_adj_update_kernel(const float4 *__restrict__ tpart, const float4 *__restrict__ spart,
+// Symmetric batched reverse-step update: target-side slots and source-side rows
+// of the body's system (a quad of threads per body), then the per-body update.
+template <int Q>
+__global__ void __launch_bounds__(256) bks_adj_update_kernel(const float4 *__restrict__ tpart, const float4 *__restrict__ spart,
                                       BatchSymDev bd, int nbody, int rb, long long total, int workers,
                                       const float4 *__restrict__ pos, const float4 *__restrict__ acc,
                                       float4 *__restrict__ lx, float4 *__restrict__ lv,
                                       float *__restrict__ gm, float4 *__restrict__ gbuf, float damping,
                                       float dt, int kick, float G, int want_next_g)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nbody) return;
-    const int s = bd.body_sys[i];
-    const int o = bd.sys_off[s];
-    const int ns = bd.sys_off[s + 1] - o;
-    const int li = i - o;
-    const int rc = rb / 32;
-    const int nc = (ns + 31) / 32;
-    const int I = li / rb;
-    const long long base = bd.it_off[s];
-    const int c0 = sk_owner(base + sym_prefix(I, nc, rc), total, workers);
-    const int c1 = sk_owner(base + sym_prefix(I + 1, nc, rc) - 1, total, workers);
-    const long long grow = (long long)bd.row_off[s] + I;
-    const int lj = li - I * rb;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int q = (int)(t % Q);
+    const bool live = t / Q < nbody;  // dead threads still take part in the shuffles
+    const int i = live ? (int)(t / Q) : 0;
     float ox = 0.f, oy = 0.f, oz = 0.f, odm = 0.f;
-    for (int c = c0; c <= c1; ++c) {
-        const float4 qv = tpart[(c + grow) * rb + lj];
-        ox += qv.x;
-        oy += qv.y;
-        oz += qv.z;
-        odm += qv.w;
-    }
-    long long off = bd.sp_off[s] + li - rb;  // row r at soff(r) + li - (r + 1) rb
-    for (int r = 0; r < I; ++r) {
-        const float4 qv = spart[off];
-        off += (long long)ns - (long long)(r + 2) * rb;
-        ox += qv.x;
-        oy += qv.y;
-        oz += qv.z;
-        odm += qv.w;
-    }
+    if (live)
+        bks_walk<Q>(i, q, tpart, spart, bd, rb, total, workers, [&](const float4 &v) {
+            ox += v.x;
+            oy += v.y;
+            oz += v.z;
+            odm += v.w;
+        });
+    ox = quad_sum<Q>(ox);
+    oy = quad_sum<Q>(oy);
+    oz = quad_sum<Q>(oz);
+    odm = quad_sum<Q>(odm);
+    if (!live || q != 0) return;
     adj_body_update(i, ox, oy, oz, odm, pos, acc, lx, lv, gm, gbuf, damping, dt, kick, G, want_next_g);
 }
 
@@ -1011,7 +1006,7 @@ static int batch_integrate(nb_batch *b, const float4 *po, float4 *pn, float4 *ve
     if (!b->plan_ok)
         return set_error(NB_ERR_STATE, "batch has no valid launch plan (a plan change or autotune failed)");
     if (b->f64) {
-        nb::bksff_integrate_kernel<<<(b->nbody + 255) / 256, 256, 0, s>>>(
+        nb::bksff_integrate_kernel<<<(b->nbody + 31) / 32, 32 * nb::kBatchSlices, 0, s>>>(
             (const double4 *)po, (double4 *)pn, (double4 *)vel, (const double4 *)b->partial,
             (const double4 *)b->spart, batch_sym_dev(b), b->nbody, 32 * p.bpt, p.total, p.workers, b->p.damping,
             b->p.dt, b->p.kick, b->p.G, b->ff_range, (double4 *)acc_out);
@@ -1019,7 +1014,9 @@ static int batch_integrate(nb_batch *b, const float4 *po, float4 *pn, float4 *ve
         return NB_OK;
     }
     if (b->sym) {
-        nb::bks_integrate_kernel<<<(b->nbody + 255) / 256, 256, 0, s>>>(
+        const bool few = b->nbody <= nb::kFewBodies;
+        auto kern = few ? nb::bks_integrate_kernel<4> : nb::bks_integrate_kernel<1>;
+        kern<<<(unsigned)(((few ? 4ll : 1ll) * b->nbody + 255) / 256), 256, 0, s>>>(
             po, pn, vel, b->partial, b->spart, batch_sym_dev(b), b->nbody, 32 * p.bpt, p.total,
             p.workers, (float)b->p.damping, (float)b->p.dt, b->p.kick, (float)b->p.G, acc_out);
         NB_LAUNCH_CHECK("bks_integrate_kernel launch");
@@ -1866,7 +1863,9 @@ int nb_batch_adj_backward(nb_batch *b, unsigned long long generation, const void
                                                          vp.total, vp.workers);
                     NB_LAUNCH_CHECK("bks_vjp_kernel launch");
                 }
-                nb::bks_adj_update_kernel<<<(b->nbody + 255) / 256, 256, 0, s>>>(
+                const bool few = b->nbody <= nb::kFewBodies;
+                auto kern = few ? nb::bks_adj_update_kernel<4> : nb::bks_adj_update_kernel<1>;
+                kern<<<(unsigned)(((few ? 4ll : 1ll) * b->nbody + 255) / 256), 256, 0, s>>>(
                     b->vpartial, b->vspart, vsd, b->nbody, 32 * vp.bpt, vp.total, vp.workers, xk, ak, b->lx,
                     b->lv, b->gm, b->gbuf, D, dt, p.kick, G, more ? 1 : 0);
                 NB_LAUNCH_CHECK("bks_adj_update_kernel launch");

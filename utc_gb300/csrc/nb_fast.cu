@@ -218,13 +218,12 @@ __global__ void sk_integrate_kernel(const float4 *pos_old, float4 *pos_new, floa
     const int c0 = sk_owner(first, total, grid);
     const int c1 = sk_owner(first + ngroups - 1, total, grid);
     float ax = 0.f, ay = 0.f, az = 0.f;
-#pragma unroll 8
-    for (int c = c0; c <= c1; ++c) {
-        const float4 q = partial[(size_t)(c + tb) * tbsize + li];
-        ax = __fadd_rn(ax, q.x);
-        ay = __fadd_rn(ay, q.y);
-        az = __fadd_rn(az, q.z);
-    }
+    walk<8>(c0, c1, 1, [&](int c) { return partial[(size_t)(c + tb) * tbsize + li]; },
+            [&](const float4 &q) {
+                ax = __fadd_rn(ax, q.x);
+                ay = __fadd_rn(ay, q.y);
+                az = __fadd_rn(az, q.z);
+            });
     if (acc_out) {
         acc_out[i] = make_float4(ax, ay, az, 0.f);
         return;

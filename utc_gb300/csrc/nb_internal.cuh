@@ -264,6 +264,22 @@ int pdl_launch(const char *what, void (*k)(P...), unsigned grid, unsigned block,
     return e == cudaSuccess ? NB_OK : cuda_error(e, what);
 }
 
+// add(load(c)) for c = first, first + step, ... <= last, in that order, with B loads
+// in flight: a loop left to the compiler takes the last ones, and where the sums
+// are compensated all of them, one at a time.
+template <int B, class Load, class Add>
+__device__ __forceinline__ void walk(int first, int last, int step, Load load, Add add)
+{
+    for (int c = first; c <= last; c += B * step) {
+        decltype(load(0)) v[B];
+#pragma unroll
+        for (int k = 0; k < B; ++k) v[k] = load(c + k * step <= last ? c + k * step : c);
+#pragma unroll
+        for (int k = 0; k < B; ++k)
+            if (c + k * step <= last) add(v[k]);
+    }
+}
+
 // ldexp(a, k), by one product with an exact power of two wherever that is a
 // normal number
 __device__ __forceinline__ double mul_pow2(double a, int k)

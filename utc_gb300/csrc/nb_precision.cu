@@ -45,6 +45,10 @@ __global__ void comp_join_kernel(const double4 *__restrict__ pos64, const float4
     }
 }
 
+struct HiLo {
+    float4 h, l;
+};
+
 // Compensated sum of a target's partial slots (hi and lo blocks).
 __device__ __forceinline__ void comp_slot_sum(const float4 *__restrict__ partial, long long lo_off,
                                               int tb, int li, int tbsize, long long total,
@@ -55,22 +59,29 @@ __device__ __forceinline__ void comp_slot_sum(const float4 *__restrict__ partial
     const int c1 = sk_owner(first + ngroups - 1, total, grid);
     S = make_float4(0.f, 0.f, 0.f, 0.f);
     C = S;
-    for (int c = c0; c <= c1; ++c) {
-        const size_t k = (size_t)(c + tb) * tbsize + li;
-        const float4 h = partial[k];
-        const float4 l = partial[lo_off + k];
-        float e;
-        two_sum(S.x, h.x, S.x, e); C.x = __fadd_rn(C.x, __fadd_rn(e, l.x));
-        two_sum(S.y, h.y, S.y, e); C.y = __fadd_rn(C.y, __fadd_rn(e, l.y));
-        two_sum(S.z, h.z, S.z, e); C.z = __fadd_rn(C.z, __fadd_rn(e, l.z));
-        two_sum(S.w, h.w, S.w, e); C.w = __fadd_rn(C.w, __fadd_rn(e, l.w));
-    }
+    walk<8>(
+        c0, c1, 1,
+        [&](int c) {
+            const size_t k = (size_t)(c + tb) * tbsize + li;
+            return HiLo{partial[k], partial[lo_off + k]};
+        },
+        [&](const HiLo &p) {
+            const float4 h = p.h, l = p.l;
+            float e;
+            two_sum(S.x, h.x, S.x, e); C.x = __fadd_rn(C.x, __fadd_rn(e, l.x));
+            two_sum(S.y, h.y, S.y, e); C.y = __fadd_rn(C.y, __fadd_rn(e, l.y));
+            two_sum(S.z, h.z, S.z, e); C.z = __fadd_rn(C.z, __fadd_rn(e, l.z));
+            two_sum(S.w, h.w, S.w, e); C.w = __fadd_rn(C.w, __fadd_rn(e, l.w));
+        });
 }
 
 // Bare accelerations of every target, and in w the potential sum over
 // j != i: the force pass sums j == i too (its term is m_i * rsqrt(eps2),
 // computed here exactly as the pass computed it) and it is taken out here.
 // Plain slots: float4 out; compensated slots: double4 out = hi + lo.
+// A chain of loads bounds it for small systems (50 slots a body): eight are
+// fetched at a time, added in the same order (compensated, N = 5432: 18.9 us
+// with a plain loop, 8.2 now).
 __global__ void sk_reduce_kernel(const float4 *__restrict__ partial, int n, int tbsize,
                                  long long total, int ngroups, int grid, long long lo_off,
                                  int comp, const float4 *__restrict__ pos32, float eps2,
@@ -93,13 +104,13 @@ __global__ void sk_reduce_kernel(const float4 *__restrict__ partial, int n, int 
     const int c0 = sk_owner(first, total, grid);
     const int c1 = sk_owner(first + ngroups - 1, total, grid);
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int c = c0; c <= c1; ++c) {
-        const float4 q = partial[(size_t)(c + tb) * tbsize + li];
-        a.x = __fadd_rn(a.x, q.x);
-        a.y = __fadd_rn(a.y, q.y);
-        a.z = __fadd_rn(a.z, q.z);
-        a.w = __fadd_rn(a.w, q.w);
-    }
+    walk<8>(c0, c1, 1, [&](int c) { return partial[(size_t)(c + tb) * tbsize + li]; },
+            [&](const float4 &q) {
+                a.x = __fadd_rn(a.x, q.x);
+                a.y = __fadd_rn(a.y, q.y);
+                a.z = __fadd_rn(a.z, q.z);
+                a.w = __fadd_rn(a.w, q.w);
+            });
     a.w = __fsub_rn(a.w, self);
     out32[i] = a;
 }
@@ -157,44 +168,71 @@ __global__ void comp_integrate_kernel(const float4 *__restrict__ partial, int n,
 // Compensated symmetric partials: the target-side slots (CTA order) and the
 // source-side rows 0..I-1 (row order), hi and lo halves, summed with
 // two-sums; then the compensated kick / drift, or (acc_out != nullptr) the
-// bare acceleration hi + lo in FP64.
-__global__ void sym_comp_integrate_kernel(const float4 *__restrict__ tpart, const float4 *__restrict__ spart,
-                                          long long tlo, long long slo, int n, int rb, int nc, int nrb,
-                                          long long total, int grid, double4 *__restrict__ pos64,
-                                          float4 *__restrict__ pos32, float4 *__restrict__ vhi,
-                                          float4 *__restrict__ vlo, float damping, float dt,
-                                          double dt64, int kick, float G, double4 *__restrict__ acc_out,
-                                          const float4 *__restrict__ accsum)
+// bare acceleration hi + lo in FP64.  A block takes 32 bodies x 8 slices: slice q
+// sums slots c0 + q, c0 + q + 8, ... and rows q, q + 8, ..., the slices are
+// merged in order (deterministic; every merge is a two-sum too).  One thread
+// per body was a chain of loads: 13.5 us at N = 1149 and 32 at N = 10958, beside
+// 8 and 45 us of force; now 5.0 and 7.3.
+constexpr int kCompSlices = 8;
+
+__global__ void __launch_bounds__(32 * kCompSlices)
+    sym_comp_integrate_kernel(const float4 *__restrict__ tpart, const float4 *__restrict__ spart,
+                              long long tlo, long long slo, int n, int rb, int nc, int nrb,
+                              long long total, int grid, double4 *__restrict__ pos64,
+                              float4 *__restrict__ pos32, float4 *__restrict__ vhi,
+                              float4 *__restrict__ vlo, float damping, float dt,
+                              double dt64, int kick, float G, double4 *__restrict__ acc_out,
+                              const float4 *__restrict__ accsum)
 {
+    __shared__ float red[6][kCompSlices][32];
+    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
     // bodies from the last one down: the longest row walks start first
-    const int i = n - 1 - (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (i < 0) return;
+    const int i = n - 1 - (int)(blockIdx.x * 32 + lane);
     float4 S = make_float4(0.f, 0.f, 0.f, 0.f), C = S;
-    if (accsum) {  // banded plan: the compensated fold's (S, C)
-        S = accsum[i];
-        C = accsum[(size_t)n + i];
-    } else {
+    auto add = [&](const HiLo &p) {
+        float e;
+        two_sum(S.x, p.h.x, S.x, e); C.x = __fadd_rn(C.x, __fadd_rn(e, p.l.x));
+        two_sum(S.y, p.h.y, S.y, e); C.y = __fadd_rn(C.y, __fadd_rn(e, p.l.y));
+        two_sum(S.z, p.h.z, S.z, e); C.z = __fadd_rn(C.z, __fadd_rn(e, p.l.z));
+    };
+    if (i >= 0 && accsum) {  // banded plan: the compensated fold's (S, C)
+        if (q == 0) {
+            S = accsum[i];
+            C = accsum[(size_t)n + i];
+        }
+    } else if (i >= 0) {
         const int rc = rb / 32;
         const int I = i / rb;
         const int c0 = sk_owner(sym_prefix(I, nc, rc), total, grid);
         const int c1 = sk_owner(sym_prefix(I + 1, nc, rc) - 1, total, grid);
         const int li = i - I * rb;
-        float e;
-        auto add = [&](const float4 h, const float4 l) {
-            two_sum(S.x, h.x, S.x, e); C.x = __fadd_rn(C.x, __fadd_rn(e, l.x));
-            two_sum(S.y, h.y, S.y, e); C.y = __fadd_rn(C.y, __fadd_rn(e, l.y));
-            two_sum(S.z, h.z, S.z, e); C.z = __fadd_rn(C.z, __fadd_rn(e, l.z));
-        };
-        for (int c = c0; c <= c1; ++c) {
-            const size_t k = (size_t)(c + I) * rb + li;
-            add(tpart[k], tpart[tlo + k]);
-        }
-        long long off = (long long)i - rb;  // row r at soff(r) + i - (r + 1) rb
-        for (int r = 0; r < I; ++r) {
-            add(spart[off], spart[slo + off]);
-            off += (long long)n - (long long)(r + 2) * rb;
-        }
+        walk<4>(
+            c0 + q, c1, kCompSlices,
+            [&](int c) {
+                const size_t k = (size_t)(c + I) * rb + li;
+                return HiLo{tpart[k], tpart[tlo + k]};
+            },
+            add);
+        walk<4>(
+            q, I - 1, kCompSlices,
+            [&](int r) {
+                const long long k = sym_soff(r, n, rb) + (i - (long long)(r + 1) * rb);
+                return HiLo{spart[k], spart[slo + k]};
+            },
+            add);
     }
+    red[0][q][lane] = S.x;
+    red[1][q][lane] = S.y;
+    red[2][q][lane] = S.z;
+    red[3][q][lane] = C.x;
+    red[4][q][lane] = C.y;
+    red[5][q][lane] = C.z;
+    __syncthreads();
+    if (q != 0 || i < 0) return;
+#pragma unroll
+    for (int k = 1; k < kCompSlices; ++k)
+        add(HiLo{make_float4(red[0][k][lane], red[1][k][lane], red[2][k][lane], 0.f),
+                 make_float4(red[3][k][lane], red[4][k][lane], red[5][k][lane], 0.f)});
     if (acc_out) {
         acc_out[i] = make_double4((double)S.x + (double)C.x, (double)S.y + (double)C.y,
                                   (double)S.z + (double)C.z, 0.0);
@@ -305,7 +343,7 @@ int fast_reduce(const SkPlan &p, const float4 *partial, int comp, const float4 *
     if (p.n == 0) return NB_OK;
     const long long lo_off = (long long)p.slots * p.tbsize;
     const SkLayout l = sk_layout(p);
-    sk_reduce_kernel<<<(p.n + 255) / 256, 256, 0, s>>>(partial, p.n, l.tbsize, l.total, l.ngroups,
+    sk_reduce_kernel<<<(p.n + 63) / 64, 64, 0, s>>>(partial, p.n, l.tbsize, l.total, l.ngroups,
                                                       l.grid, lo_off, comp, pos32, eps2, out32,
                                                       out64);
     NB_LAUNCH_CHECK("sk_reduce_kernel launch");
@@ -318,7 +356,7 @@ int comp_integrate(const SkPlan &p, const float4 *partial, double4 *pos64, float
 {
     if (p.n == 0) return NB_OK;
     const long long lo_off = (long long)p.slots * p.tbsize;
-    comp_integrate_kernel<<<(p.n + 255) / 256, 256, 0, s>>>(partial, p.n, p.tbsize, p.total,
+    comp_integrate_kernel<<<(p.n + 63) / 64, 64, 0, s>>>(partial, p.n, p.tbsize, p.total,
                                                            p.ngroups, p.grid, lo_off, pos64, pos32,
                                                            vhi, vlo, damping, dt, dt64, kick, G);
     NB_LAUNCH_CHECK("comp_integrate_kernel launch");
@@ -332,7 +370,7 @@ int sym_comp_integrate(const SymPlan &p, const float4 *tpart, const float4 *spar
     if (p.n == 0) return NB_OK;
     if (!p.comp) return set_error(NB_ERR_INVALID, "sym_comp_integrate needs a compensated plan");
     if (p.nbands > 1 && !accsum) return set_error(NB_ERR_INVALID, "sym_comp_integrate: a banded plan needs its sums");
-    sym_comp_integrate_kernel<<<(p.n + 255) / 256, 256, 0, s>>>(
+    sym_comp_integrate_kernel<<<(p.n + 31) / 32, 32 * kCompSlices, 0, s>>>(
         tpart, spart, (long long)p.slots * p.rb, p.spart_size, p.n, p.rb, p.nc, p.nrb, p.total,
         p.grid, pos64, pos32, vhi, vlo, damping, dt, dt64, kick, G, acc_out, p.nbands > 1 ? accsum : nullptr);
     NB_LAUNCH_CHECK("sym_comp_integrate_kernel launch");

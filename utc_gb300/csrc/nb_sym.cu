@@ -302,21 +302,14 @@ __global__ void __launch_bounds__(kSymIntegBlock) sym_integrate_kernel(
         const int c0 = sk_owner(sym_prefix(I, nc, rc), total, grid);
         const int c1 = sk_owner(sym_prefix(I + 1, nc, rc) - 1, total, grid);
         const int li = i - I * rb;
-        for (int c = c0 + q; c <= c1; c += 4) {
-            const float4 v4 = tpart[(size_t)(c + I) * rb + li];
+        auto add = [&](const float4 &v4) {
             ax = __fadd_rn(ax, v4.x);
             ay = __fadd_rn(ay, v4.y);
             az = __fadd_rn(az, v4.z);
-        }
-        if (!fxacc) {
-#pragma unroll 4
-            for (int r = q; r < I; r += 4) {
-                const float4 v4 = spart[sym_soff(r, n, rb) + (i - (long long)(r + 1) * rb)];
-                ax = __fadd_rn(ax, v4.x);
-                ay = __fadd_rn(ay, v4.y);
-                az = __fadd_rn(az, v4.z);
-            }
-        }
+        };
+        walk<4>(c0 + q, c1, 4, [&](int c) { return tpart[(size_t)(c + I) * rb + li]; }, add);
+        if (!fxacc)
+            walk<4>(q, I - 1, 4, [&](int r) { return spart[sym_soff(r, n, rb) + (i - (long long)(r + 1) * rb)]; }, add);
     }
     ax = __fadd_rn(ax, __shfl_xor_sync(0xffffffffu, ax, 1));
     ay = __fadd_rn(ay, __shfl_xor_sync(0xffffffffu, ay, 1));

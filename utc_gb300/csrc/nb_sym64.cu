@@ -17,7 +17,8 @@
 // Results agree with the FP64 oracle to rounding (the tests hold them to
 // 1e-13 relative); they are not bit-identical to it (NB_ALGO_EXACT is).
 // Range: d2 must be a normal FP64 number (eps2 > 0 keeps it there).
-#include "nb_internal.cuh"
+#include "nb_ff.cuh"
+#include "nb_integ.cuh"
 
 namespace nb {
 
@@ -136,23 +137,13 @@ __global__ void __launch_bounds__(32 * W, MINB) sym64_force_kernel(const double4
     }
 }
 
-// Per body: target-side slots + source-side rows 0..I-1, then the reference's
-// kick / damping / drift in its order with unfused IEEE operations
-// (bodysystem.cc:135-182), or the bare acceleration (with the potential sum
-// in w when the force pass recorded it: the float-float energy pass).
-//
-// Reads all partials once (N^2 / (2 rb) double4), so memory and the narrow
-// FP64 pipe's additions bound it; for small systems the chain of FP64
-// operations after the sums, which is why each component has a warp of its
-// own and fetches its old state first (N = 1000: 9.2 us with one warp doing
-// all of it and 64-bit divisions for the slots, now 6.5).  A block takes 32 bodies x 8 slices: slice
-// q sums slots c0 + q, c0 + q + 8, ... and rows q, q + 8, ... in order, and the
-// slices are added in slice order (fixed order: deterministic); the w sums
-// only where they are asked for.  With one thread per body the walk over up to
-// 255 rows was a chain of loads (N = 16384, rb = 64: 84 us a step).
-constexpr int kSym64Slices = 8;
-
-__global__ void __launch_bounds__(32 * kSym64Slices)
+// Per body: target-side slots + source-side rows 0..I-1, then kick / damping /
+// drift, or the bare acceleration (with the potential sum in w when the force
+// pass recorded it: the float-float energy pass).  A block takes 32 bodies x 8
+// slices (integrate64): slice q sums slots c0 + q, c0 + q + 8, ... and rows q,
+// q + 8, ... in order (deterministic).  With one thread per body the walk over
+// up to 255 rows was a chain of loads (N = 16384, rb = 64: 84 us a step).
+__global__ void __launch_bounds__(32 * kIntegSlices)
     sym64_integrate_kernel(const double4 *__restrict__ pos_old, double4 *__restrict__ pos_new,
                            double4 *__restrict__ vel, const double4 *__restrict__ tpart,
                            const double4 *__restrict__ spart, int n, int rb, int nc, int nrb, long long total,
@@ -160,81 +151,31 @@ __global__ void __launch_bounds__(32 * kSym64Slices)
                            double4 *__restrict__ acc_out, const unsigned long long *__restrict__ ffrange,
                            const double4 *__restrict__ accsum)
 {
-    __shared__ double red[4][kSym64Slices][32];
-    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
     // bodies from the last one down: the longest row walks start first
-    const int i = n - 1 - (int)(blockIdx.x * 32 + lane);
-    const bool want_w = acc_out != nullptr;
-    // what the warp's component q needs after the sums, fetched ahead of them
-    const size_t e = 4 * (size_t)(i < 0 ? 0 : i) + q;
-    unsigned long long scale[2] = {0, 0};
-    double xo = 0.0, m = 0.0, v = 0.0;
-    if (q < 4 && i >= 0) {
-        if (ffrange) {
-            scale[0] = ffrange[0];
-            scale[1] = ffrange[1];
-        }
-        if (!acc_out) {
-            xo = reinterpret_cast<const double *>(pos_old)[e];
-            m = pos_old[i].w;
-            if (q < 3) v = reinterpret_cast<const double *>(vel)[e];
-        }
-    }
-    double ax = 0.0, ay = 0.0, az = 0.0, aw = 0.0;
-    auto add = [&](const double4 &v) {
-        ax = __dadd_rn(ax, v.x);
-        ay = __dadd_rn(ay, v.y);
-        az = __dadd_rn(az, v.z);
-        if (want_w) aw = __dadd_rn(aw, v.w);
-    };
-    if (i >= 0 && accsum) {  // banded plan: the fold kernel's sums
-        if (q == 0) add(accsum[i]);
-    } else if (i >= 0) {
-        const int rc = rb / 32;
-        const int I = i / rb;
-        const int c0 = sk_owner(sym_prefix(I, nc, rc), total, grid);
-        const int c1 = sk_owner(sym_prefix(I + 1, nc, rc) - 1, total, grid);
-        const int li = i - I * rb;
-        for (int c = c0 + q; c <= c1; c += kSym64Slices) add(tpart[(size_t)(c + I) * rb + li]);
+    const int i = n - 1 - (int)(blockIdx.x * 32 + (threadIdx.x & 31));
+    // float-float path: the sums are in units scaled by 2^kx (positions) and
+    // 2^km (masses), kx = -e(max |x|), km = -e(max m) with 2^(e-1) <= v < 2^e;
+    // a = a_scaled * 2^(2 kx - km) and phi = phi_scaled * 2^(kx - km), exact
+    const int ex = ffrange ? ff_exponent(ffrange[0]) : 0, em = ffrange ? ff_exponent(ffrange[1]) : 0;
+    integrate64<kIntegSlices>(
+        i,
+        [&](int q, auto add) {
+            if (accsum) {  // banded plan: the fold kernel's sums
+                if (q == 0) add(accsum[i]);
+                return;
+            }
+            const int rc = rb / 32;
+            const int I = i / rb;
+            const int c0 = sk_owner(sym_prefix(I, nc, rc), total, grid);
+            const int c1 = sk_owner(sym_prefix(I + 1, nc, rc) - 1, total, grid);
+            const int li = i - I * rb;
+            for (int c = c0 + q; c <= c1; c += kIntegSlices) add(tpart[(size_t)(c + I) * rb + li]);
 #pragma unroll 4
-        for (int r = q; r < I; r += kSym64Slices) add(spart[sym_soff(r, n, rb) + (i - (long long)(r + 1) * rb)]);
-    }
-    red[0][q][lane] = ax;
-    red[1][q][lane] = ay;
-    red[2][q][lane] = az;
-    red[3][q][lane] = aw;
-    __syncthreads();
-    // warp q goes on with component q of the 32 bodies: x, y, z, and w (the
-    // potential, or what the step carries along)
-    if (q > 3 || i < 0) return;
-    double a = red[q][0][lane];
-#pragma unroll
-    for (int k = 1; k < kSym64Slices; ++k) a = __dadd_rn(a, red[q][k][lane]);
-    if (ffrange) {
-        // float-float path: its sums are in units scaled by 2^kx (positions)
-        // and 2^km (masses), kx = -e(max |x|), km = -e(max m) with
-        // 2^(e-1) <= v < 2^e; a = a_scaled * 2^(2 kx - km) and
-        // phi = phi_scaled * 2^(kx - km), exact
-        auto ex = [](unsigned long long b) {
-            const int f = (int)((b >> 52) & 0x7ff);
-            return (f == 0 || f == 0x7ff) ? 0 : f - 1022;
-        };
-        const int em = ex(scale[1]), ex0 = ex(scale[0]);
-        const int k = q < 3 ? em - 2 * ex0 : em - ex0;
-        a = mul_pow2(a, k);
-    }
-    if (acc_out) {
-        reinterpret_cast<double *>(acc_out)[e] = a;
-        return;
-    }
-    if (q < 3) {
-        const double k = kick == NB_KICK_REFERENCE ? m : G;
-        v = __dadd_rn(v, __dmul_rn(__dmul_rn(a, k), dt));
-        v = __dmul_rn(v, damping);
-        reinterpret_cast<double *>(vel)[e] = v;
-        xo = __dadd_rn(xo, __dmul_rn(v, dt));
-    }
-    reinterpret_cast<double *>(pos_new)[e] = xo;  // component 3: the mass
+            for (int r = q; r < I; r += kIntegSlices)
+                add(spart[sym_soff(r, n, rb) + (i - (long long)(r + 1) * rb)]);
+        },
+        [&](int q, double a) { return ffrange ? mul_pow2(a, q < 3 ? em - 2 * ex : em - ex) : a; }, pos_old, pos_new, vel,
+        damping, dt, kick, G, acc_out);
 }
 
 typedef void (*sym64_kernel_t)(const double4 *, int, double, double4 *, double4 *, long long, int, int);
@@ -311,7 +252,7 @@ int sym64_integrate(const SymPlan &p, const double4 *pos_old, double4 *pos_new, 
 {
     if (p.n == 0) return NB_OK;
     if (p.nbands > 1 && !accsum) return set_error(NB_ERR_INVALID, "sym64_integrate: a banded plan needs its per-body sums");
-    sym64_integrate_kernel<<<(p.n + 31) / 32, 32 * kSym64Slices, 0, s>>>(pos_old, pos_new, vel, tpart, spart, p.n, p.rb,
+    sym64_integrate_kernel<<<(p.n + 31) / 32, 32 * kIntegSlices, 0, s>>>(pos_old, pos_new, vel, tpart, spart, p.n, p.rb,
                                                              p.nc, p.nrb, p.total, p.grid, damping, dt, kick,
                                                              G, acc_out, ffrange, p.nbands > 1 ? accsum : nullptr);
     NB_LAUNCH_CHECK("sym64_integrate_kernel launch");
