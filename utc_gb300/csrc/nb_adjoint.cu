@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(32 * W, MINB) sym_vjp_kernel(const float4 *__r
                                                                float4 *__restrict__ spart,
                                                                long long total, int nc, int nrb)
 {
+    pdl_wait();
     constexpr int RB = W * 32 * BPT;
     constexpr int RC = RB / 32;
     const int c = blockIdx.x;
@@ -262,11 +263,12 @@ __global__ void adj_update_kernel(const float4 *__restrict__ partial, int n, int
 constexpr int kAdjUpdBlock = 256;
 
 __global__ void __launch_bounds__(kAdjUpdBlock) adj_update_sym_kernel(
-    const float4 *__restrict__ tpart, const float4 *__restrict__ spart, int n, int rb, int nc, int nrb,
-    long long total, int grid, const float4 *__restrict__ pos, const float4 *__restrict__ acc,
-    float4 *__restrict__ lx, float4 *__restrict__ lv, float *__restrict__ gm, float4 *__restrict__ gbuf,
+    const float4 *tpart, const float4 *spart, int n, int rb, int nc, int nrb,
+    long long total, int grid, const float4 *pos, const float4 *acc,
+    float4 *lx, float4 *lv, float *gm, float4 *gbuf,
     float damping, float dt, int kick, float G, int want_next_g)
 {
+    pdl_wait();
     // bodies from the last one down, as in sym_integrate_kernel: the blocks
     // with the longest row walks start first
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -424,9 +426,8 @@ int sym_vjp(const SymPlan &p, const float4 *pos, const float4 *gbuf, float eps2,
     if (p.total == 0) return NB_OK;
     sym_vjp_kernel_t k = sym_vjp_kernel_for(p.warps, p.bpt);
     if (!k) return set_error(NB_ERR_UNSUPPORTED, "symmetric adjoint kernel shape not compiled");
-    k<<<p.grid, 32 * p.warps, 0, s>>>(pos, gbuf, p.n, eps2, tpart, spart, p.total, p.nc, p.nrb);
-    NB_LAUNCH_CHECK("sym_vjp_kernel launch");
-    return NB_OK;
+    return pdl_launch("sym_vjp_kernel launch", k, p.grid, 32 * p.warps, s, pos, gbuf, p.n, eps2, tpart, spart, p.total,
+                      p.nc, p.nrb);
 }
 
 int adj_update_sym(const SymPlan &p, const float4 *tpart, const float4 *spart, const float4 *pos_prev,
@@ -435,11 +436,9 @@ int adj_update_sym(const SymPlan &p, const float4 *tpart, const float4 *spart, c
 {
     if (p.n == 0) return NB_OK;
     const long long threads = 4ll * p.n;  // a quad of threads per body
-    adj_update_sym_kernel<<<(unsigned)((threads + kAdjUpdBlock - 1) / kAdjUpdBlock), kAdjUpdBlock, 0, s>>>(
-        tpart, spart, p.n, p.rb, p.nc, p.nrb, p.total, p.grid, pos_prev, acc, lx, lv, gm, gbuf, damping, dt,
-        kick, G, want_next_g);
-    NB_LAUNCH_CHECK("adj_update_sym_kernel launch");
-    return NB_OK;
+    return pdl_launch("adj_update_sym_kernel launch", adj_update_sym_kernel,
+                      (unsigned)((threads + kAdjUpdBlock - 1) / kAdjUpdBlock), kAdjUpdBlock, s, tpart, spart, p.n, p.rb,
+                      p.nc, p.nrb, p.total, p.grid, pos_prev, acc, lx, lv, gm, gbuf, damping, dt, kick, G, want_next_g);
 }
 
 }  // namespace nb

@@ -252,6 +252,7 @@ __global__ void __launch_bounds__(32 * WPB, 8 / WPB) bks_force_kernel(const floa
                                                              float4 *__restrict__ spart, long long total,
                                                              int workers)
 {
+    pdl_wait();
     constexpr int RB = 32 * BPT;
     constexpr int RC = BPT;
     const int w = blockIdx.x * WPB + (threadIdx.x >> 5);
@@ -320,14 +321,15 @@ __device__ __forceinline__ float quad_sum(float v)
 // loop the walk over slots and rows was a chain of loads (18 systems of 591 to
 // 2703 bodies: 13.5 us beside 20 us of force).
 template <int Q>
-__global__ void __launch_bounds__(256) bks_integrate_kernel(const float4 *__restrict__ pos_old,
-                                                            float4 *__restrict__ pos_new, float4 *__restrict__ vel,
-                                                            const float4 *__restrict__ tpart,
-                                                            const float4 *__restrict__ spart, BatchSymDev bd,
+__global__ void __launch_bounds__(256) bks_integrate_kernel(const float4 *pos_old,
+                                                            float4 *pos_new, float4 *vel,
+                                                            const float4 *tpart,
+                                                            const float4 *spart, BatchSymDev bd,
                                                             int nbody, int rb, long long total, int workers,
                                                             float damping, float dt, int kick, float G,
-                                                            float4 *__restrict__ acc_out)
+                                                            float4 *acc_out)
 {
+    pdl_wait();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int q = (int)(t % Q);
     const bool live = t / Q < nbody;  // dead threads still take part in the shuffles
@@ -416,9 +418,10 @@ __device__ __noinline__ void bksff_row_segment(const float4 *__restrict__ H, con
 template <int WPB, int BPT>
 __global__ void __launch_bounds__(32 * WPB)
     bksff_force_kernel(const float4 *__restrict__ H, const float4 *__restrict__ Mi, const float4 *__restrict__ Lo,
-                       BatchSymDev bd, double eps2, const unsigned long long *__restrict__ range,
+                       BatchSymDev bd, double eps2, const unsigned long long *range,
                        double4 *__restrict__ tpart, double4 *__restrict__ spart, long long total, int workers)
 {
+    pdl_wait();
     constexpr int RB = 32 * BPT;
     constexpr int RC = BPT;
     const int wid = threadIdx.x >> 5;
@@ -459,12 +462,13 @@ __global__ void __launch_bounds__(32 * WPB)
 constexpr int kBatchSlices = 4;
 
 __global__ void __launch_bounds__(32 * kBatchSlices)
-    bksff_integrate_kernel(const double4 *__restrict__ pos_old, double4 *__restrict__ pos_new,
-                           double4 *__restrict__ vel, const double4 *__restrict__ tpart,
-                           const double4 *__restrict__ spart, BatchSymDev bd, int nbody, int rb, long long total,
+    bksff_integrate_kernel(const double4 *pos_old, double4 *pos_new,
+                           double4 *vel, const double4 *tpart,
+                           const double4 *spart, BatchSymDev bd, int nbody, int rb, long long total,
                            int workers, double damping, double dt, int kick, double G,
-                           const unsigned long long *__restrict__ range, double4 *__restrict__ acc_out)
+                           const unsigned long long *range, double4 *acc_out)
 {
+    pdl_wait();
     const int b = blockIdx.x * 32 + (threadIdx.x & 31);
     const int i = b < nbody ? b : -1;
     const int k2 = ff_exponent(range[1]) - 2 * ff_exponent(range[0]);
@@ -978,17 +982,13 @@ static int batch_force(nb_batch *b, const float4 *po, cudaStream_t s)
         int st = nb::ff_scale_split((const double4 *)po, b->nbody, b->sms, H, M, L, b->ff_range, s);
         if (st) return st;
         nb::bksff_kernel_t k = nb::bksff_kernel_for(p.wpb, p.bpt);
-        k<<<p.grid, 32 * p.wpb, 0, s>>>(H, M, L, batch_sym_dev(b), b->p.eps2, b->ff_range, (double4 *)b->partial,
-                                        (double4 *)b->spart, p.total, p.workers);
-        NB_LAUNCH_CHECK("bksff_force_kernel launch");
-        return NB_OK;
+        return nb::pdl_launch("bksff_force_kernel launch", k, p.grid, 32 * p.wpb, s, H, M, L, batch_sym_dev(b), b->p.eps2,
+                              b->ff_range, (double4 *)b->partial, (double4 *)b->spart, p.total, p.workers);
     }
     if (b->sym) {
         nb::bks_kernel_t k = nb::bks_kernel_for(p.wpb, p.bpt);
-        k<<<p.grid, 32 * p.wpb, 0, s>>>(po, batch_sym_dev(b), (float)b->p.eps2, b->partial, b->spart,
-                                        p.total, p.workers);
-        NB_LAUNCH_CHECK("bks_force_kernel launch");
-        return NB_OK;
+        return nb::pdl_launch("bks_force_kernel launch", k, p.grid, 32 * p.wpb, s, po, batch_sym_dev(b),
+                              (float)b->p.eps2, b->partial, b->spart, p.total, p.workers);
     }
     nb::bk_kernel_t k = nb::bk_kernel_for(p.wpb, p.bpt);
     k<<<p.grid, 32 * p.wpb, 0, s>>>(po, batch_dev(b), (float)b->p.eps2, b->partial, p.total, p.workers);
@@ -1006,21 +1006,19 @@ static int batch_integrate(nb_batch *b, const float4 *po, float4 *pn, float4 *ve
     if (!b->plan_ok)
         return set_error(NB_ERR_STATE, "batch has no valid launch plan (a plan change or autotune failed)");
     if (b->f64) {
-        nb::bksff_integrate_kernel<<<(b->nbody + 31) / 32, 32 * nb::kBatchSlices, 0, s>>>(
-            (const double4 *)po, (double4 *)pn, (double4 *)vel, (const double4 *)b->partial,
-            (const double4 *)b->spart, batch_sym_dev(b), b->nbody, 32 * p.bpt, p.total, p.workers, b->p.damping,
-            b->p.dt, b->p.kick, b->p.G, b->ff_range, (double4 *)acc_out);
-        NB_LAUNCH_CHECK("bksff_integrate_kernel launch");
-        return NB_OK;
+        return nb::pdl_launch("bksff_integrate_kernel launch", nb::bksff_integrate_kernel, (b->nbody + 31) / 32,
+                              32 * nb::kBatchSlices, s, (const double4 *)po, (double4 *)pn, (double4 *)vel,
+                              (const double4 *)b->partial, (const double4 *)b->spart, batch_sym_dev(b), b->nbody,
+                              32 * p.bpt, p.total, p.workers, b->p.damping, b->p.dt, b->p.kick, b->p.G, b->ff_range,
+                              (double4 *)acc_out);
     }
     if (b->sym) {
         const bool few = b->nbody <= nb::kFewBodies;
         auto kern = few ? nb::bks_integrate_kernel<4> : nb::bks_integrate_kernel<1>;
-        kern<<<(unsigned)(((few ? 4ll : 1ll) * b->nbody + 255) / 256), 256, 0, s>>>(
-            po, pn, vel, b->partial, b->spart, batch_sym_dev(b), b->nbody, 32 * p.bpt, p.total,
-            p.workers, (float)b->p.damping, (float)b->p.dt, b->p.kick, (float)b->p.G, acc_out);
-        NB_LAUNCH_CHECK("bks_integrate_kernel launch");
-        return NB_OK;
+        return nb::pdl_launch("bks_integrate_kernel launch", kern,
+                              (unsigned)(((few ? 4ll : 1ll) * b->nbody + 255) / 256), 256, s, po, pn, vel, b->partial,
+                              b->spart, batch_sym_dev(b), b->nbody, 32 * p.bpt, p.total, p.workers, (float)b->p.damping,
+                              (float)b->p.dt, b->p.kick, (float)b->p.G, acc_out);
     }
     nb::bk_integrate_kernel<<<(b->nbody + 255) / 256, 256, 0, s>>>(
         po, pn, vel, b->partial, batch_dev(b), b->nbody, 32 * p.bpt, p.total, p.workers,

@@ -176,14 +176,15 @@ __global__ void comp_integrate_kernel(const float4 *__restrict__ partial, int n,
 constexpr int kCompSlices = 8;
 
 __global__ void __launch_bounds__(32 * kCompSlices)
-    sym_comp_integrate_kernel(const float4 *__restrict__ tpart, const float4 *__restrict__ spart,
+    sym_comp_integrate_kernel(const float4 *tpart, const float4 *spart,
                               long long tlo, long long slo, int n, int rb, int nc, int nrb,
-                              long long total, int grid, double4 *__restrict__ pos64,
-                              float4 *__restrict__ pos32, float4 *__restrict__ vhi,
-                              float4 *__restrict__ vlo, float damping, float dt,
-                              double dt64, int kick, float G, double4 *__restrict__ acc_out,
-                              const float4 *__restrict__ accsum)
+                              long long total, int grid, double4 *pos64,
+                              float4 *pos32, float4 *vhi,
+                              float4 *vlo, float damping, float dt,
+                              double dt64, int kick, float G, double4 *acc_out,
+                              const float4 *accsum)
 {
+    pdl_wait();
     __shared__ float red[6][kCompSlices][32];
     const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
     // bodies from the last one down: the longest row walks start first
@@ -370,11 +371,9 @@ int sym_comp_integrate(const SymPlan &p, const float4 *tpart, const float4 *spar
     if (p.n == 0) return NB_OK;
     if (!p.comp) return set_error(NB_ERR_INVALID, "sym_comp_integrate needs a compensated plan");
     if (p.nbands > 1 && !accsum) return set_error(NB_ERR_INVALID, "sym_comp_integrate: a banded plan needs its sums");
-    sym_comp_integrate_kernel<<<(p.n + 31) / 32, 32 * kCompSlices, 0, s>>>(
-        tpart, spart, (long long)p.slots * p.rb, p.spart_size, p.n, p.rb, p.nc, p.nrb, p.total,
-        p.grid, pos64, pos32, vhi, vlo, damping, dt, dt64, kick, G, acc_out, p.nbands > 1 ? accsum : nullptr);
-    NB_LAUNCH_CHECK("sym_comp_integrate_kernel launch");
-    return NB_OK;
+    return pdl_launch("sym_comp_integrate_kernel launch", sym_comp_integrate_kernel, (p.n + 31) / 32, 32 * kCompSlices, s,
+                      tpart, spart, (long long)p.slots * p.rb, p.spart_size, p.n, p.rb, p.nc, p.nrb, p.total, p.grid,
+                      pos64, pos32, vhi, vlo, damping, dt, dt64, kick, G, acc_out, p.nbands > 1 ? accsum : nullptr);
 }
 
 int energy_blocks(int n) { return (n + kEnergyBlock - 1) / kEnergyBlock; }

@@ -243,6 +243,7 @@ __global__ void __launch_bounds__(32 * W, MINB) sym_force_kernel(const float4 *_
                                                            long long tlo, long long slo, long long it0,
                                                            int r0, long long soff0)
 {
+    pdl_wait();
     constexpr int RB = W * 32 * BPT;
     constexpr int RC = RB / 32;
     const int c = blockIdx.x;
@@ -280,11 +281,12 @@ constexpr int kSymIntegBlock = 256;
 // consume, zeroes the body's six accumulators for the next force launch.
 // accsum != nullptr (banded plans): the folded sums, taken as they are.
 __global__ void __launch_bounds__(kSymIntegBlock) sym_integrate_kernel(
-    const float4 *__restrict__ pos_old, float4 *__restrict__ pos_new, float4 *__restrict__ vel,
-    const float4 *__restrict__ tpart, const float4 *__restrict__ spart, int n, int rb, int nc, int nrb,
-    long long total, int grid, float damping, float dt, int kick, float G, float4 *__restrict__ acc_out,
-    unsigned long long *__restrict__ fxacc, int consume, const float4 *__restrict__ accsum)
+    const float4 *pos_old, float4 *pos_new, float4 *vel,
+    const float4 *tpart, const float4 *spart, int n, int rb, int nc, int nrb,
+    long long total, int grid, float damping, float dt, int kick, float G, float4 *acc_out,
+    unsigned long long *fxacc, int consume, const float4 *accsum)
 {
+    pdl_wait();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int i = n - 1 - (int)(t >> 2), q = (int)(t & 3);
     const bool live = i >= 0;  // dead threads still take part in the shuffles
@@ -307,7 +309,7 @@ __global__ void __launch_bounds__(kSymIntegBlock) sym_integrate_kernel(
             ay = __fadd_rn(ay, v4.y);
             az = __fadd_rn(az, v4.z);
         };
-        walk<4>(c0 + q, c1, 4, [&](int c) { return tpart[(size_t)(c + I) * rb + li]; }, add);
+        walk<8>(c0 + q, c1, 4, [&](int c) { return tpart[(size_t)(c + I) * rb + li]; }, add);
         if (!fxacc)
             walk<4>(q, I - 1, 4, [&](int r) { return spart[sym_soff(r, n, rb) + (i - (long long)(r + 1) * rb)]; }, add);
     }
@@ -680,9 +682,8 @@ int sym_force(const SymPlan &p, const float4 *pos, float eps2, float4 *tpart, fl
     // lo blocks (compensated plans) follow the hi blocks
     const long long tlo = (long long)p.slots * p.rb, slo = p.spart_size;
     if (p.nbands <= 1) {
-        k<<<p.grid, 32 * p.warps, 0, s>>>(pos, p.n, eps2, tpart, spart, p.total, p.nc, p.nrb, tlo, slo, 0, 0, 0);
-        NB_LAUNCH_CHECK("sym_force_kernel launch");
-        return NB_OK;
+        return pdl_launch("sym_force_kernel launch", k, p.grid, 32 * p.warps, s, pos, p.n, eps2, tpart, spart, p.total,
+                          p.nc, p.nrb, tlo, slo, 0, 0, 0);
     }
     if (!accsum) return set_error(NB_ERR_INVALID, "sym_force: a banded plan needs its per-body sums");
     const int rc = p.rb / 32;
@@ -715,11 +716,10 @@ int sym_integrate(const SymPlan &p, const float4 *pos_old, float4 *pos_new, floa
     const long long threads = 4ll * p.n;  // a quad of threads per body
     unsigned long long *fxacc =
         p.fixed ? reinterpret_cast<unsigned long long *>(const_cast<float4 *>(spart)) : nullptr;
-    sym_integrate_kernel<<<(unsigned)((threads + kSymIntegBlock - 1) / kSymIntegBlock), kSymIntegBlock, 0, s>>>(
-        pos_old, pos_new, vel, tpart, spart, p.n, p.rb, p.nc, p.nrb, p.total, p.grid, damping, dt, kick,
-        G, acc_out, fxacc, consume, p.nbands > 1 ? accsum : nullptr);
-    NB_LAUNCH_CHECK("sym_integrate_kernel launch");
-    return NB_OK;
+    return pdl_launch("sym_integrate_kernel launch", sym_integrate_kernel,
+                      (unsigned)((threads + kSymIntegBlock - 1) / kSymIntegBlock), kSymIntegBlock, s, pos_old, pos_new,
+                      vel, tpart, spart, p.n, p.rb, p.nc, p.nrb, p.total, p.grid, damping, dt, kick, G, acc_out, fxacc,
+                      consume, p.nbands > 1 ? accsum : nullptr);
 }
 
 }  // namespace nb

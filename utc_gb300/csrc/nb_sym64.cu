@@ -144,13 +144,14 @@ __global__ void __launch_bounds__(32 * W, MINB) sym64_force_kernel(const double4
 // q + 8, ... in order (deterministic).  With one thread per body the walk over
 // up to 255 rows was a chain of loads (N = 16384, rb = 64: 84 us a step).
 __global__ void __launch_bounds__(32 * kIntegSlices)
-    sym64_integrate_kernel(const double4 *__restrict__ pos_old, double4 *__restrict__ pos_new,
-                           double4 *__restrict__ vel, const double4 *__restrict__ tpart,
-                           const double4 *__restrict__ spart, int n, int rb, int nc, int nrb, long long total,
+    sym64_integrate_kernel(const double4 *pos_old, double4 *pos_new,
+                           double4 *vel, const double4 *tpart,
+                           const double4 *spart, int n, int rb, int nc, int nrb, long long total,
                            int grid, double damping, double dt, int kick, double G,
-                           double4 *__restrict__ acc_out, const unsigned long long *__restrict__ ffrange,
-                           const double4 *__restrict__ accsum)
+                           double4 *acc_out, const unsigned long long *ffrange,
+                           const double4 *accsum)
 {
+    pdl_wait();
     // bodies from the last one down: the longest row walks start first
     const int i = n - 1 - (int)(blockIdx.x * 32 + (threadIdx.x & 31));
     // float-float path: the sums are in units scaled by 2^kx (positions) and
@@ -252,11 +253,9 @@ int sym64_integrate(const SymPlan &p, const double4 *pos_old, double4 *pos_new, 
 {
     if (p.n == 0) return NB_OK;
     if (p.nbands > 1 && !accsum) return set_error(NB_ERR_INVALID, "sym64_integrate: a banded plan needs its per-body sums");
-    sym64_integrate_kernel<<<(p.n + 31) / 32, 32 * kIntegSlices, 0, s>>>(pos_old, pos_new, vel, tpart, spart, p.n, p.rb,
-                                                             p.nc, p.nrb, p.total, p.grid, damping, dt, kick,
-                                                             G, acc_out, ffrange, p.nbands > 1 ? accsum : nullptr);
-    NB_LAUNCH_CHECK("sym64_integrate_kernel launch");
-    return NB_OK;
+    return pdl_launch("sym64_integrate_kernel launch", sym64_integrate_kernel, (p.n + 31) / 32, 32 * kIntegSlices, s,
+                      pos_old, pos_new, vel, tpart, spart, p.n, p.rb, p.nc, p.nrb, p.total, p.grid, damping, dt, kick, G,
+                      acc_out, ffrange, p.nbands > 1 ? accsum : nullptr);
 }
 
 }  // namespace nb

@@ -115,11 +115,12 @@ __device__ __forceinline__ void ff_split_body(const double4 &q, int ex, int em, 
 // split took 10.8 us at N = 1000 to 8192; now 4.1 to 4.7.
 constexpr int kFFSplitBlock = 64;
 
-__global__ void __launch_bounds__(kFFSplitBlock) ff_split_kernel(const double4 *__restrict__ pos, int n,
-                                                                 const unsigned long long *__restrict__ range,
-                                                                 float4 *__restrict__ H, float4 *__restrict__ M,
-                                                                 float4 *__restrict__ L)
+__global__ void __launch_bounds__(kFFSplitBlock) ff_split_kernel(const double4 *pos, int n,
+                                                                 const unsigned long long *range,
+                                                                 float4 *H, float4 *M,
+                                                                 float4 *L)
 {
+    pdl_wait();
     const int i = blockIdx.x * kFFSplitBlock + threadIdx.x;
     if (i >= n) return;
     ff_split_body(pos[i], ff_exponent(range[0]), ff_exponent(range[1]), H + i, M + i, L + i);
@@ -272,10 +273,11 @@ __device__ __noinline__ void symff_row_segment(const float4 *__restrict__ H, con
 template <int W, int BPT, int MINB, bool PHI, bool BAND = false>
 __global__ void __launch_bounds__(32 * W, MINB)
     symff_force_kernel(const float4 *__restrict__ H, const float4 *__restrict__ Mi, const float4 *__restrict__ Lo,
-                       int n, double eps2, const unsigned long long *__restrict__ range,
+                       int n, double eps2, const unsigned long long *range,
                        double4 *__restrict__ tpart, double4 *__restrict__ spart, long long total, int nc, int nrb,
                        long long it0, int r0, long long soff0)
 {
+    pdl_wait();
     constexpr int RB = W * 32 * BPT;
     constexpr int RC = RB / 32;
     const int c = blockIdx.x;
@@ -433,9 +435,8 @@ int ff_scale_split(const double4 *pos, int n, int sms, float4 *H, float4 *M, flo
     const long long blocks = want < cap ? want : cap;
     ff_range_kernel<<<(unsigned)blocks, 256, 0, s>>>(pos, n, range);
     NB_LAUNCH_CHECK("ff_range_kernel launch");
-    ff_split_kernel<<<(unsigned)((n + kFFSplitBlock - 1) / kFFSplitBlock), kFFSplitBlock, 0, s>>>(pos, n, range, H, M, L);
-    NB_LAUNCH_CHECK("ff_split_kernel launch");
-    return NB_OK;
+    return pdl_launch("ff_split_kernel launch", ff_split_kernel, (unsigned)((n + kFFSplitBlock - 1) / kFFSplitBlock),
+                      kFFSplitBlock, s, pos, n, range, H, M, L);
 }
 
 // ---------------------------------------------------------------------------
@@ -612,9 +613,8 @@ int symff_force(const SymPlan &p, const double4 *pos, double eps2, float4 *split
     int st = ff_scale_split(pos, p.n, p.sms, H, M, L, range, s);
     if (st) return st;
     if (p.nbands <= 1) {
-        k<<<p.grid, 32 * p.warps, 0, s>>>(H, M, L, p.n, eps2, range, tpart, spart, p.total, p.nc, p.nrb, 0, 0, 0);
-        NB_LAUNCH_CHECK("symff_force_kernel launch");
-        return NB_OK;
+        return pdl_launch("symff_force_kernel launch", k, p.grid, 32 * p.warps, s, H, M, L, p.n, eps2, range, tpart,
+                          spart, p.total, p.nc, p.nrb, 0, 0, 0);
     }
     const int rc = p.rb / 32;
     for (int b = 0; b < p.nbands; ++b) {
