@@ -301,6 +301,81 @@ __global__ void __launch_bounds__(kAdjUpdBlock) adj_update_sym_kernel(
     adj_body_update(i, ox, oy, oz, odm, pos, acc, lx, lv, gm, gbuf, damping, dt, kick, G, want_next_g);
 }
 
+// A whole reverse step of a small system in one launch, as nb_small.cu does
+// forward steps: a CTA owns TB bodies, its threads split the other side of every
+// pair, the sums are reduced in the CTA and its first threads update their
+// bodies.  The next step's g goes to gnext: other CTAs still read gbuf.
+//
+// Reverse step, GB300, us, against the symmetric kernels' two launches: N = 700
+// 4.8 (14.8), 1376 6.5 (16.1), 3000 12.8 (17.6), 5000 29.4 (39.8), 6000 37.3 (39.1),
+// 7000 50.2 (53.1), 9000 77.9 (67.4): the line is at 7000.  Bounds: latency (first
+// loads, reduction) below N about 2000, then register-file reads, 26 operations
+// for each order of a pair where the symmetric kernel takes 42 for both.  4
+// bodies a CTA; 2, 6 and 8 are within 10 % and mostly behind (N = 3000: 13.9,
+// 14.4, 14.1).
+constexpr int kVjpSmallThreads = 128;
+constexpr int kVjpSmallTargets = 4;
+constexpr int kVjpSmallBodies = 7000;
+
+template <int TB>
+__global__ void __launch_bounds__(kVjpSmallThreads, 1)
+    small_vjp_kernel(const float4 *pos, const float4 *gbuf, int n, float eps2, const float4 *acc, float4 *lx, float4 *lv,
+                     float *gm, float4 *gnext, float damping, float dt, int kick, float G, int want_next_g)
+{
+    constexpr int NP = TB / 2, TP = pow2_up(TB), NW = kVjpSmallThreads / 32;
+    __shared__ float red[NW][4 * TP];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int t0 = blockIdx.x * TB;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 pad = make_float4(kPadCoord, kPadCoord, kPadCoord, 0.f);
+    const f2 EPS2 = f2_pack(eps2, eps2);
+    pdl_wait();
+    VjpTargets<NP> T;
+    T.load([&](int t) { return t0 + t < n ? pos[t0 + t] : zero; }, [&](int t) { return t0 + t < n ? gbuf[t0 + t] : zero; });
+    VjpSums none;
+    float4 nx = tid < n ? pos[tid] : pad, ng = tid < n ? gbuf[tid] : zero;
+    for (int j = tid; j - tid < n; j += kVjpSmallThreads) {
+        VjpSource b;
+        b.load(nx, ng);
+        const int jn = j + kVjpSmallThreads;
+        nx = jn < n ? pos[jn] : pad;
+        ng = jn < n ? gbuf[jn] : zero;
+#pragma unroll
+        for (int p = 0; p < NP; ++p) T.template pair<false>(p, b, EPS2, none);
+    }
+    float s[4 * TP];
+#pragma unroll
+    for (int k = 4 * TB; k < 4 * TP; ++k) s[k] = 0.f;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        float4 a, b;
+        T.out(p, a, b);
+        s[8 * p] = a.x;
+        s[8 * p + 1] = a.y;
+        s[8 * p + 2] = a.z;
+        s[8 * p + 3] = a.w;
+        s[8 * p + 4] = b.x;
+        s[8 * p + 5] = b.y;
+        s[8 * p + 6] = b.z;
+        s[8 * p + 7] = b.w;
+    }
+    const int t = warp_sum<TP, 4>(s, lane);
+    if ((lane & (32 / TP - 1)) == 0) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) red[wid][4 * t + k] = s[k];
+    }
+    __syncthreads();
+    const int i = t0 + tid;
+    if (tid >= TB || i >= n) return;
+    float o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) o[k] += red[w][4 * tid + k];
+    }
+    adj_body_update(i, o[0], o[1], o[2], o[3], pos, acc, lx, lv, gm, gnext, damping, dt, kick, G, want_next_g);
+}
+
 typedef void (*vjp_kernel_t)(const float4 *, const float4 *, int, float, float4 *, long long, int);
 
 static vjp_kernel_t vjp_kernel_for(int block, int bpt)
@@ -416,8 +491,18 @@ int sym_vjp_plan(int n, int warps, int bpt, int device, SymPlan *pl)
     p.grid = p.total > 0 ? (int)grid : 0;
     p.slots = p.total > 0 ? p.grid + p.nrb - 1 : 0;
     p.spart_size = sym_spart_entries(n, p.rb);
+    p.small = warps == 1 && bpt == 10 && n <= kVjpSmallBodies;
     *pl = p;
     return NB_OK;
+}
+
+int small_vjp(int n, const float4 *pos, const float4 *gbuf, float eps2, const float4 *acc, float4 *lx, float4 *lv,
+              float *gm, float4 *gnext, float damping, float dt, int kick, float G, int want_next_g, cudaStream_t s)
+{
+    if (n == 0) return NB_OK;
+    return pdl_launch("small_vjp_kernel launch", small_vjp_kernel<kVjpSmallTargets>,
+                      (unsigned)((n + kVjpSmallTargets - 1) / kVjpSmallTargets), kVjpSmallThreads, s, pos, gbuf, n, eps2,
+                      acc, lx, lv, gm, gnext, damping, dt, kick, G, want_next_g);
 }
 
 int sym_vjp(const SymPlan &p, const float4 *pos, const float4 *gbuf, float eps2, float4 *tpart,

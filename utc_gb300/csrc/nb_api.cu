@@ -1040,7 +1040,7 @@ static int adj_reserve(nb_ctx *c, int nckpt, int every)
             (st = dev_alloc((void **)&A.vel_tmp2, n * sizeof(float4), "adjoint allocation")) ||
             (st = dev_alloc((void **)&A.lx, n * sizeof(float4), "adjoint allocation")) ||
             (st = dev_alloc((void **)&A.lv, n * sizeof(float4), "adjoint allocation")) ||
-            (st = dev_alloc((void **)&A.gbuf, n * sizeof(float4), "adjoint allocation")) ||
+            (st = dev_alloc((void **)&A.gbuf, (A.sym && A.splan.small ? 2 : 1) * n * sizeof(float4), "adjoint allocation")) ||
             (st = dev_alloc((void **)&A.gm, n * sizeof(float), "adjoint allocation")))
             return st;
     }
@@ -1227,6 +1227,7 @@ int nb_adj_backward(nb_ctx *c, unsigned long long generation, const void *gx_T, 
         return st;
     if (!A.taped && !live && (st = recompute(last, buf_of(last), s))) return st;
     bool have_g = false;
+    float4 *g = A.gbuf;  // small systems alternate between its two halves
     for (int seg = last; seg >= 0; --seg) {
         const int b = buf_of(seg);
         if (seg < last) NB_CUDA(cudaStreamWaitEvent(s, A.ev_rec[b], 0));
@@ -1251,6 +1252,13 @@ int nb_adj_backward(nb_ctx *c, unsigned long long generation, const void *gx_T, 
                 have_g = true;
             }
             const bool more = !(seg == 0 && k == 0);
+            if (A.sym && A.splan.small) {
+                float4 *gnext = g == A.gbuf ? A.gbuf + n : A.gbuf;
+                if ((st = nb::small_vjp(p.n, xk, g, eps2, ak, A.lx, A.lv, A.gm, gnext, D, dt, p.kick, G, more ? 1 : 0, s)))
+                    return st;
+                g = gnext;
+                continue;
+            }
             if (A.sym) {
                 if ((st = nb::sym_vjp(A.splan, xk, A.gbuf, eps2, A.sym_t, A.sym_s, s)) ||
                     (st = nb::adj_update_sym(A.splan, A.sym_t, A.sym_s, xk, ak, A.lx, A.lv, A.gm, A.gbuf, D,

@@ -568,6 +568,10 @@ int adj_update(const SkPlan &p, const float4 *partial, const float4 *pos_prev, c
 // Symmetric vector-Jacobian product (each unordered pair once) on the
 // symmetric work layout; tpart/spart as in sym_force.
 int sym_vjp_plan(int n, int warps, int bpt, int device, SymPlan *pl);
+// One reverse step of a plan with `small` set, pairs and update; g of the next
+// step (if wanted) goes to gnext, which is not gbuf.
+int small_vjp(int n, const float4 *pos, const float4 *gbuf, float eps2, const float4 *acc, float4 *lx, float4 *lv,
+              float *gm, float4 *gnext, float damping, float dt, int kick, float G, int want_next_g, cudaStream_t s);
 int sym_vjp(const SymPlan &p, const float4 *pos, const float4 *gbuf, float eps2, float4 *tpart,
             float4 *spart, cudaStream_t s);
 int adj_update_sym(const SymPlan &p, const float4 *tpart, const float4 *spart, const float4 *pos_prev,

@@ -184,6 +184,36 @@ __device__ __forceinline__ float3 chunk_react(PairTargets<NP> &t, const float4 *
     return ORDERED ? f : make_float3(f2_fold(fx), f2_fold(fy), f2_fold(fz));
 }
 
+constexpr int pow2_up(int x) { return x <= 2 ? 2 : x <= 4 ? 4 : x <= 8 ? 8 : 16; }
+
+// Sums v[0..C T) (T targets x C components) over the warp.  While more than
+// one target is left the lanes halve them: a lane keeps the half that its bit
+// selects and gives the other away, so that the first levels cost C T / 2,
+// C T / 4, ... shuffles.  Returns the lane's target; every lane of a target's
+// group has its C sums.
+template <int T, int C>
+__device__ __forceinline__ int warp_sum(float *v, int lane)
+{
+    int mine = 0, off = 16;
+#pragma unroll
+    for (int h = T / 2; h >= 1; h /= 2) {
+        const bool up = (lane & off) != 0;
+        mine = 2 * mine + (up ? 1 : 0);
+#pragma unroll
+        for (int k = 0; k < C * h; ++k) {
+            const float give = up ? v[k] : v[C * h + k], keep = up ? v[C * h + k] : v[k];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+        }
+        off /= 2;
+    }
+#pragma unroll
+    for (; off >= 1; off /= 2) {
+#pragma unroll
+        for (int k = 0; k < C; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], off);
+    }
+    return mine;
+}
+
 // Packed two-sum (Knuth): s + e == a + b exactly, s = fl(a + b).
 __device__ __forceinline__ void f2_two_sum(f2 a, f2 b, f2 &s, f2 &e)
 {

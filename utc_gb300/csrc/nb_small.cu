@@ -29,36 +29,6 @@ namespace nb {
 
 constexpr int kSmallThreads = 128;
 
-constexpr int pow2_up(int x) { return x <= 2 ? 2 : x <= 4 ? 4 : x <= 8 ? 8 : 16; }
-
-// Sums v[0..3 T) (T targets x 3 components) over the warp.  While more than
-// one target is left the lanes halve them: a lane keeps the half that its bit
-// selects and gives the other away, so that the first levels cost 3 T / 2,
-// 3 T / 4, ... shuffles.  Returns the lane's target; every lane of a target's
-// group has its three sums.
-template <int T>
-__device__ __forceinline__ int warp_sum(float *v, int lane)
-{
-    int mine = 0, off = 16;
-#pragma unroll
-    for (int h = T / 2; h >= 1; h /= 2) {
-        const bool up = (lane & off) != 0;
-        mine = 2 * mine + (up ? 1 : 0);
-#pragma unroll
-        for (int k = 0; k < 3 * h; ++k) {
-            const float give = up ? v[k] : v[3 * h + k], keep = up ? v[3 * h + k] : v[k];
-            v[k] = keep + __shfl_xor_sync(0xffffffffu, give, off);
-        }
-        off /= 2;
-    }
-#pragma unroll
-    for (; off >= 1; off /= 2) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], off);
-    }
-    return mine;
-}
-
 // pos_old is not declared __restrict__: it is written until the wait below, so
 // no load of it may take the read-only path.
 // pos_new == nullptr: no step, only acc_out; acc_out may be given beside a
@@ -112,7 +82,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_step_kernel(const floa
         s[3 * t + 1] = a.y;
         s[3 * t + 2] = a.z;
     }
-    const int t = warp_sum<TP>(s, lane);
+    const int t = warp_sum<TP, 3>(s, lane);
     if ((lane & (32 / TP - 1)) == 0) {
         red[wid][3 * t] = s[0];
         red[wid][3 * t + 1] = s[1];
