@@ -138,7 +138,7 @@ typedef struct nb_params {
  * order; or added at once into per-body 64-bit fixed-point accumulators with
  * integer atomics, 48 B per body, summed essentially exactly and still
  * deterministic (integer sums do not depend on their order), but measured
- * 2-10 % slower on GB300 at the same launch shape.  Where the triangular
+ * 3 % slower on GB300 at the same launch shape (N = 65536).  Where the triangular
  * array would pass 8 GiB even with 4 warps x 20 targets per lane (N above
  * about 1.66e6), it is cut into bands of consecutive row blocks, stepped
  * band by band through one 8 GiB buffer (nb_params.bands; the float-float
@@ -375,7 +375,10 @@ int nb_state_ptrs(nb_ctx *ctx, void **pos_dev, void **vel_dev);
  * CTA * 32, bpt = targets per lane and the target block is the row block.
  * NB_F32 symmetric contexts of up to 9000 bodies step in one launch of a
  * kernel of their own where their shape is the automatic one (unless bands
- * or NB_SOURCE_FIXED are asked for); they report that automatic shape. */
+ * or NB_SOURCE_FIXED are asked for); they report that automatic shape.  So do
+ * NB_F64 symmetric contexts of up to 2400 bodies (scaling, then one launch) and
+ * NB_F32 directed ones of up to 24576 (one launch for the sums, then the
+ * integrator). */
 int nb_plan_info(nb_ctx *ctx, int *info5);
 
 /* Source side of a symmetric context: info4 = {source side (NB_SOURCE_FIXED

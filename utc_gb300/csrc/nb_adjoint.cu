@@ -25,7 +25,9 @@
 // once on the forward symmetric kernel's layout (row blocks x 32-body
 // chunks, the chunk rotating through the warp with its accumulated reaction):
 // 18 shared operations + 8 per side = 34 FP32 operations and one rsqrt per
-// pair, 17 per ordered interaction instead of 26.
+// pair, 17 per ordered interaction instead of 26.  Systems of up to 7000 bodies
+// take both orders of every pair and a whole reverse step in one launch instead
+// (small_vjp_kernel).
 #include "nb_vjp.cuh"
 
 namespace nb {
