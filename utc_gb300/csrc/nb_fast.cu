@@ -248,7 +248,7 @@ __global__ void sk_integrate_kernel(const float4 *pos_old, float4 *pos_new, floa
 // kernel of nb_small.cu, which sums each target in one CTA, so that the
 // integrator reads one partial per body in place of up to 60.  Graph-replayed
 // step, GB300, us, against the stream-K kernel: N = 300 3.5 (5.1), 1000 3.7 (7.3),
-// 4099 10.8 (22.7), 8192 29.7 (40.0), 12345 64 (70.5), 16384 105 (110), 24000 216
+// 4099 10.8 (22.7), 8192 29.7 (40.0), 12345 64 (70.5), 16384 103 (110), 24000 216
 // (224).  At 32768, with blocks of 256 threads, stream-K is ahead (387 against
 // 393): it pads targets less there, and its CTAs end together, while the
 // CTAs of a direct launch leave a ragged last wave.

@@ -4,7 +4,7 @@
 // the sum of every body's partials), and a small system has few (row, chunk)
 // items for 152 SMs: at N = 1024 the pair terms take a third of a microsecond
 // of the chip, but the two launches took 7.4 us from a graph and 12.3 us one
-// by one.  Here a CTA owns TB bodies for the whole step: its 256 threads split
+// by one.  Here a CTA owns TB bodies for the whole step: its 128 threads split
 // the sources, every pair is evaluated from the target's side (both orders
 // are evaluated, 12 FP32 operations and one rsqrt each: twice the pair terms,
 // but no partial leaves the CTA), the sums are reduced through the warps and
@@ -15,14 +15,17 @@
 // bits.  Direct plans of nb_fast.cu use it for their force launch.
 //
 // Step time from a replayed graph, GB300, us, against the two launches:
-// N = 512 1.8 (6.4), 1024 2.2 (7.1), 2048 3.6 (9.2), 3000 5.4 (12.8), 4099
-// 9.2 (16.3), 6000 16.0 (23.7), 8192 28 (32.5).  Bounds: latency below N about
+// N = 512 1.7 (6.4), 1024 2.2 (7.1), 2048 3.6 (9.2), 3000 5.4 (12.8), 4099
+// 9.0 (16.3), 6000 15.7 (23.7), 8192 28 (32.5).  Bounds: latency below N about
 // 2000 (launch, one round of loads, the reduction), above it register-file
 // reads (26 operand reads a pair of interactions, nb_pair.cuh) and how evenly
 // the CTAs fill the SMs.  128 threads a CTA ran 5 to 30 % ahead of 256 and
 // 512; the launch bound of one CTA lets the loop have the registers that it
-// asks for (142 for 8 targets, 110 for 4; without it 64, and 3.5 us at
-// N = 1024).
+// asks for (146 for 8 targets, 108 for 4; without it 64, and 3.5 us at
+// N = 1024).  With 10 targets three CTAs an SM are asked for: with 172
+// registers there were two, and 11.8 us at N = 4099.  Sources per turn of the
+// loop: 4, with 6 targets 5 (N = 5000 12.7 us, 13.1 with 4), with 10 targets 3
+// (N = 4099 9.0, 9.7 with 4).
 #include "nb_pair.cuh"
 
 namespace nb {
@@ -34,7 +37,7 @@ constexpr int kSmallThreads = 128;
 // pos_new == nullptr: no step, only acc_out; acc_out may be given beside a
 // step too.
 template <int TB>
-__global__ void __launch_bounds__(kSmallThreads, 1) small_step_kernel(const float4 *pos_old,
+__global__ void __launch_bounds__(kSmallThreads, TB == 10 ? 3 : 1) small_step_kernel(const float4 *pos_old,
                                                                    float4 *__restrict__ pos_new,
                                                                    float4 *__restrict__ vel, int n, int lo, int hi, float eps2,
                                                                    float damping, float dt, int kick, float G,
@@ -64,6 +67,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_step_kernel(const floa
     PairTargets<NP> T;
     T.load([&](int t) { return t0 + t < n ? pos_old[t0 + t] : make_float4(0.f, 0.f, 0.f, 0.f); });
     float4 nxt = tid < n ? pos_old[tid] : pad;
+    constexpr int U = TB == 10 ? 3 : TB == 6 ? 5 : 4;
+#pragma unroll(U)
     for (int j = tid; j - tid < n; j += kSmallThreads) {
         const float4 q = nxt;
         const int jn = j + kSmallThreads;
@@ -116,19 +121,20 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_step_kernel(const floa
 // Targets per CTA: few bodies per CTA while the step is a chain of latencies
 // (below 2000 bodies), then the choice that leaves the fullest SM the least
 // to do: ceil(CTAs / SMs) CTAs of TB bodies each, plus 0.9 of a body's work per
-// CTA for its pass over the sources and its reduction (measured for 4 to 16
-// bodies at twelve sizes: N = 3000 6.0 us with 10 bodies, 6.5 with 8, 6.7
-// with 6; N = 6000 15.9 with 8, 17.3 with 6).  Above kSmallBodies 8: N = 12345 62.5
-// us (6: 62.9, 10: 64.4, 12: 65.8, 16: 75.9), N = 20000 153.6 (10: 158.5).
+// CTA for its pass over the sources and its reduction, and 3 % more for the
+// slower schedule with 8.  6 / 8 / 10 bodies, step us: N = 3000 6.5 / 6.2 / 5.4,
+// 4099 10.7 / 9.8 / 9.0, 5000 12.7 / 13.6 / 13.6, 6000 17.0 / 16.3 / 15.7, 7000 21.8 /
+// 21.9 / 21.8, 8192 28.2 / 28.5 / 29.3; the force launch of direct plans and their
+// integrator: 9001 35.6 / 37.1 / 34.2, 12345 64.0 / 65.7 / 64.7, 16384 106.2 / 107.6 /
+// 102.5, 20000 157.2 / 158.3 / 157.6, 24576 233.3 / 235.8 / 231.0.
 static int small_targets(int n, int sms)
 {
     if (n < 2000) return 4;
-    if (n > kSmallBodies) return 8;
     int best = 8;
     float least = 1e30f;
     for (int tb = 6; tb <= 10; tb += 2) {
         const int ctas = (n + tb - 1) / tb;
-        const float cost = (float)((ctas + sms - 1) / sms) * ((float)tb + 0.9f);
+        const float cost = (float)((ctas + sms - 1) / sms) * ((float)tb + 0.9f) * (tb == 8 ? 1.03f : 1.f);
         if (cost < least) {
             least = cost;
             best = tb;

@@ -156,7 +156,7 @@ __device__ __noinline__ void sym_row_segment(const float4 *__restrict__ pos, int
         if (wid == 0) nxt = jb + 32 + lane < n ? pos[jb + 32 + lane] : pad;
         if (kc < (I + 1) * RC) {
             // chunk inside the own row block: directed, target side only
-            chunk_pull<NP, COMP>(T, sC, EPS2);
+            chunk_pull(T, sC, EPS2);
         } else {
             // f: the reaction on chunk body `lane` from this warp
             const float3 f = chunk_react<NP, COMP>(T, sC, lane, EPS2);
