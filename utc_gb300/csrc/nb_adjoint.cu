@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(NT) vjp_pair_kernel(const float4 *__restrict__
 // [kc0, kc1), target-side sums to dst, reactions to sp.  Not inlined into the
 // loop over rows, as sym_row_segment of nb_sym.cu.
 template <int W, int BPT>
-__device__ __noinline__ void sym_vjp_segment(const float4 *__restrict__ pos, const float4 *__restrict__ gbuf, int n,
+__device__ __noinline__ void sym_vjp_segment(const float4 *pos, const float4 *gbuf, int n,
                                              float eps2, float4 *dst, float4 *sp, int I, int kc0, int kc1)
 {
     constexpr int NP = BPT / 2;
@@ -194,10 +194,10 @@ __device__ __noinline__ void sym_vjp_segment(const float4 *__restrict__ pos, con
 }
 
 template <int W, int BPT, int MINB>
-__global__ void __launch_bounds__(32 * W, MINB) sym_vjp_kernel(const float4 *__restrict__ pos,
-                                                               const float4 *__restrict__ gbuf, int n,
-                                                               float eps2, float4 *__restrict__ tpart,
-                                                               float4 *__restrict__ spart,
+__global__ void __launch_bounds__(32 * W, MINB) sym_vjp_kernel(const float4 *pos,
+                                                               const float4 *gbuf, int n,
+                                                               float eps2, float4 *tpart,
+                                                               float4 *spart,
                                                                long long total, int nc, int nrb)
 {
     pdl_wait();

@@ -138,10 +138,10 @@ __global__ void __launch_bounds__(32 * WPB) bk_force_kernel(const float4 *__rest
 // The reference's kick / damping / drift (unfused, its order), or the bare
 // acceleration when acc_out != nullptr.
 __device__ __forceinline__ void batch_kick_drift(int i, float ax, float ay, float az,
-                                                 const float4 *__restrict__ pos_old,
-                                                 float4 *__restrict__ pos_new, float4 *__restrict__ vel,
+                                                 const float4 *pos_old,
+                                                 float4 *pos_new, float4 *vel,
                                                  float damping, float dt, int kick, float G,
-                                                 float4 *__restrict__ acc_out)
+                                                 float4 *acc_out)
 {
     if (acc_out) {
         acc_out[i] = make_float4(ax, ay, az, 0.f);
@@ -206,7 +206,7 @@ struct BatchSymDev {
 // targets against the chunks [kc0, kc1), target-side sums to dst, reactions to
 // sp.  As sym_row_segment of nb_sym.cu, and like it not inlined.
 template <int WPB, int BPT>
-__device__ __noinline__ void bks_row_segment(const float4 *__restrict__ pos, int ns, float eps2, float4 *dst,
+__device__ __noinline__ void bks_row_segment(const float4 *pos, int ns, float eps2, float4 *dst,
                                              float4 *sp, int I, int kc0, int kc1)
 {
     constexpr int RB = 32 * BPT;
@@ -247,9 +247,9 @@ __device__ __noinline__ void bks_row_segment(const float4 *__restrict__ pos, int
 // the scalar loop that this replaces: 4341 us with 12 targets per lane, 4409
 // with 16; now 3828 and 3821.
 template <int WPB, int BPT>
-__global__ void __launch_bounds__(32 * WPB, 8 / WPB) bks_force_kernel(const float4 *__restrict__ pos, BatchSymDev bd,
-                                                             float eps2, float4 *__restrict__ tpart,
-                                                             float4 *__restrict__ spart, long long total,
+__global__ void __launch_bounds__(32 * WPB, 8 / WPB) bks_force_kernel(const float4 *pos, BatchSymDev bd,
+                                                             float eps2, float4 *tpart,
+                                                             float4 *spart, long long total,
                                                              int workers)
 {
     pdl_wait();
@@ -283,8 +283,8 @@ __global__ void __launch_bounds__(32 * WPB, 8 / WPB) bks_force_kernel(const floa
 // (warp order) and every Qth of the entries of rows 0..I-1 of its system (row
 // order); four are added pairwise.  add(v) takes a partial.
 template <int Q, class Add>
-__device__ __forceinline__ void bks_walk(int i, int q, const float4 *__restrict__ tpart,
-                                              const float4 *__restrict__ spart, const BatchSymDev &bd, int rb,
+__device__ __forceinline__ void bks_walk(int i, int q, const float4 *tpart,
+                                              const float4 *spart, const BatchSymDev &bd, int rb,
                                               long long total, int workers, Add add)
 {
     const int s = bd.body_sys[i];
@@ -351,8 +351,8 @@ __global__ void __launch_bounds__(256) bks_integrate_kernel(const float4 *pos_ol
 // A warp's share of a row of one system (its bodies from o on): as
 // symff_row_segment of nb_symff.cu, one warp.
 template <int WPB, int BPT>
-__device__ __noinline__ void bksff_row_segment(const float4 *__restrict__ H, const float4 *__restrict__ Mi,
-                                               const float4 *__restrict__ Lo, int o, int ns, float eps_h, float eps_l,
+__device__ __noinline__ void bksff_row_segment(const float4 *H, const float4 *Mi,
+                                               const float4 *Lo, int o, int ns, float eps_h, float eps_l,
                                                double4 *dst, double4 *sp, int I, int kc0, int kc1)
 {
     constexpr int NP = BPT / 2;
@@ -417,9 +417,9 @@ __device__ __noinline__ void bksff_row_segment(const float4 *__restrict__ H, con
 // each chunk's target sums folded into FP64, reactions written as FP64.
 template <int WPB, int BPT>
 __global__ void __launch_bounds__(32 * WPB)
-    bksff_force_kernel(const float4 *__restrict__ H, const float4 *__restrict__ Mi, const float4 *__restrict__ Lo,
+    bksff_force_kernel(const float4 *H, const float4 *Mi, const float4 *Lo,
                        BatchSymDev bd, double eps2, const unsigned long long *range,
-                       double4 *__restrict__ tpart, double4 *__restrict__ spart, long long total, int workers)
+                       double4 *tpart, double4 *spart, long long total, int workers)
 {
     pdl_wait();
     constexpr int RB = 32 * BPT;

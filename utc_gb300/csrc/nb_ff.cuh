@@ -201,8 +201,8 @@ struct FFTargets {
     // body(k): the index of target k of the lane, < 0 for a missing one,
     // which gets zero mass: its reactions are 0
     template <class Body>
-    __device__ __forceinline__ void load(const float4 *__restrict__ H, const float4 *__restrict__ M,
-                                         const float4 *__restrict__ L, Body body)
+    __device__ __forceinline__ void load(const float4 *H, const float4 *M,
+                                         const float4 *L, Body body)
     {
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll

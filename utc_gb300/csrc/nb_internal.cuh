@@ -244,8 +244,10 @@ __host__ __device__ __forceinline__ int sk_owner(long long it, long long total, 
 // Launch of a kernel that begins with pdl_wait(): its blocks come in as those of
 // the stream's kernel before it leave, and wait there until that kernel is
 // complete and its writes are visible (0.4 us a launch less than a plain one).
-// No argument that the kernel before writes may be read through const
-// __restrict__: read-only loads may be moved ahead of the wait.
+// Neither such a kernel nor a function that it calls, inlined or not, has a
+// __restrict__ parameter or uses a read-only load: the compiler may take the wait
+// for one that leaves memory behind a __restrict__ pointer alone, and move the
+// load of what the kernel before writes ahead of it.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <class... P, class... A>
@@ -529,10 +531,10 @@ int sym_comp_integrate(const SymPlan &p, const float4 *tpart, const float4 *spar
 // and, when want_next_g, g for the next reverse step (at the previous state,
 // whose masses are the same).
 __device__ __forceinline__ void adj_body_update(int i, float ox, float oy, float oz, float odm,
-                                                const float4 *__restrict__ pos,
-                                                const float4 *__restrict__ acc,
-                                                float4 *__restrict__ lx, float4 *__restrict__ lv,
-                                                float *__restrict__ gm, float4 *__restrict__ gbuf,
+                                                const float4 *pos,
+                                                const float4 *acc,
+                                                float4 *lx, float4 *lv,
+                                                float *gm, float4 *gbuf,
                                                 float damping, float dt, int kick, float G,
                                                 int want_next_g)
 {

@@ -117,9 +117,9 @@ __global__ void sk_reduce_kernel(const float4 *__restrict__ partial, int n, int 
 
 // Compensated kick / damping (FP32 with a carried low part) and FP64 drift,
 // given the acceleration as a compensated sum S + C.
-__device__ __forceinline__ void comp_kick_drift(int i, float4 S, float4 C, double4 *__restrict__ pos64,
-                                                float4 *__restrict__ pos32, float4 *__restrict__ vhi,
-                                                float4 *__restrict__ vlo, float damping, float dt,
+__device__ __forceinline__ void comp_kick_drift(int i, float4 S, float4 C, double4 *pos64,
+                                                float4 *pos32, float4 *vhi,
+                                                float4 *vlo, float damping, float dt,
                                                 double dt64, int kick, float G)
 {
     const float ax = __fadd_rn(S.x, C.x), ay = __fadd_rn(S.y, C.y), az = __fadd_rn(S.z, C.z);

@@ -32,16 +32,14 @@ namespace nb {
 
 constexpr int kSmallThreads = 128;
 
-// pos_old is not declared __restrict__: it is written until the wait below, so
-// no load of it may take the read-only path.
 // pos_new == nullptr: no step, only acc_out; acc_out may be given beside a
 // step too.
 template <int TB>
 __global__ void __launch_bounds__(kSmallThreads, TB == 10 ? 3 : 1) small_step_kernel(const float4 *pos_old,
-                                                                   float4 *__restrict__ pos_new,
-                                                                   float4 *__restrict__ vel, int n, int lo, int hi, float eps2,
+                                                                   float4 *pos_new,
+                                                                   float4 *vel, int n, int lo, int hi, float eps2,
                                                                    float damping, float dt, int kick, float G,
-                                                                   float4 *__restrict__ acc_out)
+                                                                   float4 *acc_out)
 {
     constexpr int NP = TB / 2, TP = pow2_up(TB);
     constexpr int NW = kSmallThreads / 32;

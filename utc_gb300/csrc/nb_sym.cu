@@ -102,7 +102,7 @@ __device__ __forceinline__ void fx_add(unsigned long long *hi_p, unsigned long l
 // A reaction (fx, fy, fz) on body j into the fixed-point accumulators.
 __device__ __forceinline__ void fx_emit(unsigned long long *acc, int n, int j, float fx, float fy, float fz)
 {
-    const float4 r = __ldg(fx_record(acc, n));
+    const float4 r = *fx_record(acc, n);
     const long long nn = n;
     fx_add(acc + j, acc + 3 * nn + j, fx, r);
     fx_add(acc + nn + j, acc + 4 * nn + j, fy, r);
@@ -116,7 +116,7 @@ __device__ __forceinline__ void fx_emit(unsigned long long *acc, int n, int j, f
 // moves per launch at N = 65536 (936 M instructions against 665 M, 3107
 // against 3660 G interactions/s on the same box).
 template <int W, int BPT, bool COMP, bool FX>
-__device__ __noinline__ void sym_row_segment(const float4 *__restrict__ pos, int n, float eps2, float4 *dst,
+__device__ __noinline__ void sym_row_segment(const float4 *pos, int n, float eps2, float4 *dst,
                                              float4 *spart, long long soff, long long tlo, long long slo, int I,
                                              int kc0, int kc1)
 {
@@ -236,9 +236,9 @@ __device__ __noinline__ void sym_row_segment(const float4 *__restrict__ pos, int
 // [it0, it0 + total) covering row blocks from r0 on: target-side slot
 // c + I - r0, source-side entries offset by soff0 (the band's first entry).
 template <int W, int BPT, int MINB, bool COMP, bool FX = false, bool BAND = false>
-__global__ void __launch_bounds__(32 * W, MINB) sym_force_kernel(const float4 *__restrict__ pos, int n,
-                                                           float eps2, float4 *__restrict__ tpart,
-                                                           float4 *__restrict__ spart,
+__global__ void __launch_bounds__(32 * W, MINB) sym_force_kernel(const float4 *pos, int n,
+                                                           float eps2, float4 *tpart,
+                                                           float4 *spart,
                                                            long long total, int nc, int nrb,
                                                            long long tlo, long long slo, long long it0,
                                                            int r0, long long soff0)

@@ -178,8 +178,8 @@ __global__ void __launch_bounds__(kFFFusedBlock) ff_range_split_kernel(const dou
 // PHI: also the potential sum_j m_j inv (j != i) in the partials' w, the
 // reaction's included (energy pass).
 template <int W, int BPT, bool PHI>
-__device__ __noinline__ void symff_row_segment(const float4 *__restrict__ H, const float4 *__restrict__ Mi,
-                                               const float4 *__restrict__ Lo, int n, float eps_h, float eps_l,
+__device__ __noinline__ void symff_row_segment(const float4 *H, const float4 *Mi,
+                                               const float4 *Lo, int n, float eps_h, float eps_l,
                                                double4 *dst, double4 *spart, long long soff, int I, int kc0, int kc1)
 {
     constexpr int NP = BPT / 2;
@@ -272,9 +272,9 @@ __device__ __noinline__ void symff_row_segment(const float4 *__restrict__ H, con
 // source-side entries offset by soff0.
 template <int W, int BPT, int MINB, bool PHI, bool BAND = false>
 __global__ void __launch_bounds__(32 * W, MINB)
-    symff_force_kernel(const float4 *__restrict__ H, const float4 *__restrict__ Mi, const float4 *__restrict__ Lo,
+    symff_force_kernel(const float4 *H, const float4 *Mi, const float4 *Lo,
                        int n, double eps2, const unsigned long long *range,
-                       double4 *__restrict__ tpart, double4 *__restrict__ spart, long long total, int nc, int nrb,
+                       double4 *tpart, double4 *spart, long long total, int nc, int nrb,
                        long long it0, int r0, long long soff0)
 {
     pdl_wait();
