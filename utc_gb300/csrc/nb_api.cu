@@ -973,21 +973,15 @@ int nb_energy(nb_ctx *c, double *out5, void *accphi_dev, void *stream)
 // ---------------------------------------------------------------------------
 // adjoint: forward with checkpoints, reverse pass with per-segment recompute
 // ---------------------------------------------------------------------------
-// Most that the states of a forward pass may take for all of them to be kept.
-// The caller's ckpt_every bounds the memory of long trajectories of large
-// systems; below this size the recomputation that it costs (a forward step per
-// reverse step: 85 of 350 us at N = 16384) buys less than a hundredth of the
-// GPU's memory.
-constexpr size_t kAdjTapeBytes = (size_t)1 << 30;
-
 // Room for a tape of `steps` steps; false when it would be too large or the
 // device has none left (the checkpoints then serve).
 static bool adj_reserve_tape(nb_ctx *c, int steps)
 {
     auto &A = c->adj;
-    const size_t n = (size_t)c->p.n, np = n * ((size_t)steps + 1);
-    const size_t na = c->p.kick == NB_KICK_REFERENCE ? n * (size_t)steps : 0;
-    if (n == 0 || (np + na) * sizeof(float4) > kAdjTapeBytes) return false;
+    const size_t n = (size_t)c->p.n;
+    const bool ref = c->p.kick == NB_KICK_REFERENCE;
+    if (!nb::adj_tape_fits(n, steps, ref, nb::kAdjTapeBytes)) return false;
+    const size_t np = n * ((size_t)steps + 1), na = ref ? n * (size_t)steps : 0;
     auto grow = [](float4 **buf, size_t *cap, size_t need) {
         if (need <= *cap) return true;
         nb::dfree(*buf);

@@ -526,6 +526,20 @@ int sym_comp_integrate(const SymPlan &p, const float4 *tpart, const float4 *spar
                        double dt64, int kick, float G, double4 *acc_out, cudaStream_t s,
                        const float4 *accsum = nullptr);
 
+// Most that the states of a forward pass may take for all of them to be kept.  The caller's
+// ckpt_every bounds the memory of long trajectories of large systems; below this
+// size the recomputation that it costs (a forward step per reverse step: 85 of
+// 350 us at N = 16384) buys less than a hundredth of the GPU's memory.
+constexpr unsigned long long kAdjTapeBytes = 1ull << 30;
+
+// steps + 1 states of n bodies, and with the reference kick steps accelerations,
+// 16 bytes a body each, fit `limit` bytes (no product that could wrap).
+inline bool adj_tape_fits(size_t n, int steps, bool ref, unsigned long long limit)
+{
+    const unsigned long long arrays = (unsigned long long)steps * (ref ? 2 : 1) + 1;
+    return n > 0 && arrays <= limit / 16 / n;
+}
+
 // One reverse step's per-body update given the summed pair terms (o, odm):
 //   lx <- lx + out;  lv <- D mu;  gm += dm (+ D dt mu.a in reference mode)
 // and, when want_next_g, g for the next reverse step (at the previous state,
