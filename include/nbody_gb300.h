@@ -218,8 +218,9 @@ int nb_energy(nb_ctx *ctx, double *out5, void *accphi_dev, void *stream);
  * nb_adj_forward advances the state like nb_step and keeps a checkpoint
  * (positions and velocities) every ckpt_every steps; where the positions of
  * all steps (and, with the reference kick, the accelerations: 16 or 32 B per
- * body and step) come to at most 1 GiB it keeps those instead, and nothing
- * below is recomputed (the gradients have the same bits).  nb_adj_backward then
+ * body and step) come to at most 1 GiB and an eighth of the memory that the
+ * device has free it keeps those instead, and nothing below is recomputed (the
+ * gradients have the same bits; nb_adj_tape_limit below).  nb_adj_backward then
  * takes the cotangents of the final positions gx_T and velocities gv_T
  * (device, n float4, xyz used; gv_T may be NULL for zero) and writes
  * dL/dx0, dL/dv0 (device n float4, w = 0) and dL/dm (device n float),
@@ -238,6 +239,11 @@ int nb_adj_forward(nb_ctx *ctx, int steps, int ckpt_every, void *stream,
                    unsigned long long *generation);
 int nb_adj_backward(nb_ctx *ctx, unsigned long long generation, const void *gx_T, const void *gv_T,
                     void *gx0, void *gv0, void *gm, void *stream);
+/* Most bytes that later nb_adj_forward calls of this context may keep all
+ * states in (1 GiB unless set; an eighth of the free memory holds besides).  0:
+ * checkpoints only, so that ckpt_every alone bounds the memory.  The buffers of
+ * one kind of pass are freed when a pass of the other kind begins. */
+int nb_adj_tape_limit(nb_ctx *ctx, unsigned long long bytes);
 
 /* The whole task run with host buffers, as BodySystemSGPU::runImpl
  * (body_task_sgpu.cu:40-137): copy pos/vel in, run `loops` steps, and after

@@ -58,6 +58,7 @@ def _declare(lib):
         "nb_step_timed": (I, [vp, I, P(C.c_float), P(C.c_float), vp]),
         "nb_energy": (I, [vp, P(D), vp, vp]),
         "nb_adj_forward": (I, [vp, I, I, vp, P(C.c_ulonglong)]),
+        "nb_adj_tape_limit": (I, [vp, C.c_ulonglong]),
         "nb_adj_backward": (I, [vp, C.c_ulonglong, vp, vp, vp, vp, vp, vp]),
         "nb_autotune": (I, [vp, I, C.c_char_p, vp, P(I)]),
         "nb_step_f32_noalloc": (I, [vp, vp, vp, I, C.c_float, C.c_float, C.c_float, I, C.c_float, vp]),

@@ -137,10 +137,11 @@ struct nb_ctx {
         bool live_last = false;
         // every state of the recorded forward pass, [steps + 1][n], and its
         // accelerations (reference kick), [steps][n]: nothing is recomputed
-        // where they fit kAdjTapeBytes
+        // where they fit tape_limit
         bool taped = false;
         float4 *tape_pos = nullptr, *tape_acc = nullptr;
         size_t cap_tape_pos = 0, cap_tape_acc = 0;  // float4 entries
+        unsigned long long tape_limit = nb::kAdjTapeBytes;
         // second segment buffer: segment s-1 is recomputed on rstream while
         // the reverse pass runs through segment s on the caller's stream
         float4 *seg_pos2 = nullptr, *seg_acc2 = nullptr, *vel_tmp2 = nullptr;
@@ -973,29 +974,52 @@ int nb_energy(nb_ctx *c, double *out5, void *accphi_dev, void *stream)
 // ---------------------------------------------------------------------------
 // adjoint: forward with checkpoints, reverse pass with per-segment recompute
 // ---------------------------------------------------------------------------
+// Free memory that a tape leaves, for each byte it takes: a program with many
+// contexts, or one that is short of memory, keeps checkpoints instead.
+constexpr size_t kAdjTapeShare = 8;
+
+static void adj_release_tape(nb_ctx *c)
+{
+    auto &A = c->adj;
+    nb::dfree(A.tape_pos);
+    nb::dfree(A.tape_acc);
+    A.tape_pos = A.tape_acc = nullptr;
+    A.cap_tape_pos = A.cap_tape_acc = 0;
+}
+
+static void adj_release_checkpoints(nb_ctx *c)
+{
+    auto &A = c->adj;
+    for (float4 **q : {&A.ckpt_pos, &A.ckpt_vel, &A.seg_pos, &A.seg_acc, &A.seg_pos2, &A.seg_acc2}) {
+        nb::dfree(*q);
+        *q = nullptr;
+    }
+    A.cap_ckpt = A.cap_seg = 0;
+}
+
 // Room for a tape of `steps` steps; false when it would be too large or the
-// device has none left (the checkpoints then serve).
+// device has too little left (the checkpoints then serve, and no part of a tape
+// is held beside them).
 static bool adj_reserve_tape(nb_ctx *c, int steps)
 {
     auto &A = c->adj;
     const size_t n = (size_t)c->p.n;
     const bool ref = c->p.kick == NB_KICK_REFERENCE;
-    if (!nb::adj_tape_fits(n, steps, ref, nb::kAdjTapeBytes)) return false;
+    if (!nb::adj_tape_fits(n, steps, ref, A.tape_limit)) return false;
     const size_t np = n * ((size_t)steps + 1), na = ref ? n * (size_t)steps : 0;
-    auto grow = [](float4 **buf, size_t *cap, size_t need) {
-        if (need <= *cap) return true;
-        nb::dfree(*buf);
-        *buf = nullptr;
-        *cap = 0;
-        if (nb::dmalloc((void **)buf, need * sizeof(float4)) != cudaSuccess) {
-            *buf = nullptr;
-            (void)cudaGetLastError();
-            return false;
-        }
-        *cap = need;
-        return true;
-    };
-    return grow(&A.tape_pos, &A.cap_tape_pos, np) && grow(&A.tape_acc, &A.cap_tape_acc, na);
+    if (np <= A.cap_tape_pos && na <= A.cap_tape_acc) return true;
+    adj_release_tape(c);
+    size_t left = 0, all = 0;
+    if (cudaMemGetInfo(&left, &all) != cudaSuccess || (np + na) * sizeof(float4) > left / kAdjTapeShare ||
+        nb::dmalloc((void **)&A.tape_pos, np * sizeof(float4)) != cudaSuccess ||
+        (na && nb::dmalloc((void **)&A.tape_acc, na * sizeof(float4)) != cudaSuccess)) {
+        (void)cudaGetLastError();
+        adj_release_tape(c);
+        return false;
+    }
+    A.cap_tape_pos = np;
+    A.cap_tape_acc = na;
+    return true;
 }
 
 static int adj_reserve(nb_ctx *c, int nckpt, int every)
@@ -1098,6 +1122,14 @@ static int adj_steps(nb_ctx *c, float4 *x, float4 *vel, float4 *acc, int len, cu
     return st;
 }
 
+int nb_adj_tape_limit(nb_ctx *c, unsigned long long bytes)
+{
+    if (!c) return set_error(NB_ERR_INVALID, "ctx is NULL");
+    if (!uses_fast(c)) return set_error(NB_ERR_UNSUPPORTED, "the adjoint needs an NB_F32 fast context");
+    c->adj.tape_limit = bytes;
+    return NB_OK;
+}
+
 int nb_adj_forward(nb_ctx *c, int steps, int ckpt_every, void *stream, unsigned long long *generation)
 {
     if (generation) *generation = 0;
@@ -1111,8 +1143,19 @@ int nb_adj_forward(nb_ctx *c, int steps, int ckpt_every, void *stream, unsigned 
     auto &A = c->adj;
     A.ready = false;  // what it holds may go from here on
     A.live_last = false;
-    const bool taped = adj_reserve_tape(c, steps);
+    // the buffers of the one kind of pass are not held through the other
+    bool taped = adj_reserve_tape(c, steps);
+    if (taped)
+        adj_release_checkpoints(c);
+    else
+        adj_release_tape(c);
     int st = taped ? adj_reserve(c, 0, 0) : adj_reserve(c, nckpt, ckpt_every);
+    if (st == NB_ERR_OOM && taped) {
+        (void)cudaGetLastError();
+        adj_release_tape(c);
+        taped = false;
+        st = adj_reserve(c, nckpt, ckpt_every);
+    }
     if (st) return st;
     cudaStream_t s = (cudaStream_t)stream;
     if ((st = fx_refresh(c, s))) return st;

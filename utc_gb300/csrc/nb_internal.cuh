@@ -526,7 +526,8 @@ int sym_comp_integrate(const SymPlan &p, const float4 *tpart, const float4 *spar
                        double dt64, int kick, float G, double4 *acc_out, cudaStream_t s,
                        const float4 *accsum = nullptr);
 
-// Most that the states of a forward pass may take for all of them to be kept.  The caller's
+// Most that the states of a recorded forward pass take, unless
+// nb_adj_tape_limit says otherwise, for all of them to be kept.  The caller's
 // ckpt_every bounds the memory of long trajectories of large systems; below this
 // size the recomputation that it costs (a forward step per reverse step: 85 of
 // 350 us at N = 16384) buys less than a hundredth of the GPU's memory.

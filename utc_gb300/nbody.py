@@ -204,7 +204,8 @@ class NBodySystem:
         return e
 
     def adj_forward(self, steps, ckpt_every, stream=None):
-        """Advance `steps` steps keeping a checkpoint every `ckpt_every` steps.
+        """Advance `steps` steps keeping a checkpoint every `ckpt_every` steps,
+        or every state where they are small (see adj_tape_limit).
         Returns the generation number of this recorded forward pass (also kept
         as self.adj_generation, the default of adj_backward)."""
         s = current_stream_handle() if stream is None else stream
@@ -213,6 +214,11 @@ class NBodySystem:
                                         C.byref(gen)), "nb_adj_forward")
         self.adj_generation = int(gen.value)
         return self.adj_generation
+
+    def adj_tape_limit(self, nbytes):
+        """Most bytes in which later forward passes may keep all their states
+        instead of checkpoints (1 GiB unless set; 0: checkpoints only)."""
+        N.check(self.lib.nb_adj_tape_limit(self.handle, C.c_ulonglong(int(nbytes))), "nb_adj_tape_limit")
 
     def adj_backward(self, gx_T, gv_T=None, stream=None, generation=None):
         """Cotangents of the final (n,4) positions / velocities (torch CUDA
