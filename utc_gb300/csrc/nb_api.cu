@@ -10,6 +10,8 @@
 #include <string>
 #include <vector>
 
+#include <cuda.h>
+
 #include "nb_internal.cuh"
 
 namespace nb {
@@ -510,24 +512,46 @@ static __global__ void state_copy_kernel(float4 *d0, const float4 *s0, float4 *d
         d1[i - n] = s1[i - n];
 }
 
+// `bytes` from q on lie in one allocation of device memory on `device`.  The
+// driver's pointer query gives the allocation's bounds too, which the runtime's
+// does not; where it cannot be had, or the range is part of something else, the
+// answer is no.
+static bool in_device_allocation(const void *q, size_t bytes, int device)
+{
+    typedef CUresult (*query_t)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+    static const query_t query = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult r = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &r) != cudaSuccess ||
+            r != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        (void)cudaGetLastError();
+        return (query_t)f;
+    }();
+    unsigned type = 0, managed = 0;
+    int ordinal = -1;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *into[] = {&type, &managed, &ordinal, &start, &size};
+    const CUdeviceptr a = (CUdeviceptr)(uintptr_t)q;
+    return query && query(5, what, into, a) == CUDA_SUCCESS && type == CU_MEMORYTYPE_DEVICE && !managed &&
+           ordinal == device && start <= a && bytes <= size && a - start <= size - bytes;
+}
+
 // Both arrays of the state between this context and a caller, `sb` bytes each,
 // in one launch where the caller's pointers are memory of this device that a
 // kernel may read 16 bytes at a time, otherwise (host memory, another device,
-// odd addresses, buffers that cross) as two copies in order.  The two copies
-// on either side of a small system's step cost the host 5.9 us each time, the
-// one launch 2.5, the step 2.0.
+// odd addresses, buffers that cross or end too early, which a copy refuses) as two
+// copies in order.  The two copies on either side of a small system's step cost
+// the host 5.9 us each time, the one launch 2.5, the step 2.0.
 static cudaError_t copy_state(const nb_ctx *c, void *d0, const void *s0, void *d1, const void *s1, size_t sb,
                               const void *user0, const void *user1, cudaStream_t s)
 {
     int dev = -1;
-    auto here = [&](const void *q) {
-        cudaPointerAttributes at;
-        if ((uintptr_t)q % 16 || cudaPointerGetAttributes(&at, q) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return false;
-        }
-        return at.type == cudaMemoryTypeDevice && at.device == c->device;
-    };
+    auto here = [&](const void *q) { return (uintptr_t)q % 16 == 0 && in_device_allocation(q, sb, c->device); };
     auto cross = [&](const void *a, const void *b) {
         const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
         return x < y + sb && y < x + sb;
