@@ -32,6 +32,7 @@ int set_error(int status, const std::string &msg)
 
 int cuda_error(cudaError_t e, const char *what)
 {
+    (void)cudaGetLastError();  // reported here: the next NB_LAUNCH_CHECK is not to find it again
     const int st = (e == cudaErrorMemoryAllocation) ? NB_ERR_OOM : NB_ERR_CUDA;
     return set_error(st, std::string(what) + ": " + cudaGetErrorName(e) + " (" +
                              cudaGetErrorString(e) + ")");
