@@ -1231,6 +1231,9 @@ int nb_batch_create(const nb_params *p, int nsys, const int *sizes, nb_batch **o
     const int wpb = p->block ? p->block / 32 : (b->sym ? 1 : 4);
     const int bpt = p->bpt ? p->bpt : (b->f64 ? 2 : (b->sym ? 12 : 4));
     int st = batch_apply_plan(b, wpb, bpt, nullptr);
+    // the source-side array of 16 targets per lane is 3/4 of that of 12: systems
+    // too large for the one may still have room for the other
+    if (st == NB_ERR_OOM && b->sym && !b->f64 && !p->block && !p->bpt) st = batch_apply_plan(b, 1, 16, nullptr);
     if (st) {
         free_batch(b);
         return st;
