@@ -20,7 +20,8 @@ Extension workloads, one JSON line each (not the headline):
                         vs compensated FP32 + FP64 positions: per-step force
                         and energy error against the FP64 oracle on a
                         4096-body subsample; forward throughput at N=1M
-  --workload adjoint    N=16384 uniform cube, 200 steps, checkpoints every 20:
+  --workload adjoint    N=16384 uniform cube, 200 steps, every state kept (53 MB,
+                        so checkpoints every 20 are not used):
                         adjoint/forward time ratio; gradient error against the
                         FP64 reference adjoint (full size) and FP64 central
                         differences (64 coordinates, N=2048 replica)
@@ -248,9 +249,9 @@ def sub_n1m_forward(peak_flops, source_side="auto"):
 
 
 def sub_adjoint(reps=3):
-    """The adjoint workload (N=16384 uniform cube, 200 steps, checkpoints
-    every 20, default symmetric kernels): medians of the plain forward, the
-    checkpointed forward and the backward (recompute + VJP)."""
+    """The adjoint workload (N=16384 uniform cube, 200 steps, default symmetric
+    kernels; all states are kept, 53 MB, and the interval of 20 is not used):
+    medians of the plain forward, the recording forward and the backward."""
     import torch
 
     from utc_gb300 import ics
@@ -290,7 +291,7 @@ def sub_adjoint(reps=3):
                 ts["adj_forward"].append(ta)
                 ts["adj_backward"].append(tb)
     med = {k: float(np.median(v)) for k, v in ts.items()}
-    return {"workload": f"adjoint, uniform cube N={n}, {T} steps, checkpoints every {K}, symmetric kernels",
+    return {"workload": f"adjoint, uniform cube N={n}, {T} steps, every state kept, symmetric kernels",
             "ms_median": med,
             "backward_over_forward": med["adj_backward"] / med["forward"],
             "backward_plus_ckpt_forward_over_forward": (med["adj_backward"] + med["adj_forward"]) / med["forward"]}
@@ -837,8 +838,8 @@ def run_adjoint(args):
         return a.elapsed_time(b)
 
     def measure(algo):
-        """Median times of the plain forward, the checkpointed forward and the
-        backward (recompute + VJP) with one algorithm's kernels."""
+        """Median times of the plain forward, the recording forward (every state
+        kept) and the backward with one algorithm's kernels."""
         sysm = NBodySystem(n, "f32", algo, kick="physical", eps2=eps2, damping=1.0, dt=dt)
         pT = torch.empty((n, 4), device="cuda")
         vT = torch.empty((n, 4), device="cuda")
@@ -867,7 +868,7 @@ def run_adjoint(args):
     other = "fast" if algo == "sym" else "sym"
     med, (gx0, gv0, gm) = measure(algo)
     med_o, g_o = measure(other)
-    out = {"workload": "adjoint", "n": n, "steps": T, "ckpt_every": K, "eps2": float(eps2),
+    out = {"workload": "adjoint", "n": n, "steps": T, "ckpt_every": K, "kept": "every state", "eps2": float(eps2),
            "dt": float(dt), "kick": "physical (G=1)", "algo": algo, "ms_median": med,
            "adjoint_over_forward": med["adj_backward"] / med["forward"],
            "adjoint_incl_ckpt_forward_over_forward": (med["adj_backward"] + med["adj_forward"]) / med["forward"],

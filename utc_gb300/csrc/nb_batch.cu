@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(32 * WPB)
 
 // Per body: FP64 sums of the target-side slots of its row (warp order) and
 // the source-side entries of rows 0..I-1 of its system (row order), every
-// eighth of them by each warp (integrate64), the batch's scaling undone (a =
+// fourth of them by each warp (integrate64), the batch's scaling undone (a =
 // a_scaled * 2^(2 kx - km), exact), then kick / damping / drift or the bare
 // acceleration.
 // Four warps a block: 53000 bodies 14.5 us, 150000 24.5 us (eight warps 22 and 35,

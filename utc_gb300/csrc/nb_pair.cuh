@@ -19,7 +19,8 @@
 // interactions/s, against 3578 for the scalar loop that it replaced, whose 17
 // issue slots per pair left no room for the operand stalls (the packed loop
 // issues 9); 4 warps x 20 targets at N = 262144: 3965 against 3574;
-// compensated 1 x 12: 3673 against 3166.  Timed beside it (the loop alone, 16
+// compensated 1 x 12 (ordered reactions, chunk_react) at N = 131072: 3624 against
+// 3166.  Timed beside it (the loop alone, 16
 // targets, 4022): the reaction folded to a scalar before each shuffle 3926,
 // the chunk stored as duplicated pairs in shared memory 3929, the reaction
 // added through shared memory 3887, packed differences with scalar

@@ -467,7 +467,7 @@ __device__ __forceinline__ void ff_add1(float &h, float &l, float gh, float gl)
     l = __fsub_rn(t, __fsub_rn(h, s));
 }
 
-// Sums (h, l)[0..3 T) over the warp as warp_sum of nb_small.cu does: the lanes
+// Sums (h, l)[0..3 T) over the warp as warp_sum of nb_pair.cuh does: the lanes
 // halve the targets while there is more than one, and the lane's target is
 // returned.
 template <int T>
